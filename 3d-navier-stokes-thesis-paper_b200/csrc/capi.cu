@@ -205,6 +205,7 @@ struct cfg_ctx {
   size_t sm_rhs64 = 0;
   // register-FFT pass-1 kernels (when the lengths are compiled in)
   bool fast_z = false, fast_x = false;
+  bool full_len = false;   // nx2 of regfft_full and nz2 rows in eights (the LES mode)
   bool use_rhs2 = true;
   int rhs2_lanes = 32;
   int rhs2_warps = 3;   // warps (wavenumbers) per k_rhs2 block
@@ -452,9 +453,11 @@ struct Impl {
     // (gP: the x stage's geometry, all kx and this rank's z2 rows)
     const Geom& gp = c->gP;
     if (c->xinv_zb && gp.nz2 % c->xinv_zb) c->xinv_zb = 0;
-    c->split_x = c->fast_x && (!getenv("CHANFLOW_FUSED_XFLUX") || c->nranks > 1) && gp.nz2 % 8 == 0 &&
-                 gp.nz2 % c->flux_zr == 0 && p1_fast_smem(3, g.nx2, f32, gp.nz2, gp.nxh, g.nz) <= 200 * 1024 &&
-                 p1_fast_smem(4, g.nx2, f32, c->flux_zr, gp.nxh, g.nz) <= 200 * 1024;
+    c->split_x = c->fast_x && (!getenv("CHANFLOW_FUSED_XFLUX") || c->nranks > 1) &&
+                 (c->nranks == 1 || gp.nz2 % 8 == 0) &&
+                 p1_fast_smem(3, g.nx2, f32, gp.nz2, gp.nxh, g.nz) <= 200 * 1024 &&
+                 p1_fast_smem(4, g.nx2, f32, flux_rows(c, false), gp.nxh, g.nz) <= 200 * 1024;
+    c->full_len = regfft_full(g.nx2) && gp.nz2 % 8 == 0;
     if (c->split_x &&
         cudaMalloc(&c->P, sizeof(T) * (size_t)(g.ny + 1) * 3 * gp.nz2 * g.nx2) != cudaSuccess) {
       cudaGetLastError();
@@ -500,17 +503,35 @@ struct Impl {
     return CFG_OK;
   }
 
+  // z rows per flux block: the tile where it divides the z2 rows (and, beside
+  // the lengths of regfft_full, where the products have that block), else 4
+  // or 2
+  static int flux_rows(const cfg_ctx* c, bool plain_products) {
+    const int zr = c->flux_zr, nz2 = c->gP.nz2;
+    if (nz2 % zr == 0 && (zr < 8 || plain_products || regfft_full(c->g.nx2))) return zr;
+    return nz2 % 4 == 0 ? 4 : 2;
+  }
+  // planes per z-transform block: the tile where its block can be launched
+  // (the lengths of regfft_full leave that to the launch)
+  static int z_planes(const cfg_ctx* c, int which, int yb) {
+    if (regfft_full(c->g.nz2)) return yb;
+    yb = std::min(yb, 5);   // 3 yb N2 <= 288 threads for N2 <= 18
+    while (yb > 1 && p1_fast_smem(which, c->g.nz2, sizeof(T) == 4, yb, c->g.nxh, c->g.nz) > 200 * 1024) --yb;
+    return yb;
+  }
+
   // the launch record of register-FFT pass-1 kernel `which` (0 k_zinv_r, 1
   // k_xflux_r, 2 k_zfwd_r, 3 k_xinv_r, 4 k_flux_r) in substep rk
   static P1Launch p1_args(const cfg_ctx* c, int rk, bool lin, int which) {
     const Geom& g = c->g;
     P1Launch a{};
     a.vel = c->vel; a.T1 = c->T1; a.T2 = c->T2; a.velout = c->vel; a.g = g; a.twx = c->twx; a.twz = c->twz;
-    a.gd = c->gd; a.fringe = c->fringe; a.has_fringe = c->has_fringe; a.YB1 = c->fYB1; a.YB3 = c->fYB3;
+    a.gd = c->gd; a.fringe = c->fringe; a.has_fringe = c->has_fringe;
+    a.YB1 = z_planes(c, 0, c->fYB1); a.YB3 = z_planes(c, 2, c->fYB3);
     a.ZR = c->fZR; a.cflbits = c->cflbits; a.do_cfl = (rk == 1); a.lin = lin ? 1 : 0; a.st = c->st;
     a.KC = (int)std::max(2L, std::min(16L, (long)(g.ny - 1) * (g.nz2 / c->fZR) / 592));
     a.P = c->P;
-    a.FZR = c->flux_zr;
+    a.FZR = flux_rows(c, !lin && !c->les_on);
     a.sc = c->scat;
     a.split = (c->mean_split && !lin && !c->les_on) ? 1 : 0;
     a.XZB = c->xinv_zb;
@@ -1524,7 +1545,8 @@ int cfg_set_les(cfg_ctx* c, const cfg_les* l) {
     return CFG_OK;
   }
   if (l->model != 1 && l->model != 2) return fail(c, CFG_E_ARG, "cfg_set_les: model %d", l->model);
-  if (!c->split_x) return fail(c, CFG_E_ARG, "cfg_set_les: needs the register-FFT x stage (nx2 of 24 .. 576)");
+  if (!c->split_x || !c->full_len)
+    return fail(c, CFG_E_ARG, "cfg_set_les: needs the register-FFT x stage (nx2 of 24 .. 576)");
   if (l->model == 2 && !l->mlp) return fail(c, CFG_E_ARG, "cfg_set_les: model 2 needs the network");
   if (!(l->cs >= 0.0) || !(l->aplus > 0.0) || !(l->beta >= 0.0)) return fail(c, CFG_E_ARG, "cfg_set_les: cs, aplus, beta");
   for (int i = 0; i < 10; ++i)
@@ -2356,7 +2378,7 @@ int cfg_group_create(const cfg_params* p, const cfg_grid* gr, int nranks, const 
     int r = create_impl(&pi, gr, &sp, &G->r[i]);
     if (r) { cfg_group_destroy(G); return r; }
     cfg_ctx* c = G->r[i];
-    if (n > 1 && !(c->split_x && c->fast_z)) {
+    if (n > 1 && !(c->split_x && c->fast_z && c->full_len && regfft_full(p->nz2))) {
       fprintf(stderr, "cfg_group_create: transform lengths %d x %d have no register-FFT kernels\n", p->nx2, p->nz2);
       cfg_group_destroy(G);
       return CFG_E_ARG;
@@ -2480,7 +2502,7 @@ int cfg_rank_create(const cfg_params* p, const cfg_grid* gr, int rank, int nrank
   SlabPart sp{rank, nranks, xs[rank], nxp[rank], zs[rank], nzp[rank]};
   int r = create_impl(p, gr, &sp, out);
   if (r) return r;
-  if (nranks > 1 && !((*out)->split_x && (*out)->fast_z)) {
+  if (nranks > 1 && !((*out)->split_x && (*out)->fast_z && (*out)->full_len && regfft_full(p->nz2))) {
     fprintf(stderr, "cfg_rank_create: transform lengths %d x %d have no register-FFT kernels\n", p->nx2, p->nz2);
     cfg_destroy(*out);
     *out = nullptr;
@@ -2702,7 +2724,7 @@ int cfg_set_tiles(cfg_ctx* c, const int* tiles) {
   if (!c || !tiles) return CFG_E_ARG;
   const int w = tiles[0], fz = tiles[1], y1 = tiles[2], y3 = tiles[3];
   if (w < 1 || w > 4 || (fz != 2 && fz != 4 && !(fz == 8 && c->mixed)) || y1 < 1 || y1 > 8 || y3 < 1 || y3 > 8 ||
-      (c->split_x && c->gP.nz2 % fz != 0))
+      (c->split_x && c->full_len && c->gP.nz2 % fz != 0))
     return fail(c, CFG_E_ARG, "cfg_set_tiles: unsupported tiles");
   c->rhs2_warps = w;
   c->flux_zr = fz;
@@ -2890,7 +2912,8 @@ void cfg_ensemble_destroy(cfg_ensemble* e) {
 
 // whether a member's step can run in the batched layout
 static bool ens_batchable(const cfg_ctx* c) {
-  return c->mixed && c->nranks == 1 && c->g.kx0 == 0 && c->split_x && c->fast_z && c->use_rhs2 && c->rhs2_tbl64 &&
+  return c->mixed && c->nranks == 1 && c->g.kx0 == 0 && c->split_x && c->fast_z && c->full_len &&
+         regfft_full(c->g.nz2) && c->use_rhs2 && c->rhs2_tbl64 &&
          c->n_fast > 0 && !c->les_on && c->p.ctrlu == 0.0 && c->p.ctrlw == 0.0 && !c->prof_on;
 }
 

@@ -1,6 +1,6 @@
 // pass1_reg.cuh -- the pass-1 kernels of pass1.cuh (same arithmetic, same
 // layouts) built on the register-resident two-stage FFTs of regfft.cuh for the
-// hot-path lengths (48 ... 576).  See pass1.cuh for what each kernel computes
+// hot-path lengths (24 ... 576).  See pass1.cuh for what each kernel computes
 // and which reference routine it replaces.
 #pragma once
 #include <type_traits>
@@ -558,13 +558,20 @@ __global__ void __launch_bounds__(256) k_xflux_r(const cplx_t<T>* __restrict__ T
 // ahead there.
 template <int N> struct FluxSeqPad;
 template <> struct FluxSeqPad<24> { static constexpr int D = 10; };
+template <> struct FluxSeqPad<36> { static constexpr int D = 0; };
 template <> struct FluxSeqPad<48> { static constexpr int D = 0; };
+template <> struct FluxSeqPad<54> { static constexpr int D = 13; };
 template <> struct FluxSeqPad<72> { static constexpr int D = 2; };
 template <> struct FluxSeqPad<96> { static constexpr int D = 0; };
+template <> struct FluxSeqPad<108> { static constexpr int D = 1; };
 template <> struct FluxSeqPad<144> { static constexpr int D = 0; };
+template <> struct FluxSeqPad<162> { static constexpr int D = 5; };
 template <> struct FluxSeqPad<192> { static constexpr int D = 12; };
+template <> struct FluxSeqPad<216> { static constexpr int D = 2; };
 template <> struct FluxSeqPad<288> { static constexpr int D = 4; };
+template <> struct FluxSeqPad<324> { static constexpr int D = 12; };
 template <> struct FluxSeqPad<384> { static constexpr int D = 8; };
+template <> struct FluxSeqPad<432> { static constexpr int D = 10; };
 template <> struct FluxSeqPad<576> { static constexpr int D = 0; };
 template <typename T, int N> struct FluxSeq {
   static constexpr bool ROWMAJOR = sizeof(T) == 8 && (N == 384 || N == 576);
@@ -592,37 +599,40 @@ template <typename T, int ZB> struct RawPitch {
   static constexpr int V = ZB + 16 / (int)sizeof(cplx_t<T>);
 };
 
-// k_xinv_r: grid (nz2/ZB, 3, ny+1), block xinv_threads (one thread per
+// k_xinv_r: grid (ceil(nz2/ZB), 3, ny+1), block xinv_threads (one thread per
 // stage-1 task, at least 128).  Inverse x transform of ZB
 // hybrid rows (one plane, one component) into physical rows, two real rows per
 // complex FFT (the x part of xz_fft_complex_to_real_parallel,
 // PFC/transform.f90:345-368).  v of plane ny+1 is not formed: no flux reads it.
+// The last block of an nz2 that ZB does not divide (nz2 is even) takes the
+// rows that are left.
 template <typename T, int NX2, int ZB>
 __device__ __forceinline__ void k_xinv_r_body(const uint3 bid, const cplx_t<T>* __restrict__ T1, T* __restrict__ P,
                                               Geom g, const cplx_t<T>* __restrict__ twx) {
   using C = cplx_t<T>;
   constexpr int N1 = Split<NX2>::N1, N2 = Split<NX2>::N2, PITCH = N2 + 1, SEQ = SeqPitch<NX2>::V;
-  constexpr int N = NX2, Nh = NX2 / 2, NS = ZB / 2, RP = RawPitch<T, ZB>::V;
+  constexpr int N = NX2, Nh = NX2 / 2, RP = RawPitch<T, ZB>::V;
   constexpr int CH = ZB * (int)sizeof(C) / 16;   // 16-byte chunks per hybrid row
   static_assert(ZB % 2 == 0 && (ZB * sizeof(C)) % 16 == 0, "ZB rows must pack in pairs and 16-byte chunks");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int NXH = g.nxh, NZ2 = g.nz2;
   C* tw = reinterpret_cast<C*>(smem_raw);   // [N]
   C* raw = tw + N;                          // [NXH][RP]
-  C* Y = raw + NXH * RP;                    // [NS][SEQ]
+  C* Y = raw + NXH * RP;                    // [ZB/2][SEQ]
   const int z0 = bid.x * ZB, c = bid.y, pl = bid.z;
   if (c == 1 && pl == g.ny) return;
+  const int rows = min(ZB, NZ2 - z0), ch = rows * (int)sizeof(C) / 16, ns = rows / 2;
   const C* src = T1 + ((size_t)pl * 3 + c) * NXH * NZ2 + z0;
   for (int idx = threadIdx.x; idx < NXH * CH; idx += blockDim.x) {
     const int kx = idx / CH, part = idx - kx * CH;
-    cp_async16(reinterpret_cast<char*>(raw + kx * RP) + part * 16,
+    if (part < ch) cp_async16(reinterpret_cast<char*>(raw + kx * RP) + part * 16,
                reinterpret_cast<const char*>(src + (size_t)kx * NZ2) + part * 16);
   }
   cp_async_commit();
   load_tw2<T, N>(tw, twx);
   cp_async_wait0();
   __syncthreads();
-  for (int t = threadIdx.x; t < NS * N2; t += blockDim.x) {
+  for (int t = threadIdx.x; t < ns * N2; t += blockDim.x) {
     const int i = t / N2, n2 = t - i * N2;
     C v[N1];
 #pragma unroll
@@ -650,7 +660,7 @@ __device__ __forceinline__ void k_xinv_r_body(const uint3 bid, const cplx_t<T>* 
     }
   }
   __syncthreads();
-  for (int t = threadIdx.x; t < NS * N1; t += blockDim.x) {
+  for (int t = threadIdx.x; t < ns * N1; t += blockDim.x) {
     const int q = t % N1, i = t / N1;
     C u[N2];
     const C* y = Y + i * SEQ + q * PITCH;

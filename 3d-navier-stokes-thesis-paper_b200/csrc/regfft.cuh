@@ -1,13 +1,13 @@
 // regfft.cuh -- register-resident FFTs for the hot-path transform lengths.
 //
-// A length N = N1*N2 transform (N1, N2 in {6, 8, 12, 16, 24}) runs in two
+// A length N = N1*N2 transform (N1, N2 in {4, 6, 8, 9, 12, 16, 18, 24}) runs in two
 // stages with one shared-memory exchange:
 //   stage 1: each thread owns one column n2, loads x[N2*n1 + n2] (n1 < N1),
 //            does an N1-point FFT in registers and applies W_N^(n2*k1);
 //   stage 2: each thread owns one row k1, does an N2-point FFT over n2 and
 //            produces X[k1 + N1*k2].
 // The small FFTs are compile-time mixed-radix compositions whose twiddles are
-// immediate constant-bank operands (W_48 table).  Sign -1 forward, +1 backward,
+// immediate constant-bank operands (W_144 table).  Sign -1 forward, +1 backward,
 // unnormalised, as FFTW.
 #pragma once
 #include <cmath>
@@ -16,43 +16,67 @@
 
 namespace cfd {
 
-// cos(2 pi m / 48) for m in [0, 12]: the quarter wave, correctly rounded
+// cos(2 pi m / 144) for m in [0, 36]: the quarter wave, correctly rounded
 // to FP64 (checked against 50-digit values).  Literals so that every twiddle
 // of the small FFTs folds to an immediate operand.
-__host__ __device__ __forceinline__ constexpr double cos48q(int m) {
+__host__ __device__ __forceinline__ constexpr double cos144q(int m) {
   return m == 0 ? 1.0
-         : m == 1 ? 0.9914448613738104
-         : m == 2 ? 0.9659258262890683
-         : m == 3 ? 0.9238795325112867
-         : m == 4 ? 0.8660254037844386
-         : m == 5 ? 0.7933533402912352
-         : m == 6 ? 0.7071067811865476
-         : m == 7 ? 0.6087614290087207
-         : m == 8 ? 0.5
-         : m == 9 ? 0.3826834323650898
-         : m == 10 ? 0.25881904510252074
-         : m == 11 ? 0.1305261922200516
+         : m == 1 ? 0.9990482215818578
+         : m == 2 ? 0.9961946980917455
+         : m == 3 ? 0.9914448613738104
+         : m == 4 ? 0.984807753012208
+         : m == 5 ? 0.9762960071199334
+         : m == 6 ? 0.9659258262890683
+         : m == 7 ? 0.9537169507482269
+         : m == 8 ? 0.9396926207859084
+         : m == 9 ? 0.9238795325112867
+         : m == 10 ? 0.9063077870366499
+         : m == 11 ? 0.8870108331782217
+         : m == 12 ? 0.8660254037844386
+         : m == 13 ? 0.8433914458128857
+         : m == 14 ? 0.8191520442889918
+         : m == 15 ? 0.7933533402912352
+         : m == 16 ? 0.766044443118978
+         : m == 17 ? 0.7372773368101241
+         : m == 18 ? 0.7071067811865476
+         : m == 19 ? 0.6755902076156602
+         : m == 20 ? 0.6427876096865394
+         : m == 21 ? 0.6087614290087207
+         : m == 22 ? 0.573576436351046
+         : m == 23 ? 0.5372996083468239
+         : m == 24 ? 0.5
+         : m == 25 ? 0.4617486132350339
+         : m == 26 ? 0.42261826174069944
+         : m == 27 ? 0.3826834323650898
+         : m == 28 ? 0.3420201433256687
+         : m == 29 ? 0.3007057995042731
+         : m == 30 ? 0.25881904510252074
+         : m == 31 ? 0.21643961393810288
+         : m == 32 ? 0.17364817766693036
+         : m == 33 ? 0.1305261922200516
+         : m == 34 ? 0.08715574274765818
+         : m == 35 ? 0.043619387365336
          : 0.0;
 }
 
-__host__ __device__ __forceinline__ constexpr double cos48_r(int r) {
-  return r <= 12 ? cos48q(r) : r <= 24 ? -cos48q(24 - r) : r <= 36 ? -cos48q(r - 24) : cos48q(48 - r);
+__host__ __device__ __forceinline__ constexpr double cos144_r(int r) {
+  return r <= 36 ? cos144q(r) : r <= 72 ? -cos144q(72 - r) : r <= 108 ? -cos144q(r - 72) : cos144q(144 - r);
 }
 
-// cos(2 pi m / 48) for any m, from the quarter wave by the symmetries
+// cos(2 pi m / 144) for any m, from the quarter wave by the symmetries
 // cos(pi - a) = -cos(a) and cos(2 pi - a) = cos(a): every entry is the
-// correctly rounded value, exact zeros at m = 12, 36 and exact halves.
-__host__ __device__ __forceinline__ constexpr double cos48(int m) {
-  return cos48_r(((m % 48) + 48) % 48);
+// correctly rounded value, exact zeros at m = 36, 108 and exact halves.
+__host__ __device__ __forceinline__ constexpr double cos144(int m) {
+  return cos144_r(((m % 144) + 144) % 144);
 }
 
 // W_N^(m) with the transform sign: sign -1 -> exp(-2 pi i m/N), +1 -> conjugate
 template <typename T, int N, int SIGN>
 __host__ __device__ __forceinline__ cplx_t<T> wconst(int m) {
-  static_assert(48 % N == 0, "small FFT length must divide 48");
-  const int q = (m % N) * (48 / N);
-  // exp(-2 pi i q/48) = cos - i sin, sin(a) = cos(a - pi/2) = cos48(q - 12)
-  return mk<cplx_t<T>>((T)cos48(q), (T)(SIGN > 0 ? 1.0 : -1.0) * (T)cos48((q + 36) % 48));
+  static_assert(144 % N == 0, "small FFT length must divide 144");
+  const int q = (m % N) * (144 / N);
+  // exp(-2 pi i q/144) = cos - i sin, sin(a) = cos(a - pi/2) = cos144(q - 36)
+  return mk<cplx_t<T>>((T)cos144(q), (T)(SIGN > 0 ? 1.0 : -1.0) * (T)cos144((q + 108) % 144));
 }
 
 template <typename C, int SIGN>
@@ -66,12 +90,12 @@ __host__ __device__ __forceinline__ C mul_i(C a) {   // (SIGN * i) * a
 template <typename T, int N, int SIGN>
 __host__ __device__ __forceinline__ cplx_t<T> twmul(cplx_t<T> x, int m) {
   using C = cplx_t<T>;
-  const int q = (m % N) * (48 / N);
+  const int q = (m % N) * (144 / N);
   if (q == 0) return x;
-  if (q == 24) return mk<C>(-x.x, -x.y);
-  // W = cos(2 pi q/48) + i SIGN sin(2 pi q/48): SIGN i at q = 12, -SIGN i at 36
-  if (q == 12) return mul_i<C, SIGN>(x);
-  if (q == 36) return mul_i<C, -SIGN>(x);
+  if (q == 72) return mk<C>(-x.x, -x.y);
+  // W = cos(2 pi q/144) + i SIGN sin(2 pi q/144): SIGN i at q = 36, -SIGN i at 108
+  if (q == 36) return mul_i<C, SIGN>(x);
+  if (q == 108) return mul_i<C, -SIGN>(x);
   return cmul(x, wconst<T, N, SIGN>(m));
 }
 
@@ -145,23 +169,44 @@ template <typename T, int P, int Q, int SIGN> struct Composite {
 
 template <typename T, int SIGN> struct SmallFFT<T, 6, SIGN> : Composite<T, 2, 3, SIGN> {};
 template <typename T, int SIGN> struct SmallFFT<T, 8, SIGN> : Composite<T, 2, 4, SIGN> {};
+template <typename T, int SIGN> struct SmallFFT<T, 9, SIGN> : Composite<T, 3, 3, SIGN> {};
 template <typename T, int SIGN> struct SmallFFT<T, 12, SIGN> : Composite<T, 4, 3, SIGN> {};
 template <typename T, int SIGN> struct SmallFFT<T, 16, SIGN> : Composite<T, 4, 4, SIGN> {};
+// (2-point FFTs first: on random rows of 324 points 20 % less rounding than 2 x 9)
+template <typename T, int SIGN> struct SmallFFT<T, 18, SIGN> : Composite<T, 9, 2, SIGN> {};
 template <typename T, int SIGN> struct SmallFFT<T, 24, SIGN> : Composite<T, 8, 3, SIGN> {};
 
 // Two-stage factorisation of the supported transform lengths.
 template <int N> struct Split;
 template <> struct Split<24> { static constexpr int N1 = 4, N2 = 6; };
+template <> struct Split<36> { static constexpr int N1 = 6, N2 = 6; };
 template <> struct Split<48> { static constexpr int N1 = 8, N2 = 6; };
+template <> struct Split<54> { static constexpr int N1 = 6, N2 = 9; };
 template <> struct Split<72> { static constexpr int N1 = 12, N2 = 6; };
 template <> struct Split<96> { static constexpr int N1 = 12, N2 = 8; };
+template <> struct Split<108> { static constexpr int N1 = 12, N2 = 9; };
 template <> struct Split<144> { static constexpr int N1 = 12, N2 = 12; };
+template <> struct Split<162> { static constexpr int N1 = 18, N2 = 9; };
 template <> struct Split<192> { static constexpr int N1 = 16, N2 = 12; };
+template <> struct Split<216> { static constexpr int N1 = 18, N2 = 12; };
 template <> struct Split<288> { static constexpr int N1 = 24, N2 = 12; };
+template <> struct Split<324> { static constexpr int N1 = 18, N2 = 18; };
 template <> struct Split<384> { static constexpr int N1 = 16, N2 = 24; };
+template <> struct Split<432> { static constexpr int N1 = 24, N2 = 18; };
 template <> struct Split<576> { static constexpr int N1 = 24, N2 = 24; };
 
+// Every 2^a 3^b length of 3/2-dealiased grids from 16 to 384 points: the
+// shared-memory Stockham passes (fft.cuh) read and write a sequence once per
+// radix and take 2.1 ms for a step at 144x100x108 (lengths 216 and 162) that
+// takes 0.67 ms here.
 __host__ __device__ constexpr bool regfft_supported(int n) {
+  return n == 24 || n == 36 || n == 48 || n == 54 || n == 72 || n == 96 || n == 108 || n == 144 || n == 162 || n == 192 ||
+         n == 216 || n == 288 || n == 324 || n == 384 || n == 432 || n == 576;
+}
+
+// The lengths of the slab ranks, the LES mode and the batched ensembles; the
+// others (36, 54, 108, 162, 216, 324, 432) serve the single-context step.
+__host__ __device__ constexpr bool regfft_full(int n) {
   return n == 24 || n == 48 || n == 72 || n == 96 || n == 144 || n == 192 || n == 288 || n == 384 || n == 576;
 }
 
