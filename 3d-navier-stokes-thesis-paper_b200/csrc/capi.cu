@@ -126,8 +126,8 @@ struct cfg_ctx {
   cudaStream_t st = nullptr;
   // side stream: the small mean-mode and FP64 low-|k| solves run beside the
   // main per-wavenumber kernel; joined back with events
-  cudaStream_t st2 = nullptr, st3 = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_join3 = nullptr;
+  cudaStream_t st2 = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   // background file output (restart file, VTK snapshot): the layout kernel
   // runs on st, the copy to pinned host memory on st_io, the file write on
   // io_thread
@@ -171,9 +171,8 @@ struct cfg_ctx {
   double* l2acc = nullptr;
   unsigned long long* divbits = nullptr;
   // lane-major grid coefficients of k_rhs2 (storage precision, rhs2_lanes
-  // lanes) and in FP64 for 32 lanes (the FP64 list and the mean mode)
+  // lanes)
   void* rhs2_tbl = nullptr;
-  void* rhs2_tbl64 = nullptr;
   // crossflow jet (cfg_set_jet): parameters, device walk state
   bool crossflow = false;
   JetParams jp{};
@@ -672,33 +671,30 @@ struct Impl {
     return les_stresses(c, F);
   }
 
-  // launch records of k_rhs2: the fast list (storage precision) or, prec,
-  // the mixed path's |k| < 4 list in FP64 on the side stream st2
-  static Rhs2Launch rhs2_args(const cfg_ctx* c, int rk, bool prec) {
+  // launch record of k_rhs2: the fast list
+  static Rhs2Launch rhs2_args(const cfg_ctx* c, int rk) {
     const Geom& g = c->g;
     Rhs2Launch a{};
     a.vel = c->vel; a.cru = c->cru; a.prs = c->prs;
     a.cbc_top = (const C*)c->cbc + 3 * (size_t)g.nw; a.cbc_bot = c->cbc;
     a.g = g; a.gd = c->gd; a.sc = c->sc; a.rkt = c->rkt; a.rk = rk; a.re = c->p.re;
-    if (prec) {
-      a.wlist = c->wl_prec; a.nlist = c->n_prec; a.warps = 1; a.lanes = 32; a.tbl = c->rhs2_tbl64;
-      a.st = c->st2;
-    } else {
-      a.wlist = c->wl_fast; a.nlist = c->n_fast; a.warps = c->rhs2_warps; a.lanes = c->rhs2_lanes;
-      a.tbl = c->rhs2_tbl;
-      a.st = c->st;
-    }
+    a.wlist = c->wl_fast; a.nlist = c->n_fast; a.warps = c->rhs2_warps; a.lanes = c->rhs2_lanes;
+    a.tbl = c->rhs2_tbl;
+    a.st = c->st;
     return a;
   }
-  // launch record of the mean mode (k_rhs_mean2) on the side stream st3
-  static RhsMeanLaunch mean_args(const cfg_ctx* c, int rk) {
+  // launch record of k_rhs_low on the side stream st2: the mean mode (on the
+  // rank that holds kx = 0) and the mixed path's |k| < 4 list
+  static RhsLowLaunch low_args(const cfg_ctx* c, int rk) {
     const Geom& g = c->g;
-    RhsMeanLaunch m{};
+    RhsLowLaunch m{};
     m.vel = c->vel; m.cru = c->cru; m.prs = c->prs; m.mvel64 = c->mvel64; m.mcru64 = c->mcru64;
     m.cbc_top = (const C*)c->cbc + 3 * (size_t)g.nw; m.cbc_bot = c->cbc;
     m.g = g; m.gd = c->gd; m.sc = c->sc; m.d_um_dy = c->d_um_dy; m.rkt = c->rkt; m.rk = rk;
-    m.re = c->p.re; m.beta = c->p.beta; m.fix_mass = c->p.fix_mass; m.tbl64 = (const double*)c->rhs2_tbl64;
-    m.st = c->st3;
+    m.re = c->p.re; m.beta = c->p.beta; m.fix_mass = c->p.fix_mass;
+    m.mean = g.kx0 == 0 ? 1 : 0;
+    m.wlist = c->wl_prec; m.nlist = c->n_prec;
+    m.st = c->st2;
     return m;
   }
 
@@ -710,45 +706,38 @@ struct Impl {
       const int r = jet(c, rk, 0.0, 0.0, 1);
       if (r) return r;
     }
-    // fork: the FP64 low-|k| list and the mean mode on two side streams, one
-    // warp per wavenumber so that they spread over many SMs beside the main
-    // kernel
+    // fork: the FP64 low-|k| list and the mean mode on a side stream, first in
+    // line so that they spread over the SMs beside the main kernel
     CK(cudaEventRecord(c->ev_fork, c->st));
     CK(cudaStreamWaitEvent(c->st2, c->ev_fork, 0));
-    CK(cudaStreamWaitEvent(c->st3, c->ev_fork, 0));
-    const bool v2 = c->use_rhs2 && c->rhs2_tbl64 && mode == 0;
-    if (c->n_prec > 0) {
-      c->prof_stream = c->st2;
-      prof_begin(c, "k_rhs_fp64");
-      if (v2 && sizeof(T) == 4) {
-        if (rhs2_launch_prec(rhs2_args(c, rk, true)) != 0) return fail(c, CFG_E_CUDA, "k_rhs2 (FP64 list) launch");
-      } else {
+    c->prof_stream = c->st2;
+    if (c->use_rhs2 && mode == 0) {
+      prof_begin(c, "k_rhs_low");
+      if (rhs_low_launch(sizeof(T) == 4, low_args(c, rk)) != 0) return fail(c, CFG_E_CUDA, "k_rhs_low launch");
+      CKL();
+    } else {
+      if (c->n_prec > 0) {
+        prof_begin(c, "k_rhs_fp64");
         k_rhs<double, T, MM><<<c->n_prec, 32, c->sm_rhs64 / 4, c->st2>>>((C*)c->vel, (C*)c->cru, (C*)c->prs,
                                                                        (const C*)c->cbc + 3 * (size_t)g.nw,
                                                                        (const C*)c->cbc, g, c->gd, c->sc, c->rkt, rk,
                                                                        c->p.re, mode, c->wl_prec, c->n_prec);
+        CKL();
       }
-      CKL();
+      if (g.kx0 == 0) {   // the mean mode lives on the rank that holds kx = 0
+        prof_begin(c, "k_rhs_mean");
+        k_rhs_mean<T, MM><<<1, 32, 0, c->st2>>>((C*)c->vel, (C*)c->cru, (C*)c->prs, c->mvel64, c->mcru64,
+                                               (const C*)c->cbc + 3 * (size_t)g.nw, (const C*)c->cbc, g, c->gd, c->sc,
+                                               c->d_um_dy, c->rkt, rk, c->p.re, c->p.beta, c->p.fix_mass, mode);
+        CKL();
+      }
     }
     if (mode == 0) c->mean64_valid = true;
-    c->prof_stream = c->st3;
-    prof_begin(c, "k_rhs_mean");
-    if (g.kx0 != 0) {
-      // the mean mode lives on the rank that holds kx = 0
-    } else if (v2) {
-      if (rhs_mean2_launch(sizeof(T) == 4, mean_args(c, rk)) != 0) return fail(c, CFG_E_CUDA, "k_rhs_mean2 launch");
-    } else {
-      k_rhs_mean<T, MM><<<1, 32, 0, c->st3>>>((C*)c->vel, (C*)c->cru, (C*)c->prs, c->mvel64, c->mcru64,
-                                             (const C*)c->cbc + 3 * (size_t)g.nw, (const C*)c->cbc, g, c->gd, c->sc,
-                                             c->d_um_dy, c->rkt, rk, c->p.re, c->p.beta, c->p.fix_mass, mode);
-    }
-    CKL();
     c->prof_stream = nullptr;
     CK(cudaEventRecord(c->ev_join, c->st2));
-    CK(cudaEventRecord(c->ev_join3, c->st3));
     if (c->n_fast > 0 && mode == 0 && c->use_rhs2) {
       prof_begin(c, "k_rhs");
-      if (rhs2_launch(sizeof(T) == 4, rhs2_args(c, rk, false)) != 0) return fail(c, CFG_E_CUDA, "k_rhs2 launch");
+      if (rhs2_launch(sizeof(T) == 4, rhs2_args(c, rk)) != 0) return fail(c, CFG_E_CUDA, "k_rhs2 launch");
       CKL();
     } else if (c->n_fast > 0) {
       dim3 gr((c->n_fast + 3) / 4);
@@ -760,7 +749,6 @@ struct Impl {
     }
     // join
     CK(cudaStreamWaitEvent(c->st, c->ev_join, 0));
-    CK(cudaStreamWaitEvent(c->st, c->ev_join3, 0));
     return CFG_OK;
   }
   static int rhs(cfg_ctx* c, int rk, int mode) {
@@ -987,8 +975,6 @@ static int create_impl(const cfg_params* p, const cfg_grid* gr, const SlabPart* 
   if (cudaSetDevice(c->dev) != cudaSuccess) { fail(c, CFG_E_CUDA, "cudaSetDevice"); delete c; return CFG_E_CUDA; }
   if (cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->st2, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaStreamCreateWithFlags(&c->st3, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaEventCreateWithFlags(&c->ev_join3, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess) {
     delete c;
@@ -1132,11 +1118,6 @@ static int create_impl(const cfg_params* p, const cfg_grid* gr, const SlabPart* 
     rhs2_table(c->mixed, ny, c->rhs2_lanes, gr->dh, gr->dn, gr->d2h, gr->d2n, ht.data());
     if (cudaMalloc(&c->rhs2_tbl, tb) != cudaSuccess) return bad(CFG_E_NOMEM);
     cudaMemcpy(c->rhs2_tbl, ht.data(), tb, cudaMemcpyHostToDevice);
-    const size_t tb64 = rhs2_table_bytes(false, g.ny1, 32);
-    std::vector<unsigned char> h64(tb64);
-    rhs2_table(false, ny, 32, gr->dh, gr->dn, gr->d2h, gr->d2n, h64.data());
-    if (cudaMalloc(&c->rhs2_tbl64, tb64) != cudaSuccess) return bad(CFG_E_NOMEM);
-    cudaMemcpy(c->rhs2_tbl64, h64.data(), tb64, cudaMemcpyHostToDevice);
   }
   if (cudaDeviceSynchronize() != cudaSuccess) return bad(CFG_E_CUDA);
   *out = c;
@@ -1160,7 +1141,7 @@ void cfg_destroy(cfg_ctx* c) {
   if (c->st_io) cudaStreamDestroy(c->st_io);
   for (void* q : c->ipc_open) cudaIpcCloseMemHandle(q);
   void* bufs[] = {c->dgrid, c->fringe, c->vel, c->cru, c->prs, c->mvel64, c->mcru64, c->T1, c->T2, c->P,
-                  c->rhs2_tbl, c->rhs2_tbl64, c->jst, c->pp_wy, c->pp_sy, c->pp_acc, c->cbc,
+                  c->rhs2_tbl, c->jst, c->pp_wy, c->pp_sy, c->pp_acc, c->cbc,
                   c->sc, c->d_um_dy, c->cflp, c->cflbits, c->l2acc, c->divbits, c->plist, c->pw_H,
                   c->pw_phys, c->pw_phys2, c->pw_in, c->stage, c->twx, c->twz, c->twxs, c->twzs,
                   c->wl_fast, c->wl_prec, c->scat_tab, c->cfl_peers, c->les_S, c->les_F, c->les_len,
@@ -1170,9 +1151,7 @@ void cfg_destroy(cfg_ctx* c) {
   for (cudaEvent_t e : c->ev_pool) cudaEventDestroy(e);
   if (c->ev_fork) cudaEventDestroy(c->ev_fork);
   if (c->ev_join) cudaEventDestroy(c->ev_join);
-  if (c->ev_join3) cudaEventDestroy(c->ev_join3);
   if (c->st2) cudaStreamDestroy(c->st2);
-  if (c->st3) cudaStreamDestroy(c->st3);
   if (c->st) cudaStreamDestroy(c->st);
   delete c;
 }
@@ -2850,18 +2829,18 @@ __global__ void k_jet_combine_b(const EnsJet* __restrict__ tab, unsigned gx) {
 // one class of a batched ensemble: members with the same grid and tiles
 struct EnsClass {
   std::vector<int> mem, jet;   // member indices; those with the wall jet
-  cudaStream_t st = nullptr, st2 = nullptr, st3 = nullptr;
-  cudaEvent_t ev_start = nullptr, ev_fork = nullptr, ev_j2 = nullptr, ev_j3 = nullptr, ev_done = nullptr;
+  cudaStream_t st = nullptr, st2 = nullptr;
+  cudaEvent_t ev_start = nullptr, ev_fork = nullptr, ev_j2 = nullptr, ev_done = nullptr;
   void* dtab = nullptr;        // every table below, one allocation
   P1Launch *zinv = nullptr, *xinv = nullptr, *zfwd = nullptr, *flux[3] = {};
-  Rhs2Launch *r2[3] = {}, *r2p[3] = {};
-  RhsMeanLaunch* rm[3] = {};
+  Rhs2Launch* r2[3] = {};
+  RhsLowLaunch* rl[3] = {};
   EnsMember* sm = nullptr;
   EnsJet* jt = nullptr;
   // the first member's records: launch shapes, on the class's streams
   P1Launch h_zinv{}, h_xinv{}, h_zfwd{}, h_flux[3] = {};
-  Rhs2Launch h_r2[3] = {}, h_r2p[3] = {};
-  RhsMeanLaunch h_rm[3] = {};
+  Rhs2Launch h_r2[3] = {};
+  RhsLowLaunch h_rl[3] = {};
   int nx = 0, nz = 0, nxh = 0, nx2 = 0, nz2 = 0;
   size_t ncbc = 0;
 };
@@ -2883,9 +2862,9 @@ struct cfg_ensemble {
 static void ens_free_classes(cfg_ensemble* e) {
   for (EnsClass& k : e->cls) {
     if (k.dtab) cudaFree(k.dtab);
-    for (cudaEvent_t v : {k.ev_start, k.ev_fork, k.ev_j2, k.ev_j3, k.ev_done})
+    for (cudaEvent_t v : {k.ev_start, k.ev_fork, k.ev_j2, k.ev_done})
       if (v) cudaEventDestroy(v);
-    for (cudaStream_t v : {k.st, k.st2, k.st3})
+    for (cudaStream_t v : {k.st, k.st2})
       if (v) cudaStreamDestroy(v);
   }
   e->cls.clear();
@@ -2913,7 +2892,7 @@ void cfg_ensemble_destroy(cfg_ensemble* e) {
 // whether a member's step can run in the batched layout
 static bool ens_batchable(const cfg_ctx* c) {
   return c->mixed && c->nranks == 1 && c->g.kx0 == 0 && c->split_x && c->fast_z && c->full_len &&
-         regfft_full(c->g.nz2) && c->use_rhs2 && c->rhs2_tbl64 &&
+         regfft_full(c->g.nz2) && c->use_rhs2 &&
          c->n_fast > 0 && !c->les_on && c->p.ctrlu == 0.0 && c->p.ctrlw == 0.0 && !c->prof_on;
 }
 
@@ -2948,15 +2927,15 @@ static int ens_build_classes(cfg_ensemble* e) {
     for (int i : k.mem)
       if (e->m[i]->crossflow) k.jet.push_back(i);
     bool ok = true;
-    for (cudaStream_t* v : {&k.st, &k.st2, &k.st3})
+    for (cudaStream_t* v : {&k.st, &k.st2})
       ok = ok && cudaStreamCreateWithFlags(v, cudaStreamNonBlocking) == cudaSuccess;
-    for (cudaEvent_t* v : {&k.ev_start, &k.ev_fork, &k.ev_j2, &k.ev_j3, &k.ev_done})
+    for (cudaEvent_t* v : {&k.ev_start, &k.ev_fork, &k.ev_j2, &k.ev_done})
       ok = ok && cudaEventCreateWithFlags(v, cudaEventDisableTiming) == cudaSuccess;
     if (!ok) return CFG_E_CUDA;
     const int n = (int)k.mem.size(), nj = (int)k.jet.size();
     std::vector<P1Launch> zinv(n), xinv(n), zfwd(n), flux(3 * n);
-    std::vector<Rhs2Launch> r2(3 * n), r2p(3 * n);
-    std::vector<RhsMeanLaunch> rm(3 * n);
+    std::vector<Rhs2Launch> r2(3 * n);
+    std::vector<RhsLowLaunch> rl(3 * n);
     std::vector<EnsMember> sm(n);
     std::vector<EnsJet> jt(nj);
     for (int q = 0; q < n; ++q) {
@@ -2966,9 +2945,8 @@ static int ens_build_classes(cfg_ensemble* e) {
       zfwd[q] = I::p1_args(c, 1, false, 2);
       for (int rk = 1; rk <= 3; ++rk) {
         flux[(rk - 1) * n + q] = I::p1_args(c, rk, false, 4);
-        r2[(rk - 1) * n + q] = I::rhs2_args(c, rk, false);
-        r2p[(rk - 1) * n + q] = I::rhs2_args(c, rk, true);
-        rm[(rk - 1) * n + q] = I::mean_args(c, rk);
+        r2[(rk - 1) * n + q] = I::rhs2_args(c, rk);
+        rl[(rk - 1) * n + q] = I::low_args(c, rk);
       }
       EnsMember& a = sm[q];
       a.m64 = c->mvel64;
@@ -3020,8 +2998,8 @@ static int ens_build_classes(cfg_ensemble* e) {
     };
     const size_t o_zinv = take(sizeof(P1Launch) * n), o_xinv = take(sizeof(P1Launch) * n),
                  o_zfwd = take(sizeof(P1Launch) * n), o_flux = take(sizeof(P1Launch) * 3 * n),
-                 o_r2 = take(sizeof(Rhs2Launch) * 3 * n), o_r2p = take(sizeof(Rhs2Launch) * 3 * n),
-                 o_rm = take(sizeof(RhsMeanLaunch) * 3 * n), o_sm = take(sizeof(EnsMember) * n),
+                 o_r2 = take(sizeof(Rhs2Launch) * 3 * n), o_rl = take(sizeof(RhsLowLaunch) * 3 * n),
+                 o_sm = take(sizeof(EnsMember) * n),
                  o_jt = take(sizeof(EnsJet) * (nj > 0 ? nj : 1));
     if (cudaMalloc(&k.dtab, off) != cudaSuccess) {
       cudaGetLastError();
@@ -3034,8 +3012,8 @@ static int ens_build_classes(cfg_ensemble* e) {
     };
     ok = put(o_zinv, zinv.data(), sizeof(P1Launch) * n) && put(o_xinv, xinv.data(), sizeof(P1Launch) * n) &&
          put(o_zfwd, zfwd.data(), sizeof(P1Launch) * n) && put(o_flux, flux.data(), sizeof(P1Launch) * 3 * n) &&
-         put(o_r2, r2.data(), sizeof(Rhs2Launch) * 3 * n) && put(o_r2p, r2p.data(), sizeof(Rhs2Launch) * 3 * n) &&
-         put(o_rm, rm.data(), sizeof(RhsMeanLaunch) * 3 * n) && put(o_sm, sm.data(), sizeof(EnsMember) * n) &&
+         put(o_r2, r2.data(), sizeof(Rhs2Launch) * 3 * n) && put(o_rl, rl.data(), sizeof(RhsLowLaunch) * 3 * n) &&
+         put(o_sm, sm.data(), sizeof(EnsMember) * n) &&
          put(o_jt, jt.data(), sizeof(EnsJet) * nj);
     if (!ok) return CFG_E_CUDA;
     k.zinv = (P1Launch*)(b + o_zinv);
@@ -3044,16 +3022,13 @@ static int ens_build_classes(cfg_ensemble* e) {
     for (int r = 0; r < 3; ++r) {
       k.flux[r] = (P1Launch*)(b + o_flux) + r * n;
       k.r2[r] = (Rhs2Launch*)(b + o_r2) + r * n;
-      k.r2p[r] = (Rhs2Launch*)(b + o_r2p) + r * n;
-      k.rm[r] = (RhsMeanLaunch*)(b + o_rm) + r * n;
+      k.rl[r] = (RhsLowLaunch*)(b + o_rl) + r * n;
       k.h_flux[r] = flux[r * n];
       k.h_flux[r].st = k.st;
       k.h_r2[r] = r2[r * n];
       k.h_r2[r].st = k.st;
-      k.h_r2p[r] = r2p[r * n];
-      k.h_r2p[r].st = k.st2;
-      k.h_rm[r] = rm[r * n];
-      k.h_rm[r].st = k.st3;
+      k.h_rl[r] = rl[r * n];
+      k.h_rl[r].st = k.st2;
     }
     k.sm = (EnsMember*)(b + o_sm);
     k.jt = (EnsJet*)(b + o_jt);
@@ -3118,21 +3093,13 @@ static int ens_class_enqueue(cfg_ensemble* e, EnsClass& k) {
     }
     // the FP64 |k| < 4 list and the mean mode beside the main kernel
     if (int r = ck(cudaEventRecord(k.ev_fork, k.st) == cudaSuccess &&
-                       cudaStreamWaitEvent(k.st2, k.ev_fork, 0) == cudaSuccess &&
-                       cudaStreamWaitEvent(k.st3, k.ev_fork, 0) == cudaSuccess,
+                       cudaStreamWaitEvent(k.st2, k.ev_fork, 0) == cudaSuccess,
                    "batched fork"))
       return r;
-    if (k.h_r2p[rk - 1].nlist > 0) {
-      if (int r = ck(rhs2_launch_prec_batch(k.h_r2p[rk - 1], k.r2p[rk - 1], n) == 0, "batched k_rhs2 (FP64 list)"))
-        return r;
-      ++launches;
-    }
-    if (int r = ck(rhs_mean2_launch_batch(true, k.h_rm[rk - 1], k.rm[rk - 1], n) == 0, "batched k_rhs_mean2")) return r;
+    if (int r = ck(rhs_low_launch_batch(true, k.h_rl[rk - 1], k.rl[rk - 1], n) == 0, "batched k_rhs_low")) return r;
     if (int r = ck(rhs2_launch_batch(true, k.h_r2[rk - 1], k.r2[rk - 1], n) == 0, "batched k_rhs2")) return r;
     launches += 2;
-    if (int r = ck(cudaEventRecord(k.ev_j2, k.st2) == cudaSuccess && cudaEventRecord(k.ev_j3, k.st3) == cudaSuccess &&
-                       cudaStreamWaitEvent(k.st, k.ev_j2, 0) == cudaSuccess &&
-                       cudaStreamWaitEvent(k.st, k.ev_j3, 0) == cudaSuccess,
+    if (int r = ck(cudaEventRecord(k.ev_j2, k.st2) == cudaSuccess && cudaStreamWaitEvent(k.st, k.ev_j2, 0) == cudaSuccess,
                    "batched join"))
       return r;
   }

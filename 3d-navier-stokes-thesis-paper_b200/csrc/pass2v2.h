@@ -26,17 +26,14 @@ struct Rhs2Launch {
 
 // 0 on success, -1 unsupported size, -2 launch error
 int rhs2_launch(bool f32, const Rhs2Launch& a);
-// the mixed path's |k| < 4 list: FP64 arithmetic over FP32 storage, tbl the
-// FP64 table for 32 lanes
-int rhs2_launch_prec(const Rhs2Launch& a);
-// the same kernels for nmem members of one grid in one launch: tab is the
+// the same kernel for nmem members of one grid in one launch: tab is the
 // members' launch records in device memory, a the first member's (host)
 // copy, which sets the launch shape and stream
 int rhs2_launch_batch(bool f32, const Rhs2Launch& a, const Rhs2Launch* tab, int nmem);
-int rhs2_launch_prec_batch(const Rhs2Launch& a, const Rhs2Launch* tab, int nmem);
 
-// the mean mode (k_rhs_mean2)
-struct RhsMeanLaunch {
+// the mean mode and, in mixed precision, the |k| < 4 list, in FP64 over the
+// stored state (k_rhs_low, pass2low.cuh)
+struct RhsLowLaunch {
   void *vel, *cru, *prs;
   double2 *mvel64, *mcru64;   // FP64 mean columns (mixed), or null
   const void *cbc_top, *cbc_bot;
@@ -48,11 +45,13 @@ struct RhsMeanLaunch {
   int rk;
   double re, beta;
   int fix_mass;
-  const double* tbl64;        // FP64 coefficient table for 32 lanes
+  int mean;                   // 1: this rank holds the mean mode
+  const int* wlist;
+  int nlist;
   cudaStream_t st;
 };
-int rhs_mean2_launch(bool f32, const RhsMeanLaunch& a);
-int rhs_mean2_launch_batch(bool f32, const RhsMeanLaunch& a, const RhsMeanLaunch* tab, int nmem);
+int rhs_low_launch(bool f32, const RhsLowLaunch& a);
+int rhs_low_launch_batch(bool f32, const RhsLowLaunch& a, const RhsLowLaunch* tab, int nmem);
 bool rhs2_supported(int ny1);
 // the lane-major grid-coefficient table the kernel reads (host side)
 size_t rhs2_table_bytes(bool f32, int ny1, int lanes);

@@ -785,11 +785,11 @@ def run_ours(args):
             lo, hi = prof.pop("k_zfwd_low"), prof["k_zfwd"]
             prof["k_zfwd"] = (hi[0], hi[1] + lo[1])
         kp = mix["prof_steps"]
-        tot_prof = sum(v[1] for k, v in prof.items() if k not in ("k_rhs_fp64", "k_rhs_mean")) or 1.0
+        tot_prof = sum(v[1] for k, v in prof.items() if k not in ("k_rhs_low", "k_rhs_fp64", "k_rhs_mean")) or 1.0
         kernels = {}
         for k, v in prof.items():
             ent = {"launches": v[0], "ms_per_launch": v[1] / max(v[0], 1)}
-            if k in ("k_rhs_fp64", "k_rhs_mean"):
+            if k in ("k_rhs_low", "k_rhs_fp64", "k_rhs_mean"):
                 ent["note"] = "side stream, overlaps k_rhs: wall time from its fork, not a serial share"
             else:
                 ent["share"] = v[1] / tot_prof
