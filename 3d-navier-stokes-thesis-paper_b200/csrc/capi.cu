@@ -126,8 +126,8 @@ struct cfg_ctx {
   cudaStream_t st = nullptr;
   // side stream: the small mean-mode and FP64 low-|k| solves run beside the
   // main per-wavenumber kernel; joined back with events
-  cudaStream_t st2 = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  cudaStream_t st2 = nullptr, st3 = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_join3 = nullptr;
   // background file output (restart file, VTK snapshot): the layout kernel
   // runs on st, the copy to pinned host memory on st_io, the file write on
   // io_thread
@@ -171,8 +171,9 @@ struct cfg_ctx {
   double* l2acc = nullptr;
   unsigned long long* divbits = nullptr;
   // lane-major grid coefficients of k_rhs2 (storage precision, rhs2_lanes
-  // lanes)
+  // lanes) and in FP64 for 32 lanes (step_keeps_sums)
   void* rhs2_tbl = nullptr;
+  void* rhs2_tbl64 = nullptr;
   // crossflow jet (cfg_set_jet): parameters, device walk state
   bool crossflow = false;
   JetParams jp{};
@@ -207,6 +208,7 @@ struct cfg_ctx {
   bool full_len = false;   // nx2 of regfft_full and nz2 rows in eights (the LES mode)
   bool use_rhs2 = true;
   int rhs2_lanes = 32;
+  bool rhs_rows = false;  // small grid: every wavenumber in k_rhs_rows, one launch
   int rhs2_warps = 3;   // warps (wavenumbers) per k_rhs2 block
   int fYB1 = 1, fYB3 = 1, fZR = 1;
   int xinv_zb = 0;      // z2 rows per k_xinv_r block (0: 16 in FP32, 8 in FP64), tuned
@@ -486,6 +488,16 @@ struct Impl {
       if (l == 32 || (l == 16 && g.ny1 <= 256) || (l == 8 && g.ny1 <= 64)) c->rhs2_lanes = l;
     }
     c->rhs2_warps = f32 ? 3 : 2;
+    // a thread per row (k_rhs_rows) for every wavenumber up to 512 rows per
+    // SM, what its registers let an SM hold at once: beyond one wave its
+    // extra (FP64) operations cost more than k_rhs2's unfilled SMs (us per
+    // step, k_rhs2 / k_rhs_rows, mixed: 32x33x32 133 / 120, 32x65x32 145 /
+    // 132, 48x49x48 175 / 173, 64x33x64 161 / 180, 96x97x96 385 / 552; FP64:
+    // 126 / 119, 148 / 136, 180 / 190, 213 / 201, 755 / 749).
+    // The whole grid's count, so that the ranks of a group solve as one
+    // context does.  CHANFLOW_RHS_ROWS=0|1 overrides.
+    c->rhs_rows = c->use_rhs2 && (size_t)g.nz * g.nxh_all * ((g.ny1 + 31) / 32 * 32) <= 148 * 512;
+    if (getenv("CHANFLOW_RHS_ROWS")) c->rhs_rows = c->use_rhs2 && atoi(getenv("CHANFLOW_RHS_ROWS"));
     c->twx = make_twiddles<T>(g.nx2);
     c->twz = make_twiddles<T>(g.nz2);
     c->twxs = make_twiddles<T>(g.nx);
@@ -671,30 +683,57 @@ struct Impl {
     return les_stresses(c, F);
   }
 
-  // launch record of k_rhs2: the fast list
-  static Rhs2Launch rhs2_args(const cfg_ctx* c, int rk) {
+  // The learned closure chooses per point between the network and the eddy
+  // viscosity: a last-bit difference in the state flips points, and forty
+  // steps later the states differ by 2e-5 (measured, against 3e-7 with the
+  // eddy viscosity).  So that its runs repeat earlier ones bit for bit, a
+  // step with it keeps the summation order of its solves: the FP64 list and
+  // the mean mode by k_rhs2's partition method, a warp per wavenumber.
+  static bool step_keeps_sums(const cfg_ctx* c) { return c->les_on && c->les.model == 2; }
+
+  // launch records of k_rhs2: the fast list (storage precision) or, prec,
+  // the mixed path's |k| < 4 list in FP64 on the side stream st2
+  static Rhs2Launch rhs2_args(const cfg_ctx* c, int rk, bool prec) {
     const Geom& g = c->g;
     Rhs2Launch a{};
     a.vel = c->vel; a.cru = c->cru; a.prs = c->prs;
     a.cbc_top = (const C*)c->cbc + 3 * (size_t)g.nw; a.cbc_bot = c->cbc;
     a.g = g; a.gd = c->gd; a.sc = c->sc; a.rkt = c->rkt; a.rk = rk; a.re = c->p.re;
-    a.wlist = c->wl_fast; a.nlist = c->n_fast; a.warps = c->rhs2_warps; a.lanes = c->rhs2_lanes;
-    a.tbl = c->rhs2_tbl;
-    a.st = c->st;
+    if (prec) {
+      a.wlist = c->wl_prec; a.nlist = c->n_prec; a.warps = 1; a.lanes = 32; a.tbl = c->rhs2_tbl64;
+      a.st = c->st2;
+    } else {
+      a.wlist = c->wl_fast; a.nlist = c->n_fast; a.warps = c->rhs2_warps; a.lanes = c->rhs2_lanes;
+      a.tbl = c->rhs2_tbl;
+      a.st = c->st;
+    }
     return a;
   }
-  // launch record of k_rhs_low on the side stream st2: the mean mode (on the
-  // rank that holds kx = 0) and the mixed path's |k| < 4 list
-  static RhsLowLaunch low_args(const cfg_ctx* c, int rk) {
+  // launch record of the mean mode (k_rhs_mean2) on the side stream st3
+  static RhsMeanLaunch mean_args(const cfg_ctx* c, int rk) {
     const Geom& g = c->g;
-    RhsLowLaunch m{};
+    RhsMeanLaunch m{};
+    m.vel = c->vel; m.cru = c->cru; m.prs = c->prs; m.mvel64 = c->mvel64; m.mcru64 = c->mcru64;
+    m.cbc_top = (const C*)c->cbc + 3 * (size_t)g.nw; m.cbc_bot = c->cbc;
+    m.g = g; m.gd = c->gd; m.sc = c->sc; m.d_um_dy = c->d_um_dy; m.rkt = c->rkt; m.rk = rk;
+    m.re = c->p.re; m.beta = c->p.beta; m.fix_mass = c->p.fix_mass; m.tbl64 = (const double*)c->rhs2_tbl64;
+    m.st = c->st3;
+    return m;
+  }
+  // launch record of k_rhs_rows: the mean mode (on the rank that holds
+  // kx = 0) and the mixed path's |k| < 4 list on the side stream st2; all
+  // wavenumbers on st where the grid is small (rhs_rows)
+  static RhsRowsLaunch rows_args(const cfg_ctx* c, int rk) {
+    const Geom& g = c->g;
+    RhsRowsLaunch m{};
     m.vel = c->vel; m.cru = c->cru; m.prs = c->prs; m.mvel64 = c->mvel64; m.mcru64 = c->mcru64;
     m.cbc_top = (const C*)c->cbc + 3 * (size_t)g.nw; m.cbc_bot = c->cbc;
     m.g = g; m.gd = c->gd; m.sc = c->sc; m.d_um_dy = c->d_um_dy; m.rkt = c->rkt; m.rk = rk;
     m.re = c->p.re; m.beta = c->p.beta; m.fix_mass = c->p.fix_mass;
     m.mean = g.kx0 == 0 ? 1 : 0;
     m.wlist = c->wl_prec; m.nlist = c->n_prec;
-    m.st = c->st2;
+    m.wfast = c->wl_fast; m.nfast = c->rhs_rows ? c->n_fast : 0;
+    m.st = c->rhs_rows ? c->st : c->st2;
     return m;
   }
 
@@ -706,14 +745,37 @@ struct Impl {
       const int r = jet(c, rk, 0.0, 0.0, 1);
       if (r) return r;
     }
+    const bool keep = c->use_rhs2 && mode == 0 && step_keeps_sums(c);
+    if (c->rhs_rows && mode == 0 && !keep) {
+      prof_begin(c, "k_rhs");
+      if (rhs_rows_launch(sizeof(T) == 4, rows_args(c, rk)) != 0) return fail(c, CFG_E_CUDA, "k_rhs_rows launch");
+      CKL();
+      c->mean64_valid = true;
+      return CFG_OK;
+    }
     // fork: the FP64 low-|k| list and the mean mode on a side stream, first in
     // line so that they spread over the SMs beside the main kernel
     CK(cudaEventRecord(c->ev_fork, c->st));
     CK(cudaStreamWaitEvent(c->st2, c->ev_fork, 0));
     c->prof_stream = c->st2;
-    if (c->use_rhs2 && mode == 0) {
+    if (keep) {
+      if (c->n_prec > 0) {
+        prof_begin(c, "k_rhs_fp64");
+        if (rhs2_launch_prec(rhs2_args(c, rk, true)) != 0) return fail(c, CFG_E_CUDA, "k_rhs2 (FP64 list) launch");
+        CKL();
+      }
+      if (g.kx0 == 0) {
+        CK(cudaStreamWaitEvent(c->st3, c->ev_fork, 0));
+        c->prof_stream = c->st3;
+        prof_begin(c, "k_rhs_mean");
+        if (rhs_mean2_launch(sizeof(T) == 4, mean_args(c, rk)) != 0) return fail(c, CFG_E_CUDA, "k_rhs_mean2 launch");
+        CKL();
+        CK(cudaEventRecord(c->ev_join3, c->st3));
+        CK(cudaStreamWaitEvent(c->st2, c->ev_join3, 0));
+      }
+    } else if (c->use_rhs2 && mode == 0) {
       prof_begin(c, "k_rhs_low");
-      if (rhs_low_launch(sizeof(T) == 4, low_args(c, rk)) != 0) return fail(c, CFG_E_CUDA, "k_rhs_low launch");
+      if (rhs_rows_launch(sizeof(T) == 4, rows_args(c, rk)) != 0) return fail(c, CFG_E_CUDA, "k_rhs_rows launch");
       CKL();
     } else {
       if (c->n_prec > 0) {
@@ -737,7 +799,7 @@ struct Impl {
     CK(cudaEventRecord(c->ev_join, c->st2));
     if (c->n_fast > 0 && mode == 0 && c->use_rhs2) {
       prof_begin(c, "k_rhs");
-      if (rhs2_launch(sizeof(T) == 4, rhs2_args(c, rk)) != 0) return fail(c, CFG_E_CUDA, "k_rhs2 launch");
+      if (rhs2_launch(sizeof(T) == 4, rhs2_args(c, rk, false)) != 0) return fail(c, CFG_E_CUDA, "k_rhs2 launch");
       CKL();
     } else if (c->n_fast > 0) {
       dim3 gr((c->n_fast + 3) / 4);
@@ -975,6 +1037,8 @@ static int create_impl(const cfg_params* p, const cfg_grid* gr, const SlabPart* 
   if (cudaSetDevice(c->dev) != cudaSuccess) { fail(c, CFG_E_CUDA, "cudaSetDevice"); delete c; return CFG_E_CUDA; }
   if (cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->st2, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&c->st3, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&c->ev_join3, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess) {
     delete c;
@@ -1118,6 +1182,11 @@ static int create_impl(const cfg_params* p, const cfg_grid* gr, const SlabPart* 
     rhs2_table(c->mixed, ny, c->rhs2_lanes, gr->dh, gr->dn, gr->d2h, gr->d2n, ht.data());
     if (cudaMalloc(&c->rhs2_tbl, tb) != cudaSuccess) return bad(CFG_E_NOMEM);
     cudaMemcpy(c->rhs2_tbl, ht.data(), tb, cudaMemcpyHostToDevice);
+    const size_t tb64 = rhs2_table_bytes(false, g.ny1, 32);
+    std::vector<unsigned char> h64(tb64);
+    rhs2_table(false, ny, 32, gr->dh, gr->dn, gr->d2h, gr->d2n, h64.data());
+    if (cudaMalloc(&c->rhs2_tbl64, tb64) != cudaSuccess) return bad(CFG_E_NOMEM);
+    cudaMemcpy(c->rhs2_tbl64, h64.data(), tb64, cudaMemcpyHostToDevice);
   }
   if (cudaDeviceSynchronize() != cudaSuccess) return bad(CFG_E_CUDA);
   *out = c;
@@ -1141,7 +1210,7 @@ void cfg_destroy(cfg_ctx* c) {
   if (c->st_io) cudaStreamDestroy(c->st_io);
   for (void* q : c->ipc_open) cudaIpcCloseMemHandle(q);
   void* bufs[] = {c->dgrid, c->fringe, c->vel, c->cru, c->prs, c->mvel64, c->mcru64, c->T1, c->T2, c->P,
-                  c->rhs2_tbl, c->jst, c->pp_wy, c->pp_sy, c->pp_acc, c->cbc,
+                  c->rhs2_tbl, c->rhs2_tbl64, c->jst, c->pp_wy, c->pp_sy, c->pp_acc, c->cbc,
                   c->sc, c->d_um_dy, c->cflp, c->cflbits, c->l2acc, c->divbits, c->plist, c->pw_H,
                   c->pw_phys, c->pw_phys2, c->pw_in, c->stage, c->twx, c->twz, c->twxs, c->twzs,
                   c->wl_fast, c->wl_prec, c->scat_tab, c->cfl_peers, c->les_S, c->les_F, c->les_len,
@@ -1151,7 +1220,9 @@ void cfg_destroy(cfg_ctx* c) {
   for (cudaEvent_t e : c->ev_pool) cudaEventDestroy(e);
   if (c->ev_fork) cudaEventDestroy(c->ev_fork);
   if (c->ev_join) cudaEventDestroy(c->ev_join);
+  if (c->ev_join3) cudaEventDestroy(c->ev_join3);
   if (c->st2) cudaStreamDestroy(c->st2);
+  if (c->st3) cudaStreamDestroy(c->st3);
   if (c->st) cudaStreamDestroy(c->st);
   delete c;
 }
@@ -2834,13 +2905,13 @@ struct EnsClass {
   void* dtab = nullptr;        // every table below, one allocation
   P1Launch *zinv = nullptr, *xinv = nullptr, *zfwd = nullptr, *flux[3] = {};
   Rhs2Launch* r2[3] = {};
-  RhsLowLaunch* rl[3] = {};
+  RhsRowsLaunch* rl[3] = {};
   EnsMember* sm = nullptr;
   EnsJet* jt = nullptr;
   // the first member's records: launch shapes, on the class's streams
   P1Launch h_zinv{}, h_xinv{}, h_zfwd{}, h_flux[3] = {};
   Rhs2Launch h_r2[3] = {};
-  RhsLowLaunch h_rl[3] = {};
+  RhsRowsLaunch h_rl[3] = {};
   int nx = 0, nz = 0, nxh = 0, nx2 = 0, nz2 = 0;
   size_t ncbc = 0;
 };
@@ -2903,7 +2974,7 @@ static bool ens_same_class(const cfg_ctx* a, const cfg_ctx* b) {
          x.ny1 == y.ny1 && x.nw == y.nw && a->gP.nz2 == b->gP.nz2 && a->fYB1 == b->fYB1 && a->fYB3 == b->fYB3 &&
          a->flux_zr == b->flux_zr && a->rhs2_warps == b->rhs2_warps && a->rhs2_lanes == b->rhs2_lanes &&
          a->mean_split == b->mean_split && a->n_fast == b->n_fast && a->n_prec == b->n_prec &&
-         a->xinv_zb == b->xinv_zb;
+         a->xinv_zb == b->xinv_zb && a->rhs_rows == b->rhs_rows;
 }
 
 // the classes, their streams and their member tables
@@ -2935,7 +3006,7 @@ static int ens_build_classes(cfg_ensemble* e) {
     const int n = (int)k.mem.size(), nj = (int)k.jet.size();
     std::vector<P1Launch> zinv(n), xinv(n), zfwd(n), flux(3 * n);
     std::vector<Rhs2Launch> r2(3 * n);
-    std::vector<RhsLowLaunch> rl(3 * n);
+    std::vector<RhsRowsLaunch> rl(3 * n);
     std::vector<EnsMember> sm(n);
     std::vector<EnsJet> jt(nj);
     for (int q = 0; q < n; ++q) {
@@ -2945,8 +3016,8 @@ static int ens_build_classes(cfg_ensemble* e) {
       zfwd[q] = I::p1_args(c, 1, false, 2);
       for (int rk = 1; rk <= 3; ++rk) {
         flux[(rk - 1) * n + q] = I::p1_args(c, rk, false, 4);
-        r2[(rk - 1) * n + q] = I::rhs2_args(c, rk);
-        rl[(rk - 1) * n + q] = I::low_args(c, rk);
+        r2[(rk - 1) * n + q] = I::rhs2_args(c, rk, false);
+        rl[(rk - 1) * n + q] = I::rows_args(c, rk);
       }
       EnsMember& a = sm[q];
       a.m64 = c->mvel64;
@@ -2998,7 +3069,7 @@ static int ens_build_classes(cfg_ensemble* e) {
     };
     const size_t o_zinv = take(sizeof(P1Launch) * n), o_xinv = take(sizeof(P1Launch) * n),
                  o_zfwd = take(sizeof(P1Launch) * n), o_flux = take(sizeof(P1Launch) * 3 * n),
-                 o_r2 = take(sizeof(Rhs2Launch) * 3 * n), o_rl = take(sizeof(RhsLowLaunch) * 3 * n),
+                 o_r2 = take(sizeof(Rhs2Launch) * 3 * n), o_rl = take(sizeof(RhsRowsLaunch) * 3 * n),
                  o_sm = take(sizeof(EnsMember) * n),
                  o_jt = take(sizeof(EnsJet) * (nj > 0 ? nj : 1));
     if (cudaMalloc(&k.dtab, off) != cudaSuccess) {
@@ -3007,12 +3078,13 @@ static int ens_build_classes(cfg_ensemble* e) {
       return CFG_E_NOMEM;
     }
     char* b = (char*)k.dtab;
+    const bool c0_rows = e->m[k.mem[0]]->rhs_rows;
     auto put = [&](size_t o, const void* src, size_t bytes) {
       return bytes == 0 || cudaMemcpy(b + o, src, bytes, cudaMemcpyHostToDevice) == cudaSuccess;
     };
     ok = put(o_zinv, zinv.data(), sizeof(P1Launch) * n) && put(o_xinv, xinv.data(), sizeof(P1Launch) * n) &&
          put(o_zfwd, zfwd.data(), sizeof(P1Launch) * n) && put(o_flux, flux.data(), sizeof(P1Launch) * 3 * n) &&
-         put(o_r2, r2.data(), sizeof(Rhs2Launch) * 3 * n) && put(o_rl, rl.data(), sizeof(RhsLowLaunch) * 3 * n) &&
+         put(o_r2, r2.data(), sizeof(Rhs2Launch) * 3 * n) && put(o_rl, rl.data(), sizeof(RhsRowsLaunch) * 3 * n) &&
          put(o_sm, sm.data(), sizeof(EnsMember) * n) &&
          put(o_jt, jt.data(), sizeof(EnsJet) * nj);
     if (!ok) return CFG_E_CUDA;
@@ -3022,13 +3094,13 @@ static int ens_build_classes(cfg_ensemble* e) {
     for (int r = 0; r < 3; ++r) {
       k.flux[r] = (P1Launch*)(b + o_flux) + r * n;
       k.r2[r] = (Rhs2Launch*)(b + o_r2) + r * n;
-      k.rl[r] = (RhsLowLaunch*)(b + o_rl) + r * n;
+      k.rl[r] = (RhsRowsLaunch*)(b + o_rl) + r * n;
       k.h_flux[r] = flux[r * n];
       k.h_flux[r].st = k.st;
       k.h_r2[r] = r2[r * n];
       k.h_r2[r].st = k.st;
       k.h_rl[r] = rl[r * n];
-      k.h_rl[r].st = k.st2;
+      k.h_rl[r].st = c0_rows ? k.st : k.st2;
     }
     k.sm = (EnsMember*)(b + o_sm);
     k.jt = (EnsJet*)(b + o_jt);
@@ -3092,11 +3164,16 @@ static int ens_class_enqueue(cfg_ensemble* e, EnsClass& k) {
       if (int r = ck(true, "batched wall jet")) return r;
     }
     // the FP64 |k| < 4 list and the mean mode beside the main kernel
+    if (c0->rhs_rows) {
+      if (int r = ck(rhs_rows_launch_batch(true, k.h_rl[rk - 1], k.rl[rk - 1], n) == 0, "batched k_rhs_rows")) return r;
+      ++launches;
+      continue;
+    }
     if (int r = ck(cudaEventRecord(k.ev_fork, k.st) == cudaSuccess &&
                        cudaStreamWaitEvent(k.st2, k.ev_fork, 0) == cudaSuccess,
                    "batched fork"))
       return r;
-    if (int r = ck(rhs_low_launch_batch(true, k.h_rl[rk - 1], k.rl[rk - 1], n) == 0, "batched k_rhs_low")) return r;
+    if (int r = ck(rhs_rows_launch_batch(true, k.h_rl[rk - 1], k.rl[rk - 1], n) == 0, "batched k_rhs_rows")) return r;
     if (int r = ck(rhs2_launch_batch(true, k.h_r2[rk - 1], k.r2[rk - 1], n) == 0, "batched k_rhs2")) return r;
     launches += 2;
     if (int r = ck(cudaEventRecord(k.ev_j2, k.st2) == cudaSuccess && cudaStreamWaitEvent(k.st, k.ev_j2, 0) == cudaSuccess,

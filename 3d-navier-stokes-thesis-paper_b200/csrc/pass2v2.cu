@@ -9,17 +9,18 @@
 namespace cfd {
 
 // Batched launches over a member table (the ensemble mode): member m of a
-// class of identical grids takes blocks m*gx ... m*gx + gx - 1 and reads its
-// arguments from its launch record in device memory.  Same body, same
-// arithmetic.
-template <typename T, int M, int G>
+// class of identical grids takes blocks m*gx ... m*gx + gx - 1 of the main
+// kernel and reads its arguments from its launch record in device memory.
+// Same body, same arithmetic.
+template <typename T, typename S, int M, int G>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 1)
 k_rhs2_b(const Rhs2Launch* __restrict__ tab, unsigned gx) {
-  using C = cplx_t<T>;
+  using CS = cplx_t<S>;
   const unsigned m = blockIdx.x / gx;
   const Rhs2Launch& a = tab[m];
-  k_rhs2_body<T, M, G>(make_uint3(blockIdx.x - m * gx, 0, 0), (C*)a.vel, (C*)a.cru, (C*)a.prs, (const C*)a.cbc_top,
-                       (const C*)a.cbc_bot, a.g, a.gd, a.sc, a.rkt, a.rk, a.re, a.wlist, a.nlist, (const T*)a.tbl);
+  k_rhs2_body<T, S, M, G>(make_uint3(blockIdx.x - m * gx, 0, 0), (CS*)a.vel, (CS*)a.cru, (CS*)a.prs,
+                          (const CS*)a.cbc_top, (const CS*)a.cbc_bot, a.g, a.gd, a.sc, a.rkt, a.rk, a.re, a.wlist,
+                          a.nlist, (const T*)a.tbl);
 }
 
 // tab: null for one domain (arguments from a), else the device table of nmem
@@ -36,8 +37,8 @@ static int launch_m(const Rhs2Launch& a, const Rhs2Launch* tab, int nmem) {
   if (cur == 0) cur = 48 * 1024;
   if (sm > cur) {
     const cudaError_t e =
-        tab ? cudaFuncSetAttribute(k_rhs2_b<T, M, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)
-            : cudaFuncSetAttribute(k_rhs2<T, M, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        tab ? cudaFuncSetAttribute(k_rhs2_b<T, T, M, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)
+            : cudaFuncSetAttribute(k_rhs2<T, T, M, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) {
       cudaGetLastError();
       return -2;
@@ -48,9 +49,9 @@ static int launch_m(const Rhs2Launch& a, const Rhs2Launch* tab, int nmem) {
   dim3 gr((a.nlist + per_block - 1) / per_block);
   using C = cplx_t<T>;
   if (tab)
-    k_rhs2_b<T, M, G><<<gr.x * (unsigned)nmem, 32 * a.warps, sm, a.st>>>(tab, gr.x);
+    k_rhs2_b<T, T, M, G><<<gr.x * (unsigned)nmem, 32 * a.warps, sm, a.st>>>(tab, gr.x);
   else
-    k_rhs2<T, M, G><<<gr, 32 * a.warps, sm, a.st>>>((C*)a.vel, (C*)a.cru, (C*)a.prs, (const C*)a.cbc_top,
+    k_rhs2<T, T, M, G><<<gr, 32 * a.warps, sm, a.st>>>((C*)a.vel, (C*)a.cru, (C*)a.prs, (const C*)a.cbc_top,
                                                     (const C*)a.cbc_bot, a.g, a.gd, a.sc, a.rkt, a.rk, a.re, a.wlist,
                                                     a.nlist, (const T*)a.tbl);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
@@ -109,6 +110,60 @@ static int launch_g16(const Rhs2Launch& a, const Rhs2Launch* tab, int nmem) {
     default: return -1;
   }
 }
+
+// FP64 arithmetic over FP32 storage, one warp (one wavenumber) per block
+template <int M>
+static int launch_prec_m(const Rhs2Launch& a) {
+  const size_t sm = rhs2_smem<double, M, 32>(1, a.g.ny1);
+  if (sm > 48 * 1024) return -1;
+  k_rhs2<double, float, M, 32><<<a.nlist, 32, sm, a.st>>>((float2*)a.vel, (float2*)a.cru, (float2*)a.prs,
+                                                         (const float2*)a.cbc_top, (const float2*)a.cbc_bot, a.g,
+                                                         a.gd, a.sc, a.rkt, a.rk, a.re, a.wlist, a.nlist,
+                                                         (const double*)a.tbl);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+int rhs2_launch_prec(const Rhs2Launch& a) {
+  const int M = (a.g.ny1 + 31) / 32;
+  switch (M < 2 ? 2 : M) {
+    case 2: return launch_prec_m<2>(a);
+    case 3: return launch_prec_m<3>(a);
+    case 4: return launch_prec_m<4>(a);
+    case 5: return launch_prec_m<5>(a);
+    case 6: return launch_prec_m<6>(a);
+    case 7: return launch_prec_m<7>(a);
+    case 8: return launch_prec_m<8>(a);
+    default: return -1;
+  }
+}
+
+template <typename S, int M>
+static int launch_mean_m(const RhsMeanLaunch& a) {
+  using CS = cplx_t<S>;
+  const size_t sm = rhs_mean2_smem<M>(a.g.ny1);
+  if (sm > 48 * 1024) return -1;
+  k_rhs_mean2<S, M><<<1, 32, sm, a.st>>>((CS*)a.vel, (CS*)a.cru, (CS*)a.prs, a.mvel64, a.mcru64,
+                                         (const CS*)a.cbc_top, (const CS*)a.cbc_bot, a.g, a.gd, a.sc, a.d_um_dy,
+                                         a.rkt, a.rk, a.re, a.beta, a.fix_mass, a.tbl64);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+template <typename S>
+static int launch_mean_t(const RhsMeanLaunch& a) {
+  const int M = (a.g.ny1 + 31) / 32;
+  switch (M < 2 ? 2 : M) {
+    case 2: return launch_mean_m<S, 2>(a);
+    case 3: return launch_mean_m<S, 3>(a);
+    case 4: return launch_mean_m<S, 4>(a);
+    case 5: return launch_mean_m<S, 5>(a);
+    case 6: return launch_mean_m<S, 6>(a);
+    case 7: return launch_mean_m<S, 7>(a);
+    case 8: return launch_mean_m<S, 8>(a);
+    default: return -1;
+  }
+}
+
+int rhs_mean2_launch(bool f32, const RhsMeanLaunch& a) { return f32 ? launch_mean_t<float>(a) : launch_mean_t<double>(a); }
 
 int rhs2_launch(bool f32, const Rhs2Launch& a) { return rhs2_launch_batch(f32, a, nullptr, 0); }
 
