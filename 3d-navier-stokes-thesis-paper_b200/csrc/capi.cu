@@ -127,7 +127,8 @@ struct cfg_ctx {
   // side stream: the small mean-mode and FP64 low-|k| solves run beside the
   // main per-wavenumber kernel; joined back with events
   cudaStream_t st2 = nullptr, st3 = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_join3 = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_join3 = nullptr, ev_jet = nullptr;
+  int jet_rk = 0;   // substep whose wall jet is enqueued on st2 (ev_jet)
   // background file output (restart file, VTK snapshot): the layout kernel
   // runs on st, the copy to pinned host memory on st_io, the file write on
   // io_thread
@@ -208,6 +209,7 @@ struct cfg_ctx {
   bool full_len = false;   // nx2 of regfft_full and nz2 rows in eights (the LES mode)
   bool use_rhs2 = true;
   int rhs2_lanes = 32;
+  bool advance = false;   // the solve being enqueued ends the step (t_total += dt)
   bool rhs_rows = false;  // small grid: every wavenumber in k_rhs_rows, one launch
   int rhs2_warps = 3;   // warps (wavenumbers) per k_rhs2 block
   int fYB1 = 1, fYB3 = 1, fZR = 1;
@@ -235,9 +237,12 @@ struct cfg_ctx {
   // precision) added by the flux kernel; the learned closure's features and
   // outputs (FP32) and its fallback counter
   // mean split of the mixed path's nonlinear products (k_zinv_r drops the
-  // mean column, k_flux_r adds its products from mean_base, FP64 (ny+1, 3))
+  // mean column, k_flux_r adds its products from its FP64 side copy mvel64, or
+  // from mean_base where that does not hold it)
   bool mean_split = false;
-  double* mean_base = nullptr;
+  double2* mean_base = nullptr;
+  const double2* mean_src = nullptr;   // of the current substep
+  bool cfl_clean = false;   // the CFL maxima are zero (k_cfl_finalize resets them on one rank)
   bool les_on = false;
   LesDev les{};
   cfg_mlp* les_mlp = nullptr;
@@ -365,12 +370,11 @@ static cudaError_t allow_smem(K kernel) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes);
 }
 
-// the real parts of the mean column (kx = kz = 0) of the velocity as the
-// (ny+1, 3) FP64 profile the mean-split flux kernel reads: from the FP64 side
-// copy m64 when given, else from the FP32 state
-__global__ void k_mean_base(const double2* __restrict__ m64, const float2* __restrict__ v32, double* __restrict__ base,
-                            int ny1) {
-  for (int i = threadIdx.x; i < 3 * ny1; i += blockDim.x) base[i] = m64 ? m64[i].x : (double)v32[i].x;
+// the mean column (kx = kz = 0) of the FP32 velocity as the (ny+1, 3) FP64
+// column the mean-split flux kernel reads, where the FP64 side copy does not
+// hold it
+__global__ void k_mean_base(const float2* __restrict__ v32, double2* __restrict__ base, int ny1) {
+  for (int i = threadIdx.x; i < 3 * ny1; i += blockDim.x) base[i] = make_double2((double)v32[i].x, (double)v32[i].y);
 }
 
 template <typename T>
@@ -469,7 +473,7 @@ struct Impl {
     // copy (CHANFLOW_NO_MEAN_SPLIT=1 keeps the whole velocity in the
     // transforms)
     c->mean_split = f32 && c->split_x && c->fast_z && c->nranks == 1 && !getenv("CHANFLOW_NO_MEAN_SPLIT");
-    if (c->mean_split && cudaMalloc(&c->mean_base, sizeof(double) * 3 * (size_t)g.ny1) != cudaSuccess) {
+    if (c->mean_split && cudaMalloc(&c->mean_base, sizeof(double2) * 3 * (size_t)g.ny1) != cudaSuccess) {
       cudaGetLastError();
       c->mean_split = false;
     }
@@ -551,7 +555,7 @@ struct Impl {
       a.g = c->gP;
       a.gd = c->gd_all;
       if (c->fringe) a.fringe = (const T*)c->fringe + (size_t)c->z0s * g.nx2;
-      if (which == 4 && a.split) a.gd.baseflow = c->mean_base;
+      if (which == 4 && a.split) a.mean64 = c->mean_src;
     }
     return a;
   }
@@ -566,15 +570,16 @@ struct Impl {
     const bool f32 = sizeof(T) == 4;
     P1Launch a = p1_args(c, rk, lin, 0);
     if (phase == 1) {
-      if (a.split) {
-        // the current mean velocity (the FP64 side copy when it holds it)
+      c->mean_src = c->mvel64;
+      if (a.split && !c->mean64_valid) {
         prof_begin(c, "k_mean_base");
-        k_mean_base<<<1, 256, 0, c->st>>>(c->mean64_valid ? c->mvel64 : nullptr, (const float2*)c->vel, c->mean_base,
-                                         g.ny1);
+        k_mean_base<<<1, 256, 0, c->st>>>((const float2*)c->vel, c->mean_base, g.ny1);
         CKL();
+        c->mean_src = c->mean_base;
       }
       c->mean64_valid = false;
-      if (do_cfl) CK(cudaMemsetAsync(c->cflbits, 0, sizeof(unsigned long long) * 3 * g.ny1, c->st));
+      if (do_cfl && !c->cfl_clean) CK(cudaMemsetAsync(c->cflbits, 0, sizeof(unsigned long long) * 3 * g.ny1, c->st));
+      if (do_cfl) c->cfl_clean = false;
       dim3 g1(g.nxh, (g.ny1 + c->YB1 - 1) / c->YB1);
       prof_begin(c, "k_zinv");
       if (c->fast_z) {
@@ -630,14 +635,17 @@ struct Impl {
       k_zfwd<T><<<g3, 256, c->sm_zfwd, c->st>>>((const C*)c->T2, (C*)c->vel, g, c->pz, (const C*)c->twz, c->gd, c->YB3);
     CKL();
     if (do_cfl) {
+      // (the other ranks may still read this rank's maxima)
+      const int reset = c->nranks == 1;
       prof_begin(c, "k_cfl_finalize");
       if (lin)
-        k_cfl_finalize<true><<<1, 256, 0, c->st>>>(c->cflbits, g, c->gd, c->sc, c->cflp, c->p.lx, c->p.lz,
+        k_cfl_finalize<true><<<1, 256, 0, c->st>>>(c->cflbits, reset, g, c->gd, c->sc, c->cflp, c->p.lx, c->p.lz,
                                                     c->p.dt_flag, c->p.cfl_max, step);
       else
-        k_cfl_finalize<false><<<1, 256, 0, c->st>>>(c->cflbits, g, c->gd, c->sc, c->cflp, c->p.lx, c->p.lz,
+        k_cfl_finalize<false><<<1, 256, 0, c->st>>>(c->cflbits, reset, g, c->gd, c->sc, c->cflp, c->p.lx, c->p.lz,
                                                      c->p.dt_flag, c->p.cfl_max, step);
       CKL();
+      c->cfl_clean = reset;
     }
     return CFG_OK;
   }
@@ -731,6 +739,7 @@ struct Impl {
     m.g = g; m.gd = c->gd; m.sc = c->sc; m.d_um_dy = c->d_um_dy; m.rkt = c->rkt; m.rk = rk;
     m.re = c->p.re; m.beta = c->p.beta; m.fix_mass = c->p.fix_mass;
     m.mean = g.kx0 == 0 ? 1 : 0;
+    m.advance = c->advance ? 1 : 0;
     m.wlist = c->wl_prec; m.nlist = c->n_prec;
     m.wfast = c->wl_fast; m.nfast = c->rhs_rows ? c->n_fast : 0;
     m.st = c->rhs_rows ? c->st : c->st2;
@@ -742,8 +751,13 @@ struct Impl {
     const Geom& g = c->g;
     // crossflow == 1: the wall jet of this substep (PFC/pass2.f90:41-43)
     if (c->crossflow && mode == 0) {
-      const int r = jet(c, rk, 0.0, 0.0, 1);
-      if (r) return r;
+      if (c->jet_rk == rk) {   // enqueued beside the nonlinear term
+        CK(cudaStreamWaitEvent(c->st, c->ev_jet, 0));
+      } else {
+        const int r = jet(c, rk, 0.0, 0.0, 1);
+        if (r) return r;
+      }
+      c->jet_rk = 0;
     }
     const bool keep = c->use_rhs2 && mode == 0 && step_keeps_sums(c);
     if (c->rhs_rows && mode == 0 && !keep) {
@@ -813,7 +827,19 @@ struct Impl {
     CK(cudaStreamWaitEvent(c->st, c->ev_join, 0));
     return CFG_OK;
   }
-  static int rhs(cfg_ctx* c, int rk, int mode) {
+  // advance: t_total += dt after the solve
+  static int rhs(cfg_ctx* c, int rk, int mode, bool advance = false) {
+    const bool fused = advance && mode == 0 && c->use_rhs2 && !step_keeps_sums(c) && c->g.kx0 == 0;
+    c->advance = fused;
+    const int r = rhs_solve(c, rk, mode);
+    c->advance = false;
+    if (r || !advance || fused) return r;
+    prof_begin(c, "k_advance_time");
+    k_advance_time<<<1, 1, 0, c->st>>>(c->sc);
+    CKL();
+    return CFG_OK;
+  }
+  static int rhs_solve(cfg_ctx* c, int rk, int mode) {
     switch (c->M) {
       case 2: return rhs_m<2>(c, rk, mode);
       case 3: return rhs_m<3>(c, rk, mode);
@@ -905,6 +931,24 @@ struct Impl {
                                                              g.nz, g.nxh, c->p.lx, c->p.lz);
     CKL();
     return CFG_OK;
+  }
+
+  // the wall jet of substep rk of a time step on the side stream, beside the
+  // nonlinear term, where dt is already final: five small kernels in a chain
+  // (25 us of a 290 us substep at 128x129x128) that only the solve needs
+  static int jet_beside(cfg_ctx* c, int rk) {
+    c->jet_rk = 0;
+    if (!c->crossflow || (rk == 1 && c->p.dt_flag == 1)) return CFG_OK;
+    CK(cudaEventRecord(c->ev_fork, c->st));
+    CK(cudaStreamWaitEvent(c->st2, c->ev_fork, 0));
+    const cudaStream_t main = c->st;
+    c->st = c->st2;
+    const int r = jet(c, rk, 0.0, 0.0, 1);
+    c->st = main;
+    CK(cudaEventRecord(c->ev_jet, c->st2));
+    CK(cudaGetLastError());
+    c->jet_rk = rk;
+    return r;
   }
 
   static int boundary(cfg_ctx* c) {
@@ -1039,6 +1083,7 @@ static int create_impl(const cfg_params* p, const cfg_grid* gr, const SlabPart* 
       cudaStreamCreateWithFlags(&c->st2, cudaStreamNonBlocking) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->st3, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->ev_join3, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&c->ev_jet, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess) {
     delete c;
@@ -1221,6 +1266,7 @@ void cfg_destroy(cfg_ctx* c) {
   if (c->ev_fork) cudaEventDestroy(c->ev_fork);
   if (c->ev_join) cudaEventDestroy(c->ev_join);
   if (c->ev_join3) cudaEventDestroy(c->ev_join3);
+  if (c->ev_jet) cudaEventDestroy(c->ev_jet);
   if (c->st2) cudaStreamDestroy(c->st2);
   if (c->st3) cudaStreamDestroy(c->st3);
   if (c->st) cudaStreamDestroy(c->st);
@@ -1389,6 +1435,7 @@ int cfg_rhs_solve(cfg_ctx* c, int step, int rk_step) {
   if (!c || rk_step < 1 || rk_step > 3) return CFG_E_ARG;
   cudaSetDevice(c->dev);
   (void)step;
+  c->jet_rk = 0;
   return DISPATCH(c, rhs(c, rk_step, 0));
 }
 
@@ -1402,14 +1449,13 @@ static int step_enqueue(cfg_ctx* c, bool lin) {
     if (r) return r;
   }
   for (int rk = 1; rk <= 3; ++rk) {
+    r = DISPATCH(c, jet_beside(c, rk));
+    if (r) return r;
     r = DISPATCH(c, nonlinear(c, c->step, rk, lin));
     if (r) return r;
-    r = DISPATCH(c, rhs(c, rk, 0));
+    r = DISPATCH(c, rhs(c, rk, 0, rk == 3));
     if (r) return r;
   }
-  prof_begin(c, "k_advance_time");
-  k_advance_time<<<1, 1, 0, c->st>>>(c->sc);
-  CKL();
   return CFG_OK;
 }
 
@@ -2495,16 +2541,10 @@ int cfg_group_timestep(cfg_group* G, int nsteps) {
         for (cfg_ctx* c : G->r) {
           cudaSetDevice(c->dev);
           if ((r = DISPATCH(c, nl_phase(c, c->step, rk, false, ph)))) return r;
-          if (ph == 3 && (r = DISPATCH(c, rhs(c, rk, 0)))) return r;
+          if (ph == 3 && (r = DISPATCH(c, rhs(c, rk, 0, rk == 3)))) return r;
         }
         if (ph < 3 && (r = group_barrier(G))) return r;
       }
-    }
-    for (cfg_ctx* c : G->r) {
-      cudaSetDevice(c->dev);
-      prof_begin(c, "k_advance_time");
-      k_advance_time<<<1, 1, 0, c->st>>>(c->sc);
-      CKL();
     }
   }
   (void)n;
@@ -2611,7 +2651,7 @@ static int rank_timestep(cfg_ctx* c, int nsteps, cfg_barrier_fn barrier, void* u
       for (int ph = 1; ph <= 3; ++ph) {
         if ((r = DISPATCH(c, nl_phase(c, c->step, rk, false, ph)))) return r;
         if (ph == 3) {
-          if ((r = DISPATCH(c, rhs(c, rk, 0)))) return r;
+          if ((r = DISPATCH(c, rhs(c, rk, 0, rk == 3)))) return r;
         } else if (c->nranks > 1) {
           // host barrier: this rank's stores into the others' buffers are
           // complete, then every rank's; stream-ordered barrier: the callback
@@ -2620,9 +2660,6 @@ static int rank_timestep(cfg_ctx* c, int nsteps, cfg_barrier_fn barrier, void* u
           if (barrier(user) != 0) return fail(c, CFG_E_ARG, "barrier callback failed");
         }
       }
-    prof_begin(c, "k_advance_time");
-    k_advance_time<<<1, 1, 0, c->st>>>(c->sc);
-    CKL();
   }
   return CFG_OK;
 }
@@ -2801,11 +2838,6 @@ int cfg_set_tiles(cfg_ctx* c, const int* tiles) {
 
 // per-member arguments of the batched small kernels (mixed precision)
 struct EnsMember {
-  // substep prologue: the mean-split base and the CFL maxima
-  const double2* m64;
-  const float2* v32;
-  double* base;
-  int ny1, split;
   unsigned long long* cflbits;
   // boundary: the wall values, zeroed at every step
   float2* cbc;
@@ -2835,17 +2867,6 @@ struct EnsJet {
   double lx, lz;
 };
 
-// k_mean_base and, at rk 1, the zeroed CFL maxima of every member; one block
-// per member
-__global__ void k_ens_prologue(const EnsMember* __restrict__ tab, int do_cfl) {
-  const EnsMember& a = tab[blockIdx.x];
-  const int n = 3 * a.ny1;
-  if (a.split)
-    for (int i = threadIdx.x; i < n; i += blockDim.x) a.base[i] = a.m64 ? a.m64[i].x : (double)a.v32[i].x;
-  if (do_cfl)
-    for (int i = threadIdx.x; i < n; i += blockDim.x) a.cflbits[i] = 0ull;
-}
-
 // the wall values zeroed (boundary without feedback); grid (blocks, members)
 __global__ void k_ens_zero_cbc(const EnsMember* __restrict__ tab) {
   const EnsMember& a = tab[blockIdx.y];
@@ -2855,13 +2876,8 @@ __global__ void k_ens_zero_cbc(const EnsMember* __restrict__ tab) {
 
 __global__ void k_cfl_finalize_b(const EnsMember* __restrict__ tab, int step) {
   const EnsMember& a = tab[blockIdx.x];
-  k_cfl_finalize_body<false>(make_uint3(0, 0, 0), a.cflbits, a.g, a.gd, a.sc, a.cflp, a.lx, a.lz, a.dt_flag,
+  k_cfl_finalize_body<false>(make_uint3(0, 0, 0), a.cflbits, 1, a.g, a.gd, a.sc, a.cflp, a.lx, a.lz, a.dt_flag,
                              a.cfl_max, step);
-}
-
-__global__ void k_ens_advance(const EnsMember* __restrict__ tab, int n) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
-  if (m < n) tab[m].sc->t_total = tab[m].sc->t_total + tab[m].sc->dt;
 }
 
 __global__ void k_jet_walk_b(const EnsJet* __restrict__ tab, int rk) {
@@ -2994,6 +3010,11 @@ static int ens_build_classes(cfg_ensemble* e) {
       e->cls.back().mem.push_back(i);
     }
   }
+  for (cfg_ctx* c : e->m)
+    if (!c->cfl_clean) {
+      if (cudaMemset(c->cflbits, 0, sizeof(unsigned long long) * 3 * c->g.ny1) != cudaSuccess) return CFG_E_CUDA;
+      c->cfl_clean = true;
+    }
   for (EnsClass& k : e->cls) {
     for (int i : k.mem)
       if (e->m[i]->crossflow) k.jet.push_back(i);
@@ -3018,13 +3039,10 @@ static int ens_build_classes(cfg_ensemble* e) {
         flux[(rk - 1) * n + q] = I::p1_args(c, rk, false, 4);
         r2[(rk - 1) * n + q] = I::rhs2_args(c, rk, false);
         rl[(rk - 1) * n + q] = I::rows_args(c, rk);
+        rl[(rk - 1) * n + q].advance = rk == 3;
+        flux[(rk - 1) * n + q].mean64 = c->mvel64;
       }
       EnsMember& a = sm[q];
-      a.m64 = c->mvel64;
-      a.v32 = (const float2*)c->vel;
-      a.base = c->mean_base;
-      a.ny1 = c->g.ny1;
-      a.split = (c->mean_split && !c->les_on) ? 1 : 0;
       a.cflbits = c->cflbits;
       a.cbc = (float2*)c->cbc;
       a.ncbc = 6 * (size_t)c->g.nw;
@@ -3135,9 +3153,6 @@ static int ens_class_enqueue(cfg_ensemble* e, EnsClass& k) {
   ++launches;
   if (int r = ck(true, "batched boundary")) return r;
   for (int rk = 1; rk <= 3; ++rk) {
-    k_ens_prologue<<<n, 256, 0, k.st>>>(k.sm, rk == 1);
-    ++launches;
-    if (int r = ck(true, "batched substep prologue")) return r;
     if (int r = ck(p1_fast_launch_batch(0, k.nz2, true, k.h_zinv, k.zinv, n) == 0, "batched k_zinv_r")) return r;
     if (int r = ck(p1_fast_launch_batch(3, k.nx2, true, k.h_xinv, k.xinv, n) == 0, "batched k_xinv_r")) return r;
     if (int r = ck(p1_fast_launch_batch(4, k.nx2, true, k.h_flux[rk - 1], k.flux[rk - 1], n) == 0, "batched k_flux_r"))
@@ -3180,9 +3195,6 @@ static int ens_class_enqueue(cfg_ensemble* e, EnsClass& k) {
                    "batched join"))
       return r;
   }
-  k_ens_advance<<<(n + 63) / 64, 64, 0, k.st>>>(k.sm, n);
-  ++launches;
-  if (int r = ck(true, "batched advance time")) return r;
   // the members' host bookkeeping, as step_enqueue keeps it (the batched
   // launches are shared: each member is credited with its share)
   for (int q = 0; q < n; ++q) {

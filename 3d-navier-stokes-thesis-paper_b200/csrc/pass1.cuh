@@ -350,8 +350,9 @@ __global__ void __launch_bounds__(256) k_zfwd(const cplx_t<T>* __restrict__ T2,
 
 // --------------------------------------------------------------------------
 // check_cfl + dt adaptation (PFC/pass1.f90:202-250, 106-124): one block.
+// reset: the maxima are cleared for the next step.
 template <bool LIN>
-__device__ __forceinline__ void k_cfl_finalize_body(const uint3 bid, const unsigned long long* __restrict__ cflbits,
+__device__ __forceinline__ void k_cfl_finalize_body(const uint3 bid, unsigned long long* __restrict__ cflbits, int reset,
                                                     Geom g, GridDev gd, DevScalars* sc, double* cfl, double lx,
                                                     double lz, int dt_flag, double cfl_max_param, int step) {
   __shared__ double smax[256];
@@ -363,6 +364,8 @@ __device__ __forceinline__ void k_cfl_finalize_body(const uint3 bid, const unsig
     double ma = __longlong_as_double((long long)cflbits[(size_t)(k - 1) * 3 + 0]);
     double mb = __longlong_as_double((long long)cflbits[(size_t)(k - 1) * 3 + 1]);
     double mc = __longlong_as_double((long long)cflbits[(size_t)(k - 1) * 3 + 2]);
+    if (reset)
+      for (int q = 0; q < 3; ++q) cflbits[(size_t)(k - 1) * 3 + q] = 0ull;
     if (LIN) {
       const double* B = gd.baseflow;
       ma = fmax(ma, fabs(B[k - 1] + B[k]));
@@ -397,9 +400,9 @@ __device__ __forceinline__ void k_cfl_finalize_body(const uint3 bid, const unsig
 }
 
 template <bool LIN>
-__global__ void k_cfl_finalize(const unsigned long long* __restrict__ cflbits, Geom g, GridDev gd, DevScalars* sc,
+__global__ void k_cfl_finalize(unsigned long long* __restrict__ cflbits, int reset, Geom g, GridDev gd, DevScalars* sc,
                                double* cfl, double lx, double lz, int dt_flag, double cfl_max_param, int step) {
-  k_cfl_finalize_body<LIN>(blockIdx, cflbits, g, gd, sc, cfl, lx, lz, dt_flag, cfl_max_param, step);
+  k_cfl_finalize_body<LIN>(blockIdx, cflbits, reset, g, gd, sc, cfl, lx, lz, dt_flag, cfl_max_param, step);
 }
 
 }  // namespace cfd

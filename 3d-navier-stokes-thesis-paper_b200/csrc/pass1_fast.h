@@ -26,7 +26,8 @@ struct P1Launch {
   int FZR;              // z rows per k_flux_r block (2 or 4)
   Scatter sc;           // transposes of a multi-rank run (n == 0: one rank)
   const void* sgs;      // LES subgrid stresses [ny+1][6][nz2][nx2] for k_flux_r, or null
-  int split;            // mean split: k_zinv_r drops the mean column, k_flux_r adds it from gd.baseflow
+  int split;            // mean split: k_zinv_r drops the mean column, k_flux_r adds it from mean64
+  const double2* mean64;   // the velocity's mean column, FP64 (ny+1, 3)
   int XZB;              // z2 rows per k_xinv_r block: 8, 16 or 24 (FP32), 0 for the default
   cudaStream_t st;
 };

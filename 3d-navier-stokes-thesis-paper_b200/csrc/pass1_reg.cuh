@@ -689,7 +689,7 @@ k_xinv_r(const cplx_t<T>* __restrict__ T1, T* __restrict__ P, Geom g, const cplx
 // output as k_xflux_r (PFC/pass1.f90:134-226, PFC/transform.f90:287-315).
 // MODE 0: the nonlinear products; 1: the linearized products about the
 // baseflow (PFC/pass1_linearized.f90:135-509); 3: the nonlinear products of
-// a field split into its plane mean B (gd.baseflow, FP64) and the rest u
+// a field split into its plane mean B (mean64, FP64) and the rest u
 // (the physical planes, mean column removed): (B + u)(B + u) - B B = the
 // linearized products plus u u, the mean-mean products being constant in x
 // and z (their divergence is the y derivative of B_i V, zero without net
@@ -703,7 +703,7 @@ __device__ __forceinline__ void k_flux_r_body(const uint3 bid, const T* __restri
                                               Geom g, const cplx_t<T>* __restrict__ twx, GridDev gd,
                                               const T* __restrict__ fringe, int has_fringe,
                                               unsigned long long* __restrict__ cflbits, int do_cfl, Scatter sc,
-                                              const T* __restrict__ S) {
+                                              const T* __restrict__ S, const double2* __restrict__ mean64) {
   constexpr bool LIN = MODE == 1, SGS = MODE == 2, SPLIT = MODE == 3;
   constexpr bool HASB = LIN || SPLIT;
   using C = cplx_t<T>;
@@ -737,11 +737,12 @@ __device__ __forceinline__ void k_flux_r_body(const uint3 bid, const T* __restri
   const T tw_ = (T)gd.target[2 * (ny + 1) + (k - 1)];
   T B0[3] = {0, 0, 0}, Bm[3] = {0, 0, 0}, Bp[3] = {0, 0, 0};
   if (HASB) {
+    auto base = [&](int q, int i) { return (T)(SPLIT ? mean64[q * (ny + 1) + i].x : gd.baseflow[q * (ny + 1) + i]); };
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
-      B0[q] = (T)gd.baseflow[q * (ny + 1) + k - 1];
-      Bm[q] = (T)gd.baseflow[q * (ny + 1) + k - 2];
-      Bp[q] = (T)gd.baseflow[q * (ny + 1) + k];
+      B0[q] = base(q, k - 1);
+      Bm[q] = base(q, k - 2);
+      Bp[q] = base(q, k);
     }
   }
   // the mean's half sums onto the y planes k-1 and k and its iu-weighted
@@ -970,8 +971,9 @@ template <typename T, int NX2, int ZR, int NT, int MODE>
 __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? (NT == 256 ? 4 : 6) : (NT == 256 ? 1 : 3))
 k_flux_r(const T* __restrict__ P, cplx_t<T>* __restrict__ T2, Geom g, const cplx_t<T>* __restrict__ twx, GridDev gd,
          const T* __restrict__ fringe, int has_fringe, unsigned long long* __restrict__ cflbits, int do_cfl,
-         Scatter sc, const T* __restrict__ S) {
-  k_flux_r_body<T, NX2, ZR, NT, MODE>(blockIdx, P, T2, g, twx, gd, fringe, has_fringe, cflbits, do_cfl, sc, S);
+         Scatter sc, const T* __restrict__ S, const double2* __restrict__ mean64) {
+  k_flux_r_body<T, NX2, ZR, NT, MODE>(blockIdx, P, T2, g, twx, gd, fringe, has_fringe, cflbits, do_cfl, sc, S,
+                                      mean64);
 }
 
 // smem sizes (bytes) of the three kernels

@@ -309,6 +309,7 @@ __device__ __forceinline__ void k_rhs_rows_body(int w, bool mean, const RhsRowsL
     const double* dm = gd.dm;
     if (j == 0) {
       a.sc->p_grad = pg;
+      if (a.advance) a.sc->t_total = a.sc->t_total + dt;
       a.d_um_dy[0] = dm[0] * sV[0].x + dm[1] * sV[1].x + dm[2] * sV[2].x;
       a.d_um_dy[ny - 1] = dm[3] * sV[ny - 2].x + dm[4] * sV[ny - 1].x + dm[5] * sV[ny].x;
     }

@@ -68,6 +68,7 @@ struct RhsRowsLaunch {
   double re, beta;
   int fix_mass;
   int mean;                   // 1: this rank holds the mean mode
+  int advance;                // the mean mode's block adds dt to t_total
   const int* wlist;           // FP64 list
   int nlist;
   const int* wfast;           // the fast list, nfast 0 where k_rhs2 takes it
