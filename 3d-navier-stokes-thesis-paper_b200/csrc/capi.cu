@@ -424,22 +424,16 @@ struct Impl {
       RHS_ATTR(2) RHS_ATTR(3) RHS_ATTR(4) RHS_ATTR(5) RHS_ATTR(6) RHS_ATTR(7) RHS_ATTR(8)
 #undef RHS_ATTR
     }
-    // register-FFT kernels: z-kernel tiles that keep four (FP32) or two (FP64)
-    // blocks per SM, matching their launch bounds
+    // register-FFT kernels
     const bool f32 = sizeof(T) == 4;
     c->fast_z = regfft_supported(g.nz2);
     c->fast_x = regfft_supported(g.nx2);
-    if (c->fast_z) {
-      const size_t zb = f32 ? 52 * 1024 : 108 * 1024;
-      // z inverse: three blocks per SM with the raw tile and the exchange
-      // (FP32); one plane per block in FP64 (measured best at 256x193x256)
-      c->fYB1 = 1;
-      for (int yb = f32 ? 4 : 1; yb >= 1; --yb)
-        if (p1_fast_smem(0, g.nz2, f32, yb, g.nxh, g.nz) <= 74 * 1024) { c->fYB1 = yb; break; }
-      c->fYB3 = 1;
-      for (int yb = 4; yb >= 1; --yb)
-        if (p1_fast_smem(2, g.nz2, f32, yb, g.nxh, g.nz) <= zb) { c->fYB3 = yb; break; }
-    }
+    // planes per z-transform block: 8 in the inverse transform (short of it the
+    // data1 runs are too short: 256x193x256 mixed 349, 100, 86 and 84 us for 1,
+    // 2, 4 and 8; FP64 206, 184, 165 and 178: 4 from 288 points on); 4 in the
+    // forward transform (248, 188, 166 and 176 us; FP64 424, 306, 313 and 364)
+    c->fYB1 = f32 || g.nz2 < 288 ? 8 : 4;
+    c->fYB3 = 4;
     if (c->fast_x) {
       c->fZR = 1;
       for (int zr : {4, 2})
@@ -526,15 +520,6 @@ struct Impl {
     if (nz2 % zr == 0 && (zr < 8 || plain_products || regfft_full(c->g.nx2))) return zr;
     return nz2 % 4 == 0 ? 4 : 2;
   }
-  // planes per z-transform block: the tile where its block can be launched
-  // (the lengths of regfft_full leave that to the launch)
-  static int z_planes(const cfg_ctx* c, int which, int yb) {
-    if (regfft_full(c->g.nz2)) return yb;
-    yb = std::min(yb, 5);   // 3 yb N2 <= 288 threads for N2 <= 18
-    while (yb > 1 && p1_fast_smem(which, c->g.nz2, sizeof(T) == 4, yb, c->g.nxh, c->g.nz) > 200 * 1024) --yb;
-    return yb;
-  }
-
   // the launch record of register-FFT pass-1 kernel `which` (0 k_zinv_r, 1
   // k_xflux_r, 2 k_zfwd_r, 3 k_xinv_r, 4 k_flux_r) in substep rk
   static P1Launch p1_args(const cfg_ctx* c, int rk, bool lin, int which) {
@@ -542,7 +527,7 @@ struct Impl {
     P1Launch a{};
     a.vel = c->vel; a.T1 = c->T1; a.T2 = c->T2; a.velout = c->vel; a.g = g; a.twx = c->twx; a.twz = c->twz;
     a.gd = c->gd; a.fringe = c->fringe; a.has_fringe = c->has_fringe;
-    a.YB1 = z_planes(c, 0, c->fYB1); a.YB3 = z_planes(c, 2, c->fYB3);
+    a.YB1 = c->fYB1; a.YB3 = c->fYB3;
     a.ZR = c->fZR; a.cflbits = c->cflbits; a.do_cfl = (rk == 1); a.lin = lin ? 1 : 0; a.st = c->st;
     a.KC = (int)std::max(2L, std::min(16L, (long)(g.ny - 1) * (g.nz2 / c->fZR) / 592));
     a.P = c->P;
@@ -2775,8 +2760,8 @@ int cfg_autotune(cfg_ctx* c, int trial_steps, int* choice) {
   if (c->fast_z) {
     // planes per z-transform block (a block too large for its launch fails
     // its trial)
-    tune(&c->fYB1, {1, 2, 3, 4, 6, 8});
-    tune(&c->fYB3, {1, 2, 3, 4, 6, 8});
+    tune(&c->fYB1, {1, 2, 4, 8});
+    tune(&c->fYB3, {1, 2, 4, 8});
   }
   // z2 rows per inverse-x block (not one of the four public tiles; a row
   // count that does not divide the slab fails its trial)
@@ -3298,8 +3283,8 @@ static int ens_tune_batched(cfg_ensemble* e, int trial_steps) {
     };
     tune(&cfg_ctx::rhs2_warps, {2, 3, 4});
     tune(&cfg_ctx::flux_zr, {2, 4, 8});
-    tune(&cfg_ctx::fYB1, {1, 2, 3, 4, 6, 8});
-    tune(&cfg_ctx::fYB3, {1, 2, 3, 4, 6, 8});
+    tune(&cfg_ctx::fYB1, {1, 2, 4, 8});
+    tune(&cfg_ctx::fYB3, {1, 2, 4, 8});
     tune(&cfg_ctx::xinv_zb, {8, 16, 24});
   }
   for (int i = 0; i < n; ++i) {

@@ -39,85 +39,113 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 __device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
 
 // --------------------------------------------------------------------------
-// k_zinv_r: grid (nxh, ceil(ny1/YB)), block zinv_r_threads(N, YB) (one thread
-// per stage-1 task).  Inverse z transform of the 3/2-padded columns
-// (xz_fft_complex_to_real_parallel, PFC/transform.f90:345-368).  The block's
-// input -- YB consecutive planes of all kz and the three components of one kx,
-// contiguous YB-value runs of data1 -- is gathered with cp.async into a raw
-// tile first, so that all of its loads are in flight at once.
-template <int N> __host__ __device__ constexpr int zinv_r_threads(int YB) {
-  return ((3 * YB * Split<N>::N2 + 31) / 32) * 32;
-}
-template <typename T> struct ZRawPad {   // 32 bytes between component blocks
-  static constexpr int V = 32 / (int)sizeof(cplx_t<T>);
+// The z transforms.  A block takes YP consecutive planes of one kx and one
+// component (k_zinv_r) or equation (k_zfwd_r): the spectral state keeps y
+// innermost, so YP is the run its reads or writes make there, 8 planes of
+// FP32 a 64-byte run, where a block of fewer planes and all three components
+// (as this was: 2 to 4 planes at 256x193x256, 1 to 2 at 384x193x384) moves 8
+// to 32 bytes of each 32-byte sector.  Everything that indexes by plane is
+// known at compile time, one thread takes one stage-1 and one stage-2 task,
+// and the 3/2-dealiased row count (DEAL: nz = 2 nz2/3) too: which of a
+// thread's N1 inputs are zero or mirrored is then a constant of n1 but for
+// the two at the edges.  us per launch before / now, mixed: k_zinv_r 121 / 84
+// and k_zfwd_r 234 / 166 at 256x193x256, 505 / 190 and 905 / 399 at
+// 384x193x384; FP64 280 / 165 and 405 / 313 at 256x193x256.  What is left is
+// latency: both move two thirds of the copy bandwidth at best (k_zinv_r 4.6,
+// k_zfwd_r 3.7 TB/s at 256x193x256 mixed).
+template <typename T, int N, int YP> struct ZShape {
+  static constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2;
+  static constexpr int PITCH = N2 | 1;   // odd: rows of the exchange buffer on different banks
+  // between sequences: lanes run over YP (k_zinv_r) or 2 YP sequences and
+  // 16/YP or 8/YP columns of an 8-byte half-warp
+  static constexpr int pad(int n, int want) { return n + ((want - n) % 16 + 16) % 16; }
+  static constexpr int INV_SEQ = pad(N1 * PITCH, 16 / YP);
+  // stage-2 output of k_zfwd_r, over the exchange buffer: lanes of the last
+  // phase run over YP planes (two sequences apart) and 16/YP values of kz
+  static constexpr int FWD_Z = N + (((8 / YP > 0 ? 8 / YP : 1) - N) % 8 + 8) % 8;
+  static constexpr int FWD_SEQ = pad(N1 * PITCH > FWD_Z ? N1 * PITCH : FWD_Z, 1);
+  static constexpr int up32(int n) { return (n + 31) / 32 * 32; }
+  static constexpr int INV_NT = up32(YP * (N1 > N2 ? N1 : N2));
+  static constexpr int FWD_NT = up32(2 * YP * (N1 > N2 ? N1 : N2));
+  // blocks per SM to compile for: the registers that keep the FFT's values
+  // (the longer of N1, N2) without spilling
+  static constexpr int LONG = N1 > N2 ? N1 : N2;
+  static constexpr int regs(bool f32) { return f32 ? (LONG > 18 ? 80 : LONG > 12 ? 64 : 56) : (LONG > 18 ? 168 : LONG > 12 ? 128 : 104); }
+  static constexpr int blocks(int nt, bool f32) { return 65536 / (nt * regs(f32)) > 0 ? (65536 / (nt * regs(f32)) > 32 ? 32 : 65536 / (nt * regs(f32))) : 1; }
 };
 
-template <typename T, int NZ2>
+// k_zinv_r: grid (nxh, ceil(ny1/YP), 3), block INV_NT.  Inverse z transform of
+// the 3/2-padded columns (xz_fft_complex_to_real_parallel,
+// PFC/transform.f90:345-368).  The block's input, YP planes of all kz, is
+// gathered with cp.async into a raw tile first, so that all of its loads are
+// in flight at once.
+template <typename T, int NZ2, int YP, bool DEAL>
 __device__ __forceinline__ void k_zinv_r_body(const uint3 bid, const cplx_t<T>* __restrict__ vel,
                                               cplx_t<T>* __restrict__ T1, Geom g, const cplx_t<T>* __restrict__ twz,
-                                              int YB, Scatter sc, int split) {
+                                              Scatter sc, int split) {
   using C = cplx_t<T>;
-  constexpr int N1 = Split<NZ2>::N1, N2 = Split<NZ2>::N2, PITCH = N2 + 1, SEQ = SeqPitch<NZ2>::V;
+  using Z = ZShape<T, NZ2, YP>;
+  constexpr int N1 = Z::N1, N2 = Z::N2, PITCH = Z::PITCH, SEQ = Z::INV_SEQ, NT = Z::INV_NT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int NZ = g.nz, NY1 = g.ny1, NXH = g.nxh;
-  const int RS = NZ * YB + ZRawPad<T>::V;   // raw stride per component
+  const int NZ = DEAL ? 2 * NZ2 / 3 : g.nz, H = NZ / 2, NY1 = g.ny1, NXH = g.nxh;
   C* tw = reinterpret_cast<C*>(smem_raw);
-  C* raw = tw + NZ2;                         // [c][kz][jj]
-  C* Y = raw + 3 * RS;
-  const int kx = bid.x;
-  const int j0 = bid.y * YB;
-  const int nj = min(YB, NY1 - j0);
-  const int nseq = 3 * YB;
-  const C* col = vel + (size_t)kx * NZ * 3 * NY1;
-  {
-    // gather: runs of nj planes at (kz, c), 16-byte pieces when aligned
-    // 16-byte pieces need 16-byte aligned sources (data1 run starts) and
-    // destinations (raw tile: the kz stride YB and the component stride RS)
-    const int rb = nj * (int)sizeof(C);
-    const bool v16 = (rb % 16) == 0 && ((size_t)NY1 * sizeof(C)) % 16 == 0 && ((size_t)j0 * sizeof(C)) % 16 == 0 &&
-                     ((size_t)YB * sizeof(C)) % 16 == 0 && ((size_t)RS * sizeof(C)) % 16 == 0 &&
-                     ((size_t)NZ2 * sizeof(C)) % 16 == 0;
-    const int psz = v16 ? 16 : 8, np = rb / psz;
-    for (int idx = threadIdx.x; idx < 3 * NZ * np; idx += blockDim.x) {
-      const int part = idx % np, r = idx / np, kz = r % NZ, c = r / NZ;
-      const char* src = reinterpret_cast<const char*>(col + ((size_t)kz * 3 + c) * NY1 + j0) + part * psz;
-      char* dst = reinterpret_cast<char*>(raw + c * RS + kz * YB) + part * psz;
-      if (v16) cp_async16(dst, src);
-      else cp_async8(dst, src);
+  C* raw = tw + NZ2;                         // [kz][YP]
+  C* Y = raw + NZ * YP;
+  const int kx = bid.x, j0 = bid.y * YP, c = bid.z, t = threadIdx.x;
+  const int nj = min(YP, NY1 - j0);
+  const C* col = vel + ((size_t)kx * NZ * 3 + c) * NY1 + j0;
+  const size_t kzs = (size_t)3 * NY1;
+  // 16-byte pieces need 16-byte aligned runs: whole groups of rows of even length
+  if (YP * sizeof(C) % 16 == 0 && nj == YP && (sizeof(C) == 16 || NY1 % 2 == 0)) {
+    constexpr int NP = YP * (int)sizeof(C) / 16 > 0 ? YP * (int)sizeof(C) / 16 : 1;
+    for (int idx = t; idx < NZ * NP; idx += NT) {
+      const int part = idx % NP, kz = idx / NP;
+      cp_async16(reinterpret_cast<char*>(raw + kz * YP) + part * 16,
+                 reinterpret_cast<const char*>(col + kz * kzs) + part * 16);
     }
-    cp_async_commit();
+  } else {
+    for (int idx = t; idx < NZ * YP; idx += NT) {
+      const int jj = idx % YP, kz = idx / YP;
+      if (jj < nj) {
+        if (sizeof(C) == 16) cp_async16(raw + idx, col + kz * kzs + jj);
+        else cp_async8(raw + idx, col + kz * kzs + jj);
+      }
+    }
   }
+  cp_async_commit();
   load_tw2<T, NZ2>(tw, twz);
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
   __syncthreads();
+  const T half = (T)0.5;
   if (split && g.kx0 + kx == 0) {
     // mean split: the kx = kz = 0 column leaves the physical fields (the
     // flux kernel adds the mean's products from its FP64 copy)
-    for (int i = threadIdx.x; i < 3 * YB; i += blockDim.x) raw[(i / YB) * RS + (i % YB)] = czero<C>();
+    if (t < YP) raw[t] = czero<C>();
     __syncthreads();
   }
-  const T half = (T)0.5;
-  const bool halve_x = (g.nx2 > g.nx) && (g.kx0 + kx == g.nxh_all - 1) && (NZ2 > NZ);
-  // stage 1: consecutive threads take consecutive sequences (planes fastest)
-  for (int t = threadIdx.x; t < nseq * N2; t += blockDim.x) {
-    const int s = t % nseq, n2 = t / nseq;
-    const int jj = s % YB, c = s / YB;
-    const C* rc = raw + c * RS + jj;
+  if ((g.nx2 > g.nx) && (g.kx0 + kx == g.nxh_all - 1) && (NZ2 > NZ)) {
+    for (int idx = t; idx < NZ * YP; idx += NT) raw[idx] = cscale(half, raw[idx]);
+    __syncthreads();
+  }
+  // stage 1: consecutive threads take consecutive planes
+  if (t < YP * N2) {
+    const int s = t % YP, n2 = t / YP;
+    const C* rc = raw + s;
     C v[N1];
 #pragma unroll
     for (int n1 = 0; n1 < N1; ++n1) {
       const int m = N2 * n1 + n2;
       C x = czero<C>();
-      if (jj < nj) {
-        if (NZ2 > NZ) {
-          if (m < NZ / 2) x = rc[m * YB];
-          else if (m == NZ / 2) x = cscale(half, rc[(NZ / 2) * YB]);
-          else if (m == NZ2 - NZ / 2) x = cscale(half, cconj(rc[(NZ / 2) * YB]));
-          else if (m > NZ2 - NZ / 2) x = rc[(m - (NZ2 - NZ)) * YB];
-          if (halve_x) x = cscale(half, x);
-        } else {
-          x = rc[m * YB];
-        }
+      if (DEAL && N2 * n1 + N2 <= NZ2 / 3) x = rc[m * YP];
+      else if (DEAL && N2 * n1 > NZ2 / 3 && N2 * n1 + N2 <= NZ2 - NZ2 / 3) {}
+      else if (DEAL && N2 * n1 > NZ2 - NZ2 / 3) x = rc[(m - NZ2 / 3) * YP];
+      else if (NZ2 > NZ) {
+        if (m < H) x = rc[m * YP];
+        else if (m == H) x = cscale(half, rc[H * YP]);
+        else if (m == NZ2 - H) x = cscale(half, cconj(rc[H * YP]));
+        else if (m > NZ2 - H) x = rc[(m - (NZ2 - NZ)) * YP];
+      } else {
+        x = rc[m * YP];
       }
       v[n1] = x;
     }
@@ -132,21 +160,20 @@ __device__ __forceinline__ void k_zinv_r_body(const uint3 bid, const cplx_t<T>* 
   }
   __syncthreads();
   // stage 2: consecutive threads take consecutive rows k1 (coalesced stores)
-  for (int t = threadIdx.x; t < nseq * N1; t += blockDim.x) {
-    const int k1 = t % N1, s = t / N1;
-    const int jj = s % YB, c = s / YB;
+  const int k1 = t % N1, s = t / N1;
+  if (s < nj) {
     C u[N2];
     const C* y = Y + s * SEQ + k1 * PITCH;
 #pragma unroll
     for (int n2 = 0; n2 < N2; ++n2) u[n2] = y[n2];
     SmallFFT<T, N2, +1>::template run<1>(u);
-    if (jj < nj && sc.n == 0) {
-      C* out = T1 + (((size_t)(j0 + jj) * 3 + c) * NXH + kx) * NZ2;
+    if (sc.n == 0) {
+      C* out = T1 + (((size_t)(j0 + s) * 3 + c) * NXH + kx) * NZ2 + k1;
 #pragma unroll
-      for (int k2 = 0; k2 < N2; ++k2) out[k1 + N1 * k2] = u[k2];
-    } else if (jj < nj) {
+      for (int k2 = 0; k2 < N2; ++k2) out[N1 * k2] = u[k2];
+    } else {
       // transpose to z2 slabs: element z2 goes to the rank that owns it
-      const long long row = ((long long)(j0 + jj) * 3 + c) * g.nxh_all + g.kx0 + kx;
+      const long long row = ((long long)(j0 + s) * 3 + c) * g.nxh_all + g.kx0 + kx;
 #pragma unroll
       for (int k2 = 0; k2 < N2; ++k2) {
         const int z = k1 + N1 * k2;
@@ -156,63 +183,62 @@ __device__ __forceinline__ void k_zinv_r_body(const uint3 bid, const cplx_t<T>* 
   }
 }
 
-template <typename T, int NZ2>
-__global__ void __launch_bounds__(288, sizeof(T) == 4 ? 3 : 1)
+template <typename T, int NZ2, int YP, bool DEAL>
+__global__ void __launch_bounds__(ZShape<T, NZ2, YP>::INV_NT, ZShape<T, NZ2, YP>::blocks(ZShape<T, NZ2, YP>::INV_NT, sizeof(T) == 4))
 k_zinv_r(const cplx_t<T>* __restrict__ vel, cplx_t<T>* __restrict__ T1, Geom g, const cplx_t<T>* __restrict__ twz,
-         int YB, Scatter sc, int split) {
-  k_zinv_r_body<T, NZ2>(blockIdx, vel, T1, g, twz, YB, sc, split);
+         Scatter sc, int split) {
+  k_zinv_r_body<T, NZ2, YP, DEAL>(blockIdx, vel, T1, g, twz, sc, split);
 }
 
 // --------------------------------------------------------------------------
-// k_zfwd_r: grid (nxh, ceil(ny1/YB)), block 256.  Forward z transform, fold,
-// scale and ikz combine (PFC/transform.f90:317-333, 639-688).
-template <typename T, int NZ2>
+// k_zfwd_r: grid (nxh, ceil(ny1/YP), 3), block FWD_NT.  Forward z transform of
+// one equation's two parts, fold, scale and ikz combine
+// (PFC/transform.f90:317-333, 639-688).
+template <typename T, int NZ2, int YP, bool DEAL>
 __device__ __forceinline__ void k_zfwd_r_body(const uint3 bid, const cplx_t<T>* __restrict__ T2,
                                               cplx_t<T>* __restrict__ vel, Geom g, const cplx_t<T>* __restrict__ twz,
-                                              GridDev gd, int YB) {
+                                              GridDev gd) {
   using C = cplx_t<T>;
-  constexpr int N1 = Split<NZ2>::N1, N2 = Split<NZ2>::N2, PITCH = N2 + 1, SEQ = SeqPitch<NZ2>::V;
-  constexpr int ZP = NZ2 + 1;   // pitch of the stage-2 output (spreads banks across sequences)
-  static_assert(ZP <= SEQ, "stage-2 output must fit in the exchange buffer");
+  using Z = ZShape<T, NZ2, YP>;
+  constexpr int N1 = Z::N1, N2 = Z::N2, PITCH = Z::PITCH, SEQ = Z::FWD_SEQ, ZP = Z::FWD_Z, NT = Z::FWD_NT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* tw = reinterpret_cast<C*>(smem_raw);
-  const int nseq = 6 * YB;
-  C* Y = tw + NZ2;
-  C* Z = Y;                      // stage 2 reads Y into registers, then overwrites it
-  const int NZ = g.nz, NY1 = g.ny1, NXH = g.nxh, ny = g.ny;
-  const int kx = bid.x;
-  const int j0 = 1 + bid.y * YB;   // 1-based first plane
+  C* Y = tw + NZ2;               // sequence 2 jj + part of plane jj
+  const int NZ = DEAL ? 2 * NZ2 / 3 : g.nz, NY1 = g.ny1, NXH = g.nxh, ny = g.ny;
+  const int kx = bid.x, j0 = 1 + bid.y * YP, e = bid.z, t = threadIdx.x;   // j0: 1-based first plane
   __shared__ T skz[NZ2];                 // kz of the retained rows (nz <= nz2)
-  load_tw2<T, NZ2>(tw, twz);
-  for (int i = threadIdx.x; i < NZ; i += blockDim.x) skz[i] = (T)gd.kz[i];
-  __syncthreads();
-  for (int t = threadIdx.x; t < nseq * N2; t += blockDim.x) {
-    const int s = t / N2, n2 = t - s * N2;
-    const int jj = s / 6, e = (s / 2) % 3, part = s & 1;
-    const int j = j0 + jj;
-    const bool valid = (j >= 2 && j <= ny) && !(e == 1 && j == ny);
+  auto valid = [&](int j) { return j >= 2 && j <= ny && !(e == 1 && j == ny); };
+  {
+    const int s = t / N2, n2 = t - s * N2, j = j0 + (s >> 1);
     C v[N1];
-    const C* src = T2 + ((((size_t)(j - 1) * 3 + e) * 2 + part) * NXH + kx) * NZ2;
+    const bool act = t < 2 * YP * N2;
+    if (act) {
+      // the loads are in flight while the tables fill
+      const bool ok = valid(j);
+      const C* src = T2 + ((((size_t)(j - 1) * 3 + e) * 2 + (s & 1)) * NXH + kx) * NZ2 + n2;
 #pragma unroll
-    for (int n1 = 0; n1 < N1; ++n1) v[n1] = valid ? src[N2 * n1 + n2] : czero<C>();
-    SmallFFT<T, N1, -1>::template run<1>(v);
-    C* y = Y + s * SEQ + n2;
+      for (int n1 = 0; n1 < N1; ++n1) v[n1] = ok ? src[N2 * n1] : czero<C>();
+    }
+    load_tw2<T, NZ2>(tw, twz);
+    for (int i = t; i < NZ; i += NT) skz[i] = (T)gd.kz[i];
+    __syncthreads();
+    if (act) {
+      SmallFFT<T, N1, -1>::template run<1>(v);
+      C* y = Y + s * SEQ + n2;
 #pragma unroll
-    for (int k1 = 0; k1 < N1; ++k1) {
-      C x = v[k1];
-      if (k1 != 0) x = cmul(x, tw[k1 * N2 + n2]);
-      y[k1 * PITCH] = x;
+      for (int k1 = 0; k1 < N1; ++k1) {
+        C x = v[k1];
+        if (k1 != 0) x = cmul(x, tw[k1 * N2 + n2]);
+        y[k1 * PITCH] = x;
+      }
     }
   }
   __syncthreads();
   const int off = NZ2 - NZ;
-  // stage 2 in rounds of whole sequences: read all rows of the round, then
-  // synchronise before overwriting the exchange buffer with the outputs (the
-  // output of sequence s only overlaps exchange rows of sequences <= s)
-  const int spr = blockDim.x / N1;
-  for (int s0 = 0; s0 < nseq; s0 += spr) {
-    const int s = s0 + (int)threadIdx.x / N1, k1 = (int)threadIdx.x % N1;
-    const bool act = ((int)threadIdx.x < spr * N1) && s < nseq;
+  {
+    // every row is read before the outputs overwrite the exchange buffer
+    const int s = t / N1, k1 = t - s * N1;
+    const bool act = s < 2 * YP;
     C u[N2];
     if (act) {
       const C* y = Y + s * SEQ + k1 * PITCH;
@@ -222,27 +248,26 @@ __device__ __forceinline__ void k_zfwd_r_body(const uint3 bid, const cplx_t<T>* 
     __syncthreads();
     if (act) {
       SmallFFT<T, N2, -1>::template run<1>(u);
-      C* z = Z + s * ZP;
+      C* z = Y + s * ZP;
 #pragma unroll
       for (int k2 = 0; k2 < N2; ++k2) {
         const int k = k1 + N1 * k2;
+        if (DEAL && N1 * k2 > NZ2 / 3 && N1 * k2 + N1 <= NZ2 - NZ2 / 3) continue;
         if (k <= NZ / 2 || k >= off + NZ / 2) z[k] = u[k2];
       }
     }
-    if (s0 + spr < nseq) __syncthreads();
   }
   __syncthreads();
   const T scale = (T)(1.0 / ((double)g.nx2 * (double)g.nz2));
   const T wsc = (g.kx0 + kx == g.nxh_all - 1) ? (T)2 * scale : scale;
-  for (int idx = threadIdx.x; idx < NZ * 3 * YB; idx += blockDim.x) {
-    const int jj = idx % YB, e = (idx / YB) % 3, kz = idx / (3 * YB);
+  for (int idx = t; idx < NZ * YP; idx += NT) {
+    const int jj = idx % YP, kz = idx / YP;
     const int j = j0 + jj;
     if (j > NY1) continue;
-    const bool valid = (j >= 2 && j <= ny) && !(e == 1 && j == ny);
     C out = czero<C>();
-    if (valid) {
-      const C* A = Z + ((jj * 3 + e) * 2 + 0) * ZP;
-      const C* Zc = Z + ((jj * 3 + e) * 2 + 1) * ZP;
+    if (valid(j)) {
+      const C* A = Y + 2 * jj * ZP;
+      const C* Zc = A + ZP;
       C fa, fz;
       if (kz < NZ / 2) { fa = A[kz]; fz = Zc[kz]; }
       else if (kz == NZ / 2) {
@@ -256,11 +281,11 @@ __device__ __forceinline__ void k_zfwd_r_body(const uint3 bid, const cplx_t<T>* 
   }
 }
 
-template <typename T, int NZ2>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2)
+template <typename T, int NZ2, int YP, bool DEAL>
+__global__ void __launch_bounds__(ZShape<T, NZ2, YP>::FWD_NT, ZShape<T, NZ2, YP>::blocks(ZShape<T, NZ2, YP>::FWD_NT, sizeof(T) == 4))
 k_zfwd_r(const cplx_t<T>* __restrict__ T2, cplx_t<T>* __restrict__ vel, Geom g, const cplx_t<T>* __restrict__ twz,
-         GridDev gd, int YB) {
-  k_zfwd_r_body<T, NZ2>(blockIdx, T2, vel, g, twz, gd, YB);
+         GridDev gd) {
+  k_zfwd_r_body<T, NZ2, YP, DEAL>(blockIdx, T2, vel, g, twz, gd);
 }
 
 // --------------------------------------------------------------------------
@@ -977,11 +1002,11 @@ k_flux_r(const T* __restrict__ P, cplx_t<T>* __restrict__ T2, Geom g, const cplx
 }
 
 // smem sizes (bytes) of the three kernels
-template <typename T, int N> size_t zinv_r_smem(int YB, int nz) {
-  return sizeof(cplx_t<T>) * (N + 3 * ((size_t)nz * YB + ZRawPad<T>::V) + (size_t)3 * YB * SeqPitch<N>::V);
+template <typename T, int N, int YP> size_t zinv_r_smem(int nz) {
+  return sizeof(cplx_t<T>) * (N + (size_t)nz * YP + (size_t)YP * ZShape<T, N, YP>::INV_SEQ);
 }
-template <typename T, int N> constexpr size_t zfwd_r_smem(int YB) {
-  return sizeof(cplx_t<T>) * (N + (size_t)6 * YB * SeqPitch<N>::V);
+template <typename T, int N, int YP> constexpr size_t zfwd_r_smem() {
+  return sizeof(cplx_t<T>) * (N + (size_t)2 * YP * ZShape<T, N, YP>::FWD_SEQ);
 }
 template <typename T, int N, int ZB> constexpr size_t xinv_r_smem(int NXH) {
   return sizeof(cplx_t<T>) * (N + (size_t)NXH * RawPitch<T, ZB>::V + (size_t)(ZB / 2) * SeqPitch<N>::V);
