@@ -3,10 +3,10 @@
 // GELU (tanh form) on the three hidden layers, BF16 weights and activations, FP32
 // accumulation in tensor memory (TMEM).
 //
-// One CTA of 128 threads (4 warps) handles a tile of 128 points: thread t owns
-// point t of the tile and TMEM lane t.  Every product is one tcgen05.mma
-// (kind::f16, M = 128, K = 16 per instruction) issued by thread 0, with both
-// operands in shared memory and the accumulator in TMEM; its completion is
+// One CTA of 128 threads (4 warps; training: 256, two per point) handles a
+// tile of 128 points: thread t owns point t of the tile and TMEM lane t.
+// Every product is one tcgen05.mma (kind::f16, M = 128, K = 16 per
+// instruction) issued by thread 0, with both operands in shared memory and the accumulator in TMEM; its completion is
 // signalled by tcgen05.commit on an mbarrier, after which the warps read their
 // 32 TMEM lanes with tcgen05.ld.
 //
@@ -32,6 +32,7 @@ constexpr int IN = 10, H = 64, OUT = 6;
 constexpr int KIN = 16;    // input features padded to one MMA K step
 constexpr int NOUT = 16;   // output rows padded to the smallest M=128 N
 constexpr int TILE = 128;  // points per CTA tile (MMA M)
+constexpr int NTH = 2 * TILE;   // threads per training CTA: two per point
 // flat FP32 parameter vector: W0[H][IN] b0[H] W1[H][H] b1[H] W2[H][H] b2[H] W3[OUT][H] b3[OUT]
 constexpr int OFF_W0 = 0, OFF_B0 = OFF_W0 + H * IN, OFF_W1 = OFF_B0 + H, OFF_B1 = OFF_W1 + H * H,
               OFF_W2 = OFF_B1 + H, OFF_B2 = OFF_W2 + H * H, OFF_W3 = OFF_B2 + H, OFF_B3 = OFF_W3 + OUT * H,
@@ -186,11 +187,13 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
       : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
   return r;
 }
-// gelu of two values, the arithmetic of gelu() two lanes at a time
+// gelu of two values, the arithmetic of gelu() two lanes at a time; TWICE:
+// 2 gelu, the same bits one exponent up
+template <bool TWICE>
 __device__ __forceinline__ float2 gelu2(float2 z) {
   const float2 w = fma2(mul2(z, z), make_float2(kGeluCA, kGeluCA), make_float2(kGeluC, kGeluC));
   const float2 u = mul2(z, w);
-  const float2 h = mul2(z, make_float2(0.5f, 0.5f));
+  const float2 h = TWICE ? z : mul2(z, make_float2(0.5f, 0.5f));
   return fma2(h, make_float2(tanh_hw(u.x), tanh_hw(u.y)), h);
 }
 
@@ -202,6 +205,18 @@ __device__ __forceinline__ uint4 pack8(const float* v) {
   h = __floats2bfloat162_rn(v[2], v[3]); u.y = *reinterpret_cast<uint32_t*>(&h);
   h = __floats2bfloat162_rn(v[4], v[5]); u.z = *reinterpret_cast<uint32_t*>(&h);
   h = __floats2bfloat162_rn(v[6], v[7]); u.w = *reinterpret_cast<uint32_t*>(&h);
+  return u;
+}
+
+// half of 8 BF16 values
+__device__ __forceinline__ uint4 half8(uint4 u) {
+  uint32_t* w = reinterpret_cast<uint32_t*>(&u);
+  const __nv_bfloat162 h = __floats2bfloat162_rn(0.5f, 0.5f);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    __nv_bfloat162 v = __hmul2(*reinterpret_cast<__nv_bfloat162*>(w + i), h);
+    w[i] = *reinterpret_cast<uint32_t*>(&v);
+  }
   return u;
 }
 
