@@ -164,6 +164,7 @@ struct cfg_ctx {
   void* P = nullptr;
   bool split_x = false;
   int flux_zr = 4;
+  bool flux_given = false;   // flux_zr was asked for: products without that block refuse it
   void* cbc = nullptr;   // [bot, top][3][nw]
   DevScalars* sc = nullptr;
   double* d_um_dy = nullptr;
@@ -447,10 +448,19 @@ struct Impl {
     // sets 8, 16 or 24 (the tuners also try them)
     c->xinv_zb = getenv("CHANFLOW_XINV_ROWS") ? atoi(getenv("CHANFLOW_XINV_ROWS")) : 0;
     if (c->xinv_zb != 8 && !(f32 && (c->xinv_zb == 16 || c->xinv_zb == 24))) c->xinv_zb = 0;
-    c->flux_zr = getenv("CHANFLOW_FLUX_ZR") ? atoi(getenv("CHANFLOW_FLUX_ZR")) : (f32 ? 4 : 2);
-    if (c->flux_zr != 2 && !(c->flux_zr == 8 && f32)) c->flux_zr = 4;   // 8 rows: FP32 only
     // (gP: the x stage's geometry, all kx and this rank's z2 rows)
     const Geom& gp = c->gP;
+    // z rows per flux block: in FP32 8 on rows of up to 192 points, where 4
+    // leave a third of its threads idle (4 / 8 rows at 48x49x48, 96x97x96,
+    // 128x200x64 and 128x129x128: 12.7 / 11.6, 38.9 / 34.0, 61.6 / 59.5, 78.1 /
+    // 74.6 us), 4 beyond (192x129x192, 256x193x256: 164 / 196, 405 / 450); 2 in
+    // FP64
+    c->flux_zr = f32 ? (g.nx2 <= 192 && gp.nz2 % 8 == 0 ? 8 : 4) : 2;
+    c->flux_given = getenv("CHANFLOW_FLUX_ZR") != nullptr;
+    if (c->flux_given) {
+      c->flux_zr = atoi(getenv("CHANFLOW_FLUX_ZR"));
+      if (c->flux_zr != 2 && !(c->flux_zr == 8 && f32)) c->flux_zr = 4;   // 8 rows: FP32 only
+    }
     if (c->xinv_zb && gp.nz2 % c->xinv_zb) c->xinv_zb = 0;
     c->split_x = c->fast_x && (!getenv("CHANFLOW_FUSED_XFLUX") || c->nranks > 1) &&
                  (c->nranks == 1 || gp.nz2 % 8 == 0) &&
@@ -512,12 +522,13 @@ struct Impl {
     return CFG_OK;
   }
 
-  // z rows per flux block: the tile where it divides the z2 rows (and, beside
-  // the lengths of regfft_full, where the products have that block), else 4
+  // z rows per flux block: the tile where it divides the z2 rows and the
+  // products have that block (8 rows: not the linearized and the LES ones;
+  // asked for, the lengths of regfft_full leave that to the launch), else 4
   // or 2
   static int flux_rows(const cfg_ctx* c, bool plain_products) {
     const int zr = c->flux_zr, nz2 = c->gP.nz2;
-    if (nz2 % zr == 0 && (zr < 8 || plain_products || regfft_full(c->g.nx2))) return zr;
+    if (nz2 % zr == 0 && (zr < 8 || plain_products || (c->flux_given && regfft_full(c->g.nx2)))) return zr;
     return nz2 % 4 == 0 ? 4 : 2;
   }
   // the launch record of register-FFT pass-1 kernel `which` (0 k_zinv_r, 1
@@ -2756,7 +2767,9 @@ int cfg_autotune(cfg_ctx* c, int trial_steps, int* choice) {
 
   // a row count that does not split, or the 8-row block outside the
   // FP32 nonlinear products, fails its trial
+  const int zr0 = c->flux_zr;
   if (c->split_x) tune(&c->flux_zr, {2, 4, 8});
+  c->flux_given = c->flux_given || c->flux_zr != zr0;
   if (c->fast_z) {
     // planes per z-transform block (a block too large for its launch fails
     // its trial)
@@ -2800,6 +2813,7 @@ int cfg_set_tiles(cfg_ctx* c, const int* tiles) {
     return fail(c, CFG_E_ARG, "cfg_set_tiles: unsupported tiles");
   c->rhs2_warps = w;
   c->flux_zr = fz;
+  c->flux_given = true;
   c->fYB1 = y1;
   c->fYB3 = y3;
   return CFG_OK;
@@ -3282,7 +3296,9 @@ static int ens_tune_batched(cfg_ensemble* e, int trial_steps) {
       for (int i : groups[q]) e->m[i]->*knob = bestv;
     };
     tune(&cfg_ctx::rhs2_warps, {2, 3, 4});
+    const int zr0 = e->m[groups[q][0]]->flux_zr;
     tune(&cfg_ctx::flux_zr, {2, 4, 8});
+    for (int i : groups[q]) e->m[i]->flux_given = e->m[i]->flux_given || e->m[i]->flux_zr != zr0;
     tune(&cfg_ctx::fYB1, {1, 2, 4, 8});
     tune(&cfg_ctx::fYB3, {1, 2, 4, 8});
     tune(&cfg_ctx::xinv_zb, {8, 16, 24});

@@ -615,97 +615,115 @@ __device__ __forceinline__ void cp_async_wait0() { asm volatile("cp.async.wait_g
 // row pitch (complex values) of the gathered hybrid rows: 16 bytes of padding
 // keeps the 16-byte cp.async destinations aligned and the stage-1 reads
 // (consecutive threads on consecutive kx) free of bank conflicts
-template <int N, int ZB> __host__ __device__ constexpr int xinv_threads() {
-  return ((ZB / 2) * Split<N>::N2 + 31) / 32 * 32 < 128 ? 128
-       : (((ZB / 2) * Split<N>::N2 + 31) / 32 * 32 > 256 ? 256 : ((ZB / 2) * Split<N>::N2 + 31) / 32 * 32);
-}
-
 template <typename T, int ZB> struct RawPitch {
   static constexpr int V = ZB + 16 / (int)sizeof(cplx_t<T>);
 };
 
-// k_xinv_r: grid (ceil(nz2/ZB), 3, ny+1), block xinv_threads (one thread per
-// stage-1 task, at least 128).  Inverse x transform of ZB
-// hybrid rows (one plane, one component) into physical rows, two real rows per
-// complex FFT (the x part of xz_fft_complex_to_real_parallel,
+// one thread per task in both stages
+template <int N, int ZB> __host__ __device__ constexpr int xinv_threads() {
+  return (ZB / 2 * (Split<N>::N1 > Split<N>::N2 ? Split<N>::N1 : Split<N>::N2) + 31) / 32 * 32;
+}
+
+// k_xinv_r: grid (ceil(nz2/ZB), 3, ny+1), block xinv_threads.  Inverse x
+// transform of ZB hybrid rows (one plane, one component) into physical rows,
+// two real rows per complex FFT (the x part of xz_fft_complex_to_real_parallel,
 // PFC/transform.f90:345-368).  v of plane ny+1 is not formed: no flux reads it.
 // The last block of an nz2 that ZB does not divide (nz2 is even) takes the
-// rows that are left.
-template <typename T, int NX2, int ZB>
+// rows that are left.  With 3/2 dealiasing (DEAL: nx = 2 nx2/3) the third of
+// the inputs that is zero is known at compile time; the exchange buffer takes
+// the gathered rows' place once they are in registers, for five blocks per SM
+// where the two beside each other left four.  us per launch, before / now:
+// 133 / 106 at 256x193x256 mixed (5.4 TB/s), 389 / 256 at 384x193x384, 304 /
+// 220 in FP64 at 256x193x256.
+template <typename T, int NX2, int ZB, bool DEAL>
 __device__ __forceinline__ void k_xinv_r_body(const uint3 bid, const cplx_t<T>* __restrict__ T1, T* __restrict__ P,
                                               Geom g, const cplx_t<T>* __restrict__ twx) {
   using C = cplx_t<T>;
   constexpr int N1 = Split<NX2>::N1, N2 = Split<NX2>::N2, PITCH = N2 + 1, SEQ = SeqPitch<NX2>::V;
-  constexpr int N = NX2, Nh = NX2 / 2, RP = RawPitch<T, ZB>::V;
+  constexpr int N = NX2, Nh = NX2 / 2, RP = RawPitch<T, ZB>::V, NT = xinv_threads<NX2, ZB>();
   constexpr int CH = ZB * (int)sizeof(C) / 16;   // 16-byte chunks per hybrid row
   static_assert(ZB % 2 == 0 && (ZB * sizeof(C)) % 16 == 0, "ZB rows must pack in pairs and 16-byte chunks");
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int NXH = g.nxh, NZ2 = g.nz2;
+  const int NXH = DEAL ? NX2 / 3 + 1 : g.nxh, NZ2 = g.nz2;
   C* tw = reinterpret_cast<C*>(smem_raw);   // [N]
   C* raw = tw + N;                          // [NXH][RP]
-  C* Y = raw + NXH * RP;                    // [ZB/2][SEQ]
-  const int z0 = bid.x * ZB, c = bid.y, pl = bid.z;
+  C* Y = raw;                               // [ZB/2][SEQ], after raw
+  const int z0 = bid.x * ZB, c = bid.y, pl = bid.z, t = threadIdx.x;
   if (c == 1 && pl == g.ny) return;
   const int rows = min(ZB, NZ2 - z0), ch = rows * (int)sizeof(C) / 16, ns = rows / 2;
   const C* src = T1 + ((size_t)pl * 3 + c) * NXH * NZ2 + z0;
-  for (int idx = threadIdx.x; idx < NXH * CH; idx += blockDim.x) {
+  for (int idx = t; idx < NXH * CH; idx += NT) {
     const int kx = idx / CH, part = idx - kx * CH;
-    if (part < ch) cp_async16(reinterpret_cast<char*>(raw + kx * RP) + part * 16,
-               reinterpret_cast<const char*>(src + (size_t)kx * NZ2) + part * 16);
+    if (part < ch)
+      cp_async16(reinterpret_cast<char*>(raw + kx * RP) + part * 16,
+                 reinterpret_cast<const char*>(src + (size_t)kx * NZ2) + part * 16);
   }
   cp_async_commit();
   load_tw2<T, N>(tw, twx);
   cp_async_wait0();
   __syncthreads();
-  for (int t = threadIdx.x; t < ns * N2; t += blockDim.x) {
+  {
     const int i = t / N2, n2 = t - i * N2;
+    const bool act = i < ns;
     C v[N1];
+    if (act) {
+      // the two real rows' spectra x1, x2 at k as those of x1 + i x2
+      struct __align__(16) Pair { C a, b; };
 #pragma unroll
-    for (int n1 = 0; n1 < N1; ++n1) {
-      const int k = N2 * n1 + n2;
-      const int kk = (k <= Nh) ? k : N - k;
-      C x1 = czero<C>(), x2 = czero<C>();
-      if (kk < NXH) {
-        x1 = raw[kk * RP + 2 * i];
-        x2 = raw[kk * RP + 2 * i + 1];
+      for (int n1 = 0; n1 < N1; ++n1) {
+        const int k = N2 * n1 + n2;
+        const bool zero = DEAL && N2 * n1 > N / 3 && N2 * n1 + N2 <= N - N / 3;
+        const bool low = DEAL && N2 * n1 + N2 <= N / 3, high = DEAL && N2 * n1 > N - N / 3;
+        const int kk = low || (!high && k <= Nh) ? k : N - k;
+        C z = czero<C>();
+        if (!zero && (low || high || kk < NXH)) {
+          const Pair x = *reinterpret_cast<const Pair*>(raw + kk * RP + 2 * i);
+          if ((!high && k == 0) || (!low && !high && k == Nh)) z = mk<C>(x.a.x, x.b.x);
+          else if (low || (!high && k < Nh)) z = mk<C>(x.a.x - x.b.y, x.a.y + x.b.x);
+          else z = mk<C>(x.a.x + x.b.y, -x.a.y + x.b.x);
+        }
+        v[n1] = z;
       }
-      C z;
-      if (k == 0 || k == Nh) z = mk<C>(x1.x, x2.x);
-      else if (k < Nh) z = mk<C>(x1.x - x2.y, x1.y + x2.x);
-      else z = mk<C>(x1.x + x2.y, -x1.y + x2.x);
-      v[n1] = z;
     }
-    SmallFFT<T, N1, +1>::template run<1>(v);
-    C* y = Y + i * SEQ + n2;
+    __syncthreads();
+    if (act) {
+      SmallFFT<T, N1, +1>::template run<1>(v);
+      C* y = Y + i * SEQ + n2;
 #pragma unroll
-    for (int q = 0; q < N1; ++q) {
-      C x = v[q];
-      if (q != 0) x = cmul(x, cconj(tw[q * N2 + n2]));
-      y[q * PITCH] = x;
+      for (int q = 0; q < N1; ++q) {
+        C x = v[q];
+        if (q != 0) x = cmul(x, cconj(tw[q * N2 + n2]));
+        y[q * PITCH] = x;
+      }
     }
   }
   __syncthreads();
-  for (int t = threadIdx.x; t < ns * N1; t += blockDim.x) {
-    const int q = t % N1, i = t / N1;
+  const int q = t % N1, i = t / N1;
+  if (i < ns) {
     C u[N2];
     const C* y = Y + i * SEQ + q * PITCH;
 #pragma unroll
     for (int n2 = 0; n2 < N2; ++n2) u[n2] = y[n2];
     SmallFFT<T, N2, +1>::template run<1>(u);
-    T* w1 = P + (((size_t)pl * 3 + c) * NZ2 + z0 + 2 * i) * N;
+    T* w1 = P + (((size_t)pl * 3 + c) * NZ2 + z0 + 2 * i) * N + q;
     T* w2 = w1 + N;
 #pragma unroll
     for (int k2 = 0; k2 < N2; ++k2) {
-      w1[q + N1 * k2] = u[k2].x;
-      w2[q + N1 * k2] = u[k2].y;
+      w1[N1 * k2] = u[k2].x;
+      w2[N1 * k2] = u[k2].y;
     }
   }
 }
 
-template <typename T, int NX2, int ZB>
-__global__ void __launch_bounds__(256)
+template <typename T, int N, int ZB> constexpr int xinv_blocks() {
+  constexpr int nt = xinv_threads<N, ZB>(), r = sizeof(T) == 4 ? 64 : ZShape<T, N, 1>::regs(false);
+  return 65536 / (nt * r) > 0 ? (65536 / (nt * r) > 32 ? 32 : 65536 / (nt * r)) : 1;
+}
+
+template <typename T, int NX2, int ZB, bool DEAL>
+__global__ void __launch_bounds__(xinv_threads<NX2, ZB>(), xinv_blocks<T, NX2, ZB>())
 k_xinv_r(const cplx_t<T>* __restrict__ T1, T* __restrict__ P, Geom g, const cplx_t<T>* __restrict__ twx) {
-  k_xinv_r_body<T, NX2, ZB>(blockIdx, T1, P, g, twx);
+  k_xinv_r_body<T, NX2, ZB, DEAL>(blockIdx, T1, P, g, twx);
 }
 
 // k_flux_r: grid (nz2/ZR, ny-1), block NT.  Fluxes of plane k = 2 + blockIdx.y
@@ -1009,7 +1027,8 @@ template <typename T, int N, int YP> constexpr size_t zfwd_r_smem() {
   return sizeof(cplx_t<T>) * (N + (size_t)2 * YP * ZShape<T, N, YP>::FWD_SEQ);
 }
 template <typename T, int N, int ZB> constexpr size_t xinv_r_smem(int NXH) {
-  return sizeof(cplx_t<T>) * (N + (size_t)NXH * RawPitch<T, ZB>::V + (size_t)(ZB / 2) * SeqPitch<N>::V);
+  const size_t raw = (size_t)NXH * RawPitch<T, ZB>::V, y = (size_t)(ZB / 2) * SeqPitch<N>::V;
+  return sizeof(cplx_t<T>) * (N + (raw > y ? raw : y));
 }
 template <typename T, int N, int ZR> constexpr size_t flux_r_smem() {
   return sizeof(cplx_t<T>) * (N + (size_t)(4 * ZR) * FluxSeq<T, N>::V);

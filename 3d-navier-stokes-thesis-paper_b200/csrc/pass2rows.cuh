@@ -49,6 +49,7 @@ template <typename T, int NM, int NR>
 __device__ __forceinline__ void pcr_rows(T (&a)[NM], T (&c)[NM], T (&e)[NM], cplx_t<T> (&f)[NR], int n, void* buf) {
   using C = cplx_t<T>;
   const int j = threadIdx.x, nt = blockDim.x;
+  const T tiny = (T)1e-30;   // couplings that no longer reach the last bit
   T* const base = reinterpret_cast<T*>(buf);
   const int half = nt * (3 * NM + 2 * NR + (NM & 1));   // (complex values stay aligned)
   int h = 0;
@@ -64,7 +65,11 @@ __device__ __forceinline__ void pcr_rows(T (&a)[NM], T (&c)[NM], T (&e)[NM], cpl
     }
 #pragma unroll
     for (int r = 0; r < NR; ++r) fs[r * nt + j] = f[r];
-    __syncthreads();
+    // decoupled rows (a viscous step couples a row to few neighbours): done
+    bool open = false;
+#pragma unroll
+    for (int m = 0; m < NM; ++m) open = open || a[m] > tiny || c[m] > tiny;
+    if (!__syncthreads_or(open)) break;
     // a coupling past an end is zero: the clamped neighbour's values drop out
     const int l = max(j - s, 0), u = min(j + s, nt - 1);
     T rb[NM], fa[NM], fc[NM];
