@@ -210,6 +210,7 @@ struct cfg_ctx {
   bool full_len = false;   // nx2 of regfft_full and nz2 rows in eights (the LES mode)
   bool use_rhs2 = true;
   int rhs2_lanes = 32;
+  bool chained = false;   // a time step is being enqueued: dependent launches (launch_chained)
   bool advance = false;   // the solve being enqueued ends the step (t_total += dt)
   bool rhs_rows = false;  // small grid: every wavenumber in k_rhs_rows, one launch
   int rhs2_warps = 3;   // warps (wavenumbers) per k_rhs2 block
@@ -540,6 +541,7 @@ struct Impl {
     a.gd = c->gd; a.fringe = c->fringe; a.has_fringe = c->has_fringe;
     a.YB1 = c->fYB1; a.YB3 = c->fYB3;
     a.ZR = c->fZR; a.cflbits = c->cflbits; a.do_cfl = (rk == 1); a.lin = lin ? 1 : 0; a.st = c->st;
+    a.pdl = c->chained ? 1 : 0;
     a.KC = (int)std::max(2L, std::min(16L, (long)(g.ny - 1) * (g.nz2 / c->fZR) / 592));
     a.P = c->P;
     a.FZR = flux_rows(c, !lin && !c->les_on);
@@ -594,6 +596,7 @@ struct Impl {
         if (p1_fast_launch(3, g.nx2, f32, a) != 0) return fail(c, CFG_E_CUDA, "k_xinv_r launch");
         CKL();
         a = p1_args(c, rk, lin, 4);
+        a.keep = step < 0;
         if (c->les_on && !lin) {
           const int r = les_stresses(c, c->les_F);
           if (r) return r;
@@ -634,12 +637,8 @@ struct Impl {
       // (the other ranks may still read this rank's maxima)
       const int reset = c->nranks == 1;
       prof_begin(c, "k_cfl_finalize");
-      if (lin)
-        k_cfl_finalize<true><<<1, 256, 0, c->st>>>(c->cflbits, reset, g, c->gd, c->sc, c->cflp, c->p.lx, c->p.lz,
-                                                    c->p.dt_flag, c->p.cfl_max, step);
-      else
-        k_cfl_finalize<false><<<1, 256, 0, c->st>>>(c->cflbits, reset, g, c->gd, c->sc, c->cflp, c->p.lx, c->p.lz,
-                                                     c->p.dt_flag, c->p.cfl_max, step);
+      launch_chained(c->chained, lin ? k_cfl_finalize<true> : k_cfl_finalize<false>, dim3(1), dim3(256), 0, c->st,
+                     c->cflbits, reset, g, c->gd, c->sc, c->cflp, c->p.lx, c->p.lz, c->p.dt_flag, c->p.cfl_max, step);
       CKL();
       c->cfl_clean = reset;
     }
@@ -710,6 +709,7 @@ struct Impl {
       a.wlist = c->wl_fast; a.nlist = c->n_fast; a.warps = c->rhs2_warps; a.lanes = c->rhs2_lanes;
       a.tbl = c->rhs2_tbl;
       a.st = c->st;
+      a.pdl = c->chained ? 1 : 0;
     }
     return a;
   }
@@ -739,6 +739,7 @@ struct Impl {
     m.wlist = c->wl_prec; m.nlist = c->n_prec;
     m.wfast = c->wl_fast; m.nfast = c->rhs_rows ? c->n_fast : 0;
     m.st = c->rhs_rows ? c->st : c->st2;
+    m.pdl = c->chained && c->rhs_rows ? 1 : 0;   // (the side stream's launch follows an event)
     return m;
   }
 
@@ -1459,11 +1460,11 @@ static int timestep_impl(cfg_ctx* c, int nsteps, bool lin) {
   if (!c || nsteps < 0) return CFG_E_ARG;
   if (c->nranks > 1) return single_only(c, "cfg_timestep");
   cudaSetDevice(c->dev);
-  for (int s = 0; s < nsteps; ++s) {
-    const int r = step_enqueue(c, lin);
-    if (r) return r;
-  }
-  return CFG_OK;
+  c->chained = true;
+  int r = CFG_OK;
+  for (int s = 0; s < nsteps && !r; ++s) r = step_enqueue(c, lin);
+  c->chained = false;
+  return r;
 }
 
 int cfg_timestep(cfg_ctx* c, int nsteps) { return timestep_impl(c, nsteps, false); }

@@ -86,6 +86,34 @@ struct Scatter {
   const long long* xpitch;
 };
 
+// Programmatic dependent launch: the kernels of a step's chain let the next
+// one's blocks start once their own have all started, and wait for the
+// previous kernel's results before they touch them, so that a launch and the
+// fill of the SMs run under the previous kernel's last blocks (a chain of
+// twelve 5 us kernels a step on the smallest grids).  Without the launch
+// attribute both are no-ops.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename K, typename... A>
+inline void launch_chained(bool pdl, K kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  if (!pdl) {
+    kernel<<<grid, block, smem, st>>>(args...);
+    return;
+  }
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // FFT plan for one length: Stockham passes, radices in {2,3,4,8}.
 struct FftPlan {
   int n, npass;

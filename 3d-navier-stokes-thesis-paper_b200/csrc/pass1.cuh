@@ -357,6 +357,8 @@ __device__ __forceinline__ void k_cfl_finalize_body(const uint3 bid, unsigned lo
                                                     double lz, int dt_flag, double cfl_max_param, int step) {
   __shared__ double smax[256];
   const int ny = g.ny;
+  pdl_trigger();
+  pdl_wait();
   const double dt = sc->dt;
   double m = 0;
   int bad = 0;

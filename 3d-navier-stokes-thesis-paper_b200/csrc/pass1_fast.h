@@ -29,6 +29,8 @@ struct P1Launch {
   int split;            // mean split: k_zinv_r drops the mean column, k_flux_r adds it from mean64
   const double2* mean64;   // the velocity's mean column, FP64 (ny+1, 3)
   int XZB;              // z2 rows per k_xinv_r block: 8, 16 or 24 (FP32), 0 for the default
+  int keep;             // the initial pressure: FLUX_KEEP
+  int pdl;              // launched as the dependent of the kernel before it
   cudaStream_t st;
 };
 

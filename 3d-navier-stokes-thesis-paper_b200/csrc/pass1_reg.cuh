@@ -18,9 +18,8 @@ template <int N> struct SeqPitch {
 
 // Stage-1 twiddles W_N^(n2*q) stored as tw2[q*N2 + n2] so that consecutive
 // threads (consecutive n2) read consecutive words.
-template <typename T, int N>
+template <typename T, int N, int N1 = Split<N>::N1, int N2 = Split<N>::N2>
 __device__ __forceinline__ void load_tw2(cplx_t<T>* tw2, const cplx_t<T>* __restrict__ tw) {
-  constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2;
   for (int i = threadIdx.x; i < N1 * N2; i += blockDim.x) {
     const int q = i / N2, n2 = i - q * N2;
     tw2[i] = tw[n2 * q];
@@ -95,6 +94,8 @@ __device__ __forceinline__ void k_zinv_r_body(const uint3 bid, const cplx_t<T>* 
   const int nj = min(YP, NY1 - j0);
   const C* col = vel + ((size_t)kx * NZ * 3 + c) * NY1 + j0;
   const size_t kzs = (size_t)3 * NY1;
+  pdl_trigger();
+  pdl_wait();
   // 16-byte pieces need 16-byte aligned runs: whole groups of rows of even length
   if (YP * sizeof(C) % 16 == 0 && nj == YP && (sizeof(C) == 16 || NY1 % 2 == 0)) {
     constexpr int NP = YP * (int)sizeof(C) / 16 > 0 ? YP * (int)sizeof(C) / 16 : 1;
@@ -208,6 +209,8 @@ __device__ __forceinline__ void k_zfwd_r_body(const uint3 bid, const cplx_t<T>* 
   const int kx = bid.x, j0 = 1 + bid.y * YP, e = bid.z, t = threadIdx.x;   // j0: 1-based first plane
   __shared__ T skz[NZ2];                 // kz of the retained rows (nz <= nz2)
   auto valid = [&](int j) { return j >= 2 && j <= ny && !(e == 1 && j == ny); };
+  pdl_trigger();
+  pdl_wait();
   {
     const int s = t / N2, n2 = t - s * N2, j = j0 + (s >> 1);
     C v[N1];
@@ -598,9 +601,26 @@ template <> struct FluxSeqPad<324> { static constexpr int D = 12; };
 template <> struct FluxSeqPad<384> { static constexpr int D = 8; };
 template <> struct FluxSeqPad<432> { static constexpr int D = 10; };
 template <> struct FluxSeqPad<576> { static constexpr int D = 0; };
-template <typename T, int N> struct FluxSeq {
+// MODE of k_flux_r + FLUX_KEEP: the same products with the factorisation of
+// Split<N>.  The learned closure amplifies last bits (step_keeps_sums in
+// capi.cu), so the subgrid mode and the initial pressure, from which its runs
+// start, keep that one.
+constexpr int FLUX_KEEP = 16;
+
+// Factorisation and layout of k_flux_r's transforms in FP32: with N2 = 16 the row
+// pitch N2 + 1 skews every 16 values by one bank pair, which frees the point
+// phase's stores too (a thread's two neighbouring points put its lanes two
+// values apart: twice the wavefronts with any other N2) and leaves no padding
+// between the sequences.  Wavefronts per row by the model above, before / now:
+// 220 / 147 at 96 points, 256 / 232 at 144, 340 / 293 at 192, 534 / 464 at
+// 288, 676 / 612 at 384.
+// us per launch, before / now: 39 / 32 at 96x97x96, 62 / 51 at 128x200x64, 78 /
+// 64 at 128x129x128 (with 8 rows per block), 405 / 383 at 256x193x256.
+template <typename T, int N, int MODE> struct FluxSplit {
+  static constexpr bool N16 = sizeof(T) == 4 && MODE != 2 && MODE < FLUX_KEEP && (N == 96 || N == 144 || N == 192 || N == 288 || N == 384);
+  static constexpr int N1 = N16 ? N / 16 : Split<N>::N1, N2 = N16 ? 16 : Split<N>::N2;
   static constexpr bool ROWMAJOR = sizeof(T) == 8 && (N == 384 || N == 576);
-  static constexpr int V = ROWMAJOR ? SeqPitch<N>::V : Split<N>::N1 * (Split<N>::N2 + 1) + FluxSeqPad<N>::D;
+  static constexpr int SEQ = ROWMAJOR ? SeqPitch<N>::V : N1 * (N2 + 1) + (N16 ? 0 : FluxSeqPad<N>::D);
   static constexpr bool EMAJOR = !ROWMAJOR;
 };
 
@@ -649,6 +669,8 @@ __device__ __forceinline__ void k_xinv_r_body(const uint3 bid, const cplx_t<T>* 
   C* raw = tw + N;                          // [NXH][RP]
   C* Y = raw;                               // [ZB/2][SEQ], after raw
   const int z0 = bid.x * ZB, c = bid.y, pl = bid.z, t = threadIdx.x;
+  pdl_trigger();
+  pdl_wait();
   if (c == 1 && pl == g.ny) return;
   const int rows = min(ZB, NZ2 - z0), ch = rows * (int)sizeof(C) / 16, ns = rows / 2;
   const C* src = T1 + ((size_t)pl * 3 + c) * NXH * NZ2 + z0;
@@ -741,18 +763,32 @@ k_xinv_r(const cplx_t<T>* __restrict__ T1, T* __restrict__ P, Geom g, const cplx
 // (components 11, 22, 33, 12, 13, 23; zero on the walls), added to the
 // momentum fluxes at the same points (y-plane values interpolated as the
 // velocities are: half sums for the u and w equations, iu for the v one).
+// threads and blocks per SM of a flux block: 576-point rows (81 KB for four
+// in FP32 or 86 KB for two in FP64, two blocks per SM) take one thread per
+// task of either stage, 384 or 192 (384x193x384 with 256 / 384 threads: 1153 /
+// 943 us; FP64 with 128 / 192: 2563 / 1825)
+template <typename T, int N, int ZR> __host__ __device__ constexpr int flux_threads() {
+  return ZR == 2 ? (sizeof(T) == 8 && N == 576 ? 192 : 128) : (sizeof(T) == 4 && N == 576 && ZR == 4 ? 384 : 256);
+}
+template <typename T, int NT> __host__ __device__ constexpr int flux_blocks() {
+  return sizeof(T) == 4 ? (NT == 384 ? 2 : NT == 256 ? 4 : 6) : (NT == 256 ? 1 : NT == 192 ? 2 : 3);
+}
+
 template <typename T, int NX2, int ZR, int NT, int MODE>
 __device__ __forceinline__ void k_flux_r_body(const uint3 bid, const T* __restrict__ P, cplx_t<T>* __restrict__ T2,
                                               Geom g, const cplx_t<T>* __restrict__ twx, GridDev gd,
                                               const T* __restrict__ fringe, int has_fringe,
                                               unsigned long long* __restrict__ cflbits, int do_cfl, Scatter sc,
                                               const T* __restrict__ S, const double2* __restrict__ mean64) {
-  constexpr bool LIN = MODE == 1, SGS = MODE == 2, SPLIT = MODE == 3;
+  constexpr int PROD = MODE % FLUX_KEEP;
+  constexpr bool LIN = PROD == 1, SGS = PROD == 2, SPLIT = PROD == 3;
+  constexpr bool OLDSUM = SGS || MODE >= FLUX_KEEP;
   constexpr bool HASB = LIN || SPLIT;
   using C = cplx_t<T>;
-  constexpr int N1 = Split<NX2>::N1, N2 = Split<NX2>::N2, PITCH = N2 + 1, SEQ = FluxSeq<T, NX2>::V;
+  using FS = FluxSplit<T, NX2, MODE>;
+  constexpr int N1 = FS::N1, N2 = FS::N2, PITCH = N2 + 1, SEQ = FS::SEQ;
   // sequence of component pair e of row r
-  auto sidx = [](int r, int e) { return FluxSeq<T, NX2>::EMAJOR ? e * ZR + r : 4 * r + e; };
+  auto sidx = [](int r, int e) { return FS::EMAJOR ? e * ZR + r : 4 * r + e; };
   constexpr int N = NX2;
   // four packed sequences per row: (xfu,dyu) (xfw,dyw) (xfv,dyv) (zfw,zfv);
   // zfu = w*u equals xfw = u*w (and likewise in the linearized products), so
@@ -765,10 +801,13 @@ __device__ __forceinline__ void k_flux_r_body(const uint3 bid, const T* __restri
   __shared__ T red[3][NW];
   __shared__ T skx[NX2 / 2 + 2];             // kx of the retained columns (nx/2+1 <= nx2/2+1)
   const int NXH = g.nxh, NZ2 = g.nz2, ny = g.ny;
+  const bool deal = 3 * (NXH - 1) == N;
   const int z0 = bid.x * ZR;
   const int k = 2 + bid.y;
-  load_tw2<T, N>(tw, twx);
+  pdl_trigger();
+  load_tw2<T, N, N1, N2>(tw, twx);
   for (int i = threadIdx.x; i < g.nxh; i += NT) skx[i] = (T)gd.kx[i];
+  pdl_wait();
   auto px = [](int x) { return (x / N2) * PITCH + (x % N2); };
   const T half = (T)0.5, two = (T)2.0;
   const T dhk = (T)gd.dh[k - 1];
@@ -851,8 +890,18 @@ __device__ __forceinline__ void k_flux_r_body(const uint3 bid, const T* __restri
   }
   // the fringe acts on the whole velocity (its mean included when split)
   const T Uf = SPLIT ? U + B0[0] : U, Wf = SPLIT ? W + B0[2] : W, Vf = SPLIT ? V + B0[1] : V;
-  const T dyu = dhk * (fpu - fpu0) + fr * (Uf - tu);
-  const T dyw = dhk * (fpw - fpw0) + fr * (Wf - tw_);
+  T dyu, dyw;
+  if (OLDSUM) {
+    dyu = dhk * (fpu - fpu0) + fr * (Uf - tu);
+    dyw = dhk * (fpw - fpw0) + fr * (Wf - tw_);
+  } else {
+    dyu = dhk * (fpu - fpu0);
+    dyw = dhk * (fpw - fpw0);
+    if (has_fringe) {
+      dyu += fr * (Uf - tu);
+      dyw += fr * (Wf - tw_);
+    }
+  }
   T xfv = 0, dyv = 0, zfv = 0;
   if (veq) {
     T fp0 = 0, fp = 0;
@@ -881,7 +930,12 @@ __device__ __forceinline__ void k_flux_r_body(const uint3 bid, const T* __restri
       xfv += B0[1] * (iu1 * U + iu2 * Up) + V * (iu1 * B0[0] + iu2 * Bp[0]);
       zfv += B0[1] * (iu1 * W + iu2 * Wp) + V * (iu1 * B0[2] + iu2 * Bp[2]);
     }
-    dyv = dnk * (fp - fp0) + fr * (Vf - tv);
+    if (OLDSUM) {
+      dyv = dnk * (fp - fp0) + fr * (Vf - tv);
+    } else {
+      dyv = dnk * (fp - fp0);
+      if (has_fringe) dyv += fr * (Vf - tv);
+    }
   }
   const int pxx = px(x);
   (void)zfu;
@@ -977,8 +1031,15 @@ __device__ __forceinline__ void k_flux_r_body(const uint3 bid, const T* __restri
 #pragma unroll
     for (int n2 = 0; n2 < N2; ++n2) u[n2] = row[n2];
     SmallFFT<T, N2, -1>::template run<1>(u);
+    // with 3/2 dealiasing the middle third of the spectrum is not read
 #pragma unroll
-    for (int k2 = 0; k2 < N2; ++k2) row[k2] = u[k2];
+    for (int k2 = 0; k2 < N2; ++k2)
+      if (!(N1 * k2 > N / 3 && N1 * k2 + N1 <= N - N / 3)) row[k2] = u[k2];
+    if (!deal) {
+#pragma unroll
+      for (int k2 = 0; k2 < N2; ++k2)
+        if (N1 * k2 > N / 3 && N1 * k2 + N1 <= N - N / 3) row[k2] = u[k2];
+    }
   }
   __syncthreads();
   auto X = [&](int i, int kk) -> C { return FP[i * SEQ + (kk % N1) * PITCH + kk / N1]; };
@@ -1011,7 +1072,7 @@ __device__ __forceinline__ void k_flux_r_body(const uint3 bid, const T* __restri
 }
 
 template <typename T, int NX2, int ZR, int NT, int MODE>
-__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? (NT == 256 ? 4 : 6) : (NT == 256 ? 1 : 3))
+__global__ void __launch_bounds__(NT, flux_blocks<T, NT>())
 k_flux_r(const T* __restrict__ P, cplx_t<T>* __restrict__ T2, Geom g, const cplx_t<T>* __restrict__ twx, GridDev gd,
          const T* __restrict__ fringe, int has_fringe, unsigned long long* __restrict__ cflbits, int do_cfl,
          Scatter sc, const T* __restrict__ S, const double2* __restrict__ mean64) {
@@ -1030,8 +1091,8 @@ template <typename T, int N, int ZB> constexpr size_t xinv_r_smem(int NXH) {
   const size_t raw = (size_t)NXH * RawPitch<T, ZB>::V, y = (size_t)(ZB / 2) * SeqPitch<N>::V;
   return sizeof(cplx_t<T>) * (N + (raw > y ? raw : y));
 }
-template <typename T, int N, int ZR> constexpr size_t flux_r_smem() {
-  return sizeof(cplx_t<T>) * (N + (size_t)(4 * ZR) * FluxSeq<T, N>::V);
+template <typename T, int N, int ZR, int MODE> constexpr size_t flux_r_smem() {
+  return sizeof(cplx_t<T>) * (N + (size_t)(4 * ZR) * FluxSplit<T, N, MODE>::SEQ);
 }
 template <typename T, int N> constexpr size_t xflux_r_smem(int ZR, int NXH) {
   return sizeof(cplx_t<T>) * N + sizeof(T) * 9 * (size_t)ZR * N + sizeof(cplx_t<T>) * (6 * (size_t)ZR * NXH)

@@ -29,8 +29,8 @@ int rhs_rows_launch_batch(bool f32, const RhsRowsLaunch& a, const RhsRowsLaunch*
   const size_t sm = rhs_rows_smem(a.g.ny1);
   if (tab && f32) k_rhs_rows_b<float><<<gx * nmem, nt, sm, a.st>>>(tab, gx);
   else if (tab) k_rhs_rows_b<double><<<gx * nmem, nt, sm, a.st>>>(tab, gx);
-  else if (f32) k_rhs_rows<float><<<gx, nt, sm, a.st>>>(a);
-  else k_rhs_rows<double><<<gx, nt, sm, a.st>>>(a);
+  else if (f32) launch_chained(a.pdl, k_rhs_rows<float>, dim3(gx), dim3(nt), sm, a.st, a);
+  else launch_chained(a.pdl, k_rhs_rows<double>, dim3(gx), dim3(nt), sm, a.st, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

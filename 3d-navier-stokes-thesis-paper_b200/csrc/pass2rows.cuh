@@ -130,6 +130,8 @@ __device__ __forceinline__ void k_rhs_rows_body(int w, bool mean, const RhsRowsL
   C* const sV = reinterpret_cast<C*>(smem_raw);   // 3 columns of nt rows
   C* const sP = sV + 3 * nt;                      // 1 column
   const C zero = czero<C>();
+  pdl_trigger();
+  pdl_wait();
 
   // this row of cru, the nonlinear term and the pressure
   C cr[3], nl[3], p = zero;

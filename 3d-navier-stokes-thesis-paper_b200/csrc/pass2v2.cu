@@ -51,9 +51,9 @@ static int launch_m(const Rhs2Launch& a, const Rhs2Launch* tab, int nmem) {
   if (tab)
     k_rhs2_b<T, T, M, G><<<gr.x * (unsigned)nmem, 32 * a.warps, sm, a.st>>>(tab, gr.x);
   else
-    k_rhs2<T, T, M, G><<<gr, 32 * a.warps, sm, a.st>>>((C*)a.vel, (C*)a.cru, (C*)a.prs, (const C*)a.cbc_top,
-                                                    (const C*)a.cbc_bot, a.g, a.gd, a.sc, a.rkt, a.rk, a.re, a.wlist,
-                                                    a.nlist, (const T*)a.tbl);
+    launch_chained(a.pdl, k_rhs2<T, T, M, G>, gr, dim3(32 * a.warps), sm, a.st, (C*)a.vel, (C*)a.cru, (C*)a.prs,
+                   (const C*)a.cbc_top, (const C*)a.cbc_bot, a.g, a.gd, a.sc, a.rkt, a.rk, a.re, a.wlist, a.nlist,
+                   (const T*)a.tbl);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

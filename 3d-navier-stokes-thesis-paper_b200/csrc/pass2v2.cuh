@@ -191,6 +191,8 @@ __device__ __forceinline__ void k_rhs2_body(const uint3 bid, cplx_t<S>* __restri
   CS* gcru = cru + (size_t)w * 3 * n1;
   CS* gprs = prs + (size_t)w * n1;
 
+  pdl_trigger();
+  pdl_wait();
   // ---- asynchronous staging of the seven input columns: cru (u,v,w), p, NL (u,v,w)
   if (valid && sizeof(S) != sizeof(T)) {
     // widening copy (mixed storage, FP64 arithmetic)

@@ -21,6 +21,7 @@ struct Rhs2Launch {
   int warps;   // warps per block
   int lanes;   // lanes per wavenumber: 32, or 16 or 8 (FP32 only)
   const void* tbl;   // coefficient table of rhs2_table for these lanes
+  int pdl;           // launched as the dependent of the kernel before it
   cudaStream_t st;
 };
 
@@ -73,6 +74,7 @@ struct RhsRowsLaunch {
   int nlist;
   const int* wfast;           // the fast list, nfast 0 where k_rhs2 takes it
   int nfast;
+  int pdl;
   cudaStream_t st;
 };
 int rhs_rows_launch(bool f32, const RhsRowsLaunch& a);
