@@ -127,7 +127,7 @@ struct cfg_ctx {
   // side stream: the small mean-mode and FP64 low-|k| solves run beside the
   // main per-wavenumber kernel; joined back with events
   cudaStream_t st2 = nullptr, st3 = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_join3 = nullptr, ev_jet = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_join3 = nullptr, ev_jet = nullptr, ev_len = nullptr;
   int jet_rk = 0;   // substep whose wall jet is enqueued on st2 (ev_jet)
   // background file output (restart file, VTK snapshot): the layout kernel
   // runs on st, the copy to pinned host memory on st_io, the file write on
@@ -250,7 +250,7 @@ struct cfg_ctx {
   cfg_mlp* les_mlp = nullptr;
   void* les_S = nullptr;
   float* les_F = nullptr;
-  double* les_len = nullptr;   // the eddy viscosity's length per plane (model 2)
+  double* les_len = nullptr;   // the eddy viscosity's length per plane
   unsigned long long* les_nfall = nullptr;
   unsigned long long les_points = 0;
 };
@@ -568,6 +568,10 @@ struct Impl {
     const bool f32 = sizeof(T) == 4;
     P1Launch a = p1_args(c, rk, lin, 0);
     if (phase == 1) {
+      if (c->les_on && !lin && c->split_x) {
+        const int r = les_lengths(c);
+        if (r) return r;
+      }
       c->mean_src = c->mvel64;
       if (a.split && !c->mean64_valid) {
         prof_begin(c, "k_mean_base");
@@ -645,20 +649,30 @@ struct Impl {
     return CFG_OK;
   }
 
+  // the planes' eddy-viscosity lengths, from the mean shear of the last solve,
+  // on the side stream beside the inverse transforms
+  static int les_lengths(cfg_ctx* c) {
+    CK(cudaEventRecord(c->ev_fork, c->st));
+    CK(cudaStreamWaitEvent(c->st2, c->ev_fork, 0));
+    k_les_lengths<<<1, 128, 0, c->st2>>>(c->les_len, c->gd, c->les, c->d_um_dy, c->g.ny);
+    c->launches++;
+    CK(cudaGetLastError());
+    CK(cudaEventRecord(c->ev_len, c->st2));
+    return CFG_OK;
+  }
+
   // the LES mode's subgrid stresses from the physical planes P (after
-  // k_xinv_r): eddy viscosity, and for model 2 the network and the checks
+  // k_xinv_r) and the lengths (les_lengths): eddy viscosity, and for model 2 the network and the checks
   static int les_stresses(cfg_ctx* c, float* F) {
     const Geom& g = c->g;
-    dim3 gr((g.nx2 + 127) / 128, g.nz2, g.ny - 1);
+    dim3 gr((g.nz2 * g.nx2 + 255) / 256, g.ny - 1);
+    CK(cudaStreamWaitEvent(c->st, c->ev_len, 0));
     prof_begin(c, "k_les_sgs");
-    k_les_sgs<T><<<gr, 128, 0, c->st>>>((const T*)c->P, (T*)c->les_S, F, g, c->gd, c->les, c->d_um_dy);
+    k_les_sgs<T><<<gr, 256, 0, c->st>>>((const T*)c->P, (T*)c->les_S, F, g, c->gd, c->les, c->les_len);
     CKL();
     if (c->les.model == 2 && F == c->les_F) {
-      // the planes' eddy-viscosity lengths, then the network with the checks
-      // and the blend in its output layer's epilogue (the outputs never go
-      // to memory)
-      k_les_lengths<<<1, 128, 0, c->st>>>(c->les_len, c->gd, c->les, c->d_um_dy, g.ny);
-      CKL();
+      // the network with the checks and the blend in its output layer's
+      // epilogue (the outputs never go to memory)
       prof_begin(c, "k_mlp_fwd");
       const LesBlend<T> b{(T*)c->les_S, c->les_F, c->les_len, c->gd, c->les, g.nx2, g.nz2, c->les_nfall};
       if (mlp_forward_blend<T>(c->les_mlp, (long long)c->les_points, b, c->st) != CFG_OK)
@@ -674,6 +688,8 @@ struct Impl {
   static int les_features(cfg_ctx* c, float* F) {
     const Geom& g = c->g;
     const bool f32 = sizeof(T) == 4;
+    const int rl = les_lengths(c);
+    if (rl) return rl;
     P1Launch a{};
     a.vel = c->vel; a.T1 = c->T1; a.g = g; a.twx = c->twx; a.twz = c->twz; a.gd = c->gd; a.YB1 = c->fYB1;
     a.st = c->st; a.P = c->P; a.FZR = c->flux_zr; a.sc = c->scat;
@@ -1081,6 +1097,7 @@ static int create_impl(const cfg_params* p, const cfg_grid* gr, const SlabPart* 
       cudaStreamCreateWithFlags(&c->st3, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->ev_join3, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->ev_jet, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&c->ev_len, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess) {
     delete c;
@@ -1264,6 +1281,7 @@ void cfg_destroy(cfg_ctx* c) {
   if (c->ev_join) cudaEventDestroy(c->ev_join);
   if (c->ev_join3) cudaEventDestroy(c->ev_join3);
   if (c->ev_jet) cudaEventDestroy(c->ev_jet);
+  if (c->ev_len) cudaEventDestroy(c->ev_len);
   if (c->st2) cudaStreamDestroy(c->st2);
   if (c->st3) cudaStreamDestroy(c->st3);
   if (c->st) cudaStreamDestroy(c->st);
@@ -1649,13 +1667,13 @@ int cfg_set_les(cfg_ctx* c, const cfg_les* l) {
   const size_t tsz = c->mixed ? sizeof(float) : sizeof(double);
   c->les_points = (unsigned long long)(g.ny - 1) * cs;
   if (!c->les_S) {
-    if (cudaMalloc(&c->les_S, tsz * 6 * cs * g.ny1) != cudaSuccess || cudaMalloc(&c->les_nfall, 8) != cudaSuccess)
+    if (cudaMalloc(&c->les_S, tsz * 6 * cs * g.ny1) != cudaSuccess || cudaMalloc(&c->les_nfall, 8) != cudaSuccess ||
+        cudaMalloc(&c->les_len, sizeof(double) * (g.ny + 1)) != cudaSuccess)
       return fail(c, CFG_E_NOMEM, "LES stresses");
     CK(cudaMemsetAsync(c->les_S, 0, tsz * 6 * cs * g.ny1, c->st));   // wall planes stay zero
   }
   if (l->model == 2 && !c->les_F) {
-    if (cudaMalloc(&c->les_F, sizeof(float) * 10 * c->les_points) != cudaSuccess ||
-        cudaMalloc(&c->les_len, sizeof(double) * (g.ny + 1)) != cudaSuccess)
+    if (cudaMalloc(&c->les_F, sizeof(float) * 10 * c->les_points) != cudaSuccess)
       return fail(c, CFG_E_NOMEM, "LES closure buffers");
   }
   CK(cudaMemsetAsync(c->les_nfall, 0, 8, c->st));

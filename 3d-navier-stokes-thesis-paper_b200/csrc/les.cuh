@@ -62,8 +62,7 @@ __device__ __forceinline__ void les_gradient(const T* __restrict__ P, const Geom
   G[8] = (at(P0, 2, zp, x) - at(P0, 2, zm, x)) * ihz;
 }
 
-// the eddy viscosity's length of plane k, Cs Delta (1 - exp(-y+/A+)): one
-// value per plane, computed once per block (the caller's threads share k)
+// the eddy viscosity's length of plane k, Cs Delta (1 - exp(-y+/A+))
 __device__ __forceinline__ double les_nut_length(const GridDev& gd, const LesDev& les,
                                                  const double* __restrict__ d_um_dy, int ny, int k) {
   const double dy = gd.y[k - 1] - gd.y[k - 2];
@@ -71,15 +70,6 @@ __device__ __forceinline__ double les_nut_length(const GridDev& gd, const LesDev
   const double utau = sqrt(0.5 * (fabs(d_um_dy[0]) + fabs(d_um_dy[ny - 1])) / les.re);
   const double yplus = (1.0 - fabs(gd.yh[k - 1])) * utau * les.re;
   return les.cs * delta * (1.0 - exp(-yplus / les.aplus));
-}
-
-// the length above shared by a block: thread 0 computes it
-__device__ __forceinline__ double les_block_length(const GridDev& gd, const LesDev& les,
-                                                   const double* __restrict__ d_um_dy, int ny, int k) {
-  __shared__ double len;
-  if (threadIdx.x == 0) len = les_nut_length(gd, les, d_um_dy, ny, k);
-  __syncthreads();
-  return len;
 }
 
 // trace-free strain rate (11, 22, 33, 12, 13, 23) and the eddy viscosity
@@ -98,28 +88,43 @@ __device__ __forceinline__ double les_strain_nut(const double G[9], double f, do
 }
 
 // model 1 stresses into S and, for model 2, the network's input features
-// F[(k - 2) * nz2 * nx2 + z * nx2 + x][10] (normalised, FP32).  Grid
-// (nx2/128 rounded up, nz2, ny - 1), block 128.
+// F[(k - 2) * nz2 * nx2 + z * nx2 + x][10] (normalised, FP32); len: the
+// planes' lengths (k_les_lengths).  Grid (nz2 nx2 / 256 rounded up, ny - 1),
+// block 256, a point per thread along the plane: rows of 192 points leave no
+// thread idle, and a cube root, a square root and an exponential per plane
+// are no longer computed by one thread of every block while the others wait.
+// The features leave through shared memory in whole lines (ten of a thread
+// lie 40 bytes from its neighbour's).  What is left is the FP64 arithmetic,
+// half of it conversions.  us per launch, before / now, 128x65x128: 57 / 47
+// without the features, 73 / 63 with them.
 template <typename T>
-__global__ void __launch_bounds__(128) k_les_sgs(const T* __restrict__ P, T* __restrict__ S, float* __restrict__ F,
-                                                 Geom g, GridDev gd, LesDev les, const double* __restrict__ d_um_dy) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x, z = blockIdx.y, k = 2 + blockIdx.z;
-  const double len = les_block_length(gd, les, d_um_dy, g.ny, k);
-  if (x >= g.nx2) return;
-  double G[9], Sd[6];
-  les_gradient<T>(P, g, gd, les, k, z, x, G);
-  const double nut = les_strain_nut(G, len, Sd);
-  const size_t cs = (size_t)g.nz2 * g.nx2, o = (size_t)(k - 1) * 6 * cs + (size_t)z * g.nx2 + x;
+__global__ void __launch_bounds__(256) k_les_sgs(const T* __restrict__ P, T* __restrict__ S, float* __restrict__ F,
+                                                 Geom g, GridDev gd, LesDev les, const double* __restrict__ len) {
+  __shared__ __align__(16) float sf[256 * 10];
+  const int plane = g.nz2 * g.nx2, base = blockIdx.x * 256, idx = base + (int)threadIdx.x, k = 2 + blockIdx.y;
+  if (idx < plane) {
+    const int z = idx / g.nx2, x = idx - z * g.nx2;
+    double G[9], Sd[6];
+    les_gradient<T>(P, g, gd, les, k, z, x, G);
+    const double nut = les_strain_nut(G, len[k], Sd);
+    const size_t cs = (size_t)plane, o = (size_t)(k - 1) * 6 * cs + idx;
 #pragma unroll
-  for (int c = 0; c < 6; ++c) S[o + c * cs] = (T)(-2.0 * nut * Sd[c]);
+    for (int c = 0; c < 6; ++c) S[o + c * cs] = (T)(-2.0 * nut * Sd[c]);
+    if (les.model == 2) {
+      // mirrored into the lower half: components with one y index flip
+      const double sgn = gd.yh[k - 1] > 0.0 ? -1.0 : 1.0;
+      const double f[10] = {G[0], sgn * G[1], G[2], sgn * G[3], G[4], sgn * G[5], G[6], sgn * G[7], G[8],
+                            1.0 - fabs(gd.yh[k - 1])};
+#pragma unroll
+      for (int i = 0; i < 10; ++i) sf[threadIdx.x * 10 + i] = (float)((f[i] - les.in_shift[i]) * les.in_iscale[i]);
+    }
+  }
   if (les.model == 2) {
-    // mirrored into the lower half: components with one y index flip
-    const double sgn = gd.yh[k - 1] > 0.0 ? -1.0 : 1.0;
-    const double f[10] = {G[0], sgn * G[1], G[2], sgn * G[3], G[4], sgn * G[5], G[6], sgn * G[7], G[8],
-                          1.0 - fabs(gd.yh[k - 1])};
-    float* out = F + (((size_t)(k - 2) * g.nz2 + z) * g.nx2 + x) * 10;
-#pragma unroll
-    for (int i = 0; i < 10; ++i) out[i] = (float)((f[i] - les.in_shift[i]) * les.in_iscale[i]);
+    __syncthreads();
+    // (plane is even, so the block's part of F starts on 8 bytes)
+    const int n2 = min(256, plane - base) * 5;
+    float2* const out = reinterpret_cast<float2*>(F + ((size_t)(k - 2) * plane + base) * 10);
+    for (int i = threadIdx.x; i < n2; i += 256) out[i] = reinterpret_cast<const float2*>(sf)[i];
   }
 }
 
