@@ -456,7 +456,7 @@ struct Impl {
     // 128x200x64 and 128x129x128: 12.7 / 11.6, 38.9 / 34.0, 61.6 / 59.5, 78.1 /
     // 74.6 us), 4 beyond (192x129x192, 256x193x256: 164 / 196, 405 / 450); 2 in
     // FP64
-    c->flux_zr = f32 ? (g.nx2 <= 192 && gp.nz2 % 8 == 0 ? 8 : 4) : 2;
+    c->flux_zr = f32 ? (g.nx2 <= 192 && (gp.nz2 % 8 == 0 || !regfft_full(g.nx2)) ? 8 : 4) : 2;
     c->flux_given = getenv("CHANFLOW_FLUX_ZR") != nullptr;
     if (c->flux_given) {
       c->flux_zr = atoi(getenv("CHANFLOW_FLUX_ZR"));
@@ -523,15 +523,17 @@ struct Impl {
     return CFG_OK;
   }
 
-  // z rows per flux block: the tile where it divides the z2 rows and the
-  // products have that block (8 rows: not the linearized and the LES ones;
-  // asked for, the lengths of regfft_full leave that to the launch), else 4
-  // or 2
+  // z rows per flux block: the tile where the products have that block (8
+  // rows: not the linearized and the LES ones; asked for, the lengths of
+  // regfft_full leave that to the launch), else 4; lengths of regfft_full also
+  // want it to divide the z2 rows
   static int flux_rows(const cfg_ctx* c, bool plain_products) {
     const int zr = c->flux_zr, nz2 = c->gP.nz2;
-    if (nz2 % zr == 0 && (zr < 8 || plain_products || (c->flux_given && regfft_full(c->g.nx2)))) return zr;
-    return nz2 % 4 == 0 ? 4 : 2;
+    const bool full = regfft_full(c->g.nx2);
+    if ((nz2 % zr == 0 || !full) && (zr < 8 || plain_products || (c->flux_given && full))) return zr;
+    return nz2 % 4 == 0 || !full ? 4 : 2;
   }
+
   // the launch record of register-FFT pass-1 kernel `which` (0 k_zinv_r, 1
   // k_xflux_r, 2 k_zfwd_r, 3 k_xinv_r, 4 k_flux_r) in substep rk
   static P1Launch p1_args(const cfg_ctx* c, int rk, bool lin, int which) {

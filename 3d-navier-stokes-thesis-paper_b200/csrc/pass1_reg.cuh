@@ -748,7 +748,8 @@ k_xinv_r(const cplx_t<T>* __restrict__ T1, T* __restrict__ P, Geom g, const cplx
   k_xinv_r_body<T, NX2, ZB, DEAL>(blockIdx, T1, P, g, twx);
 }
 
-// k_flux_r: grid (nz2/ZR, ny-1), block NT.  Fluxes of plane k = 2 + blockIdx.y
+// k_flux_r: grid (ceil(nz2/ZR), ny-1), block NT (the last block of an nz2 that
+// ZR does not divide takes the rows that are left).  Fluxes of plane k = 2 + blockIdx.y
 // on ZR rows of z from the physical planes k-1, k, k+1, then the forward x
 // transform and the Hermitian unpacking into T2 -- the same arithmetic and
 // output as k_xflux_r (PFC/pass1.f90:134-226, PFC/transform.f90:287-315).
@@ -803,6 +804,7 @@ __device__ __forceinline__ void k_flux_r_body(const uint3 bid, const T* __restri
   const int NXH = g.nxh, NZ2 = g.nz2, ny = g.ny;
   const bool deal = 3 * (NXH - 1) == N;
   const int z0 = bid.x * ZR;
+  const int nr = min(ZR, NZ2 - z0);
   const int k = 2 + bid.y;
   pdl_trigger();
   load_tw2<T, N, N1, N2>(tw, twx);
@@ -965,6 +967,7 @@ __device__ __forceinline__ void k_flux_r_body(const uint3 bid, const T* __restri
     const int idx = it * NT + (int)threadIdx.x;
     if ((ZR * N / 2) % NT != 0 && idx >= ZR * N / 2) break;
     const int x = 2 * (idx % (N / 2)), r = idx / (N / 2);
+    if (r >= nr) break;
     const size_t o = (size_t)r * N + x;
     auto ld2 = [&](const T* b) { return __ldg(reinterpret_cast<const V2*>(b + o)); };
     const V2 U = ld2(P0), V = ld2(P0 + cs), W = ld2(P0 + 2 * cs);
@@ -1046,6 +1049,7 @@ __device__ __forceinline__ void k_flux_r_body(const uint3 bid, const T* __restri
   const size_t base = (size_t)(k - 1) * 6;
   for (int idx = threadIdx.x; idx < NXH * ZR; idx += NT) {
     const int r = idx % ZR, kx = idx / ZR;
+    if (r >= nr) continue;
     const T kxv = skx[kx];
     const int km = (kx == 0) ? 0 : N - kx;
     // one rank: local layout; several: column kx goes to the rank that owns it
