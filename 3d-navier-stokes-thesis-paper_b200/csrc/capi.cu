@@ -1480,7 +1480,9 @@ static int timestep_impl(cfg_ctx* c, int nsteps, bool lin) {
   if (!c || nsteps < 0) return CFG_E_ARG;
   if (c->nranks > 1) return single_only(c, "cfg_timestep");
   cudaSetDevice(c->dev);
-  c->chained = true;
+  // dependent launches, but not into a graph that the caller is capturing
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  c->chained = cudaStreamIsCapturing(c->st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
   int r = CFG_OK;
   for (int s = 0; s < nsteps && !r; ++s) r = step_enqueue(c, lin);
   c->chained = false;

@@ -13,6 +13,7 @@
 #include "chanflow.h"
 #include "mlp.cuh"
 #include "mlp_les.h"
+#include "cfd_common.cuh"
 
 using namespace cfd::mlp;
 
@@ -241,6 +242,9 @@ __global__ void __launch_bounds__(NTH, 1) k_mlp_train(const uint4* __restrict__ 
   const int warp = (tid >> 5) & 3, lane = tid & 31;   // warp: of the tile's four groups of 32 points
   const int r = blockIdx.x * TILE + p;
   const bool valid = r < batch;
+  // (everything the kernel reads may come from the kernel before it)
+  cfd::pdl_trigger();
+  cfd::pdl_wait();
   const long long row = valid ? (long long)idx[r] : 0;
   for (int i = tid; i < IMG_UNITS; i += NTH) sm[Smem::W + i] = img[i];
   for (int i = tid; i < NBIAS; i += NTH) sb[i] = bias[i];
@@ -373,10 +377,12 @@ __global__ void __launch_bounds__(NTH, 1) k_mlp_train(const uint4* __restrict__ 
 __global__ void __launch_bounds__(64) k_mlp_reduce(const float* __restrict__ part, int ntiles, float* __restrict__ G,
                              float* __restrict__ loss) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  cfd::pdl_trigger();
+  cfd::pdl_wait();
   if (i > NPARAM) return;
   float s = 0.f;
 #pragma unroll 16
-  for (int b = 0; b < ntiles; ++b) s += __ldg(part + (size_t)b * PART_STRIDE + i);
+  for (int b = 0; b < ntiles; ++b) s += __ldcg(part + (size_t)b * PART_STRIDE + i);
   if (i < NPARAM) G[i] += s;
   else *loss += s;
 }
@@ -552,8 +558,14 @@ int cfg_mlp_accumulate_grad(cfg_mlp* m, const float* x, const float* t, const in
     if (cudaMalloc(&m->part, (size_t)ntiles * PART_STRIDE * sizeof(float)) != cudaSuccess) return CFG_E_NOMEM;
     m->part_tiles = ntiles;
   }
-  k_mlp_train<<<ntiles, NTH, SMEM_TRAIN, (cudaStream_t)stream>>>(m->img, m->bias, x, t, idx, batch, m->part, m->err);
-  k_mlp_reduce<<<(NPARAM + 1 + 63) / 64, 64, 0, (cudaStream_t)stream>>>(m->part, ntiles, m->G, m->loss);
+  // dependent launches, but not into a graph that the caller is capturing
+  const cudaStream_t st = (cudaStream_t)stream;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  const bool pdl = cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+  cfd::launch_chained(pdl, k_mlp_train, dim3(ntiles), dim3(NTH), SMEM_TRAIN, st, (const uint4*)m->img,
+                      (const float*)m->bias, x, t, idx, batch, m->part, m->err);
+  cfd::launch_chained(pdl, k_mlp_reduce, dim3((NPARAM + 1 + 63) / 64), dim3(64), 0, st, (const float*)m->part, ntiles,
+                      m->G, m->loss);
   return cudaGetLastError() == cudaSuccess ? CFG_OK : CFG_E_CUDA;
 }
 
