@@ -431,9 +431,9 @@ struct Impl {
     c->fast_z = regfft_supported(g.nz2);
     c->fast_x = regfft_supported(g.nx2);
     // planes per z-transform block: 8 in the inverse transform (short of it the
-    // data1 runs are too short: 256x193x256 mixed 349, 100, 86 and 84 us for 1,
+    // data1 runs are too short: 256x193x256 mixed 349, 99, 85 and 80 us for 1,
     // 2, 4 and 8; FP64 206, 184, 165 and 178: 4 from 288 points on); 4 in the
-    // forward transform (248, 188, 166 and 176 us; FP64 424, 306, 313 and 364)
+    // forward transform (248, 189, 160 and 177 us; FP64 424, 306, 313 and 364)
     c->fYB1 = f32 || g.nz2 < 288 ? 8 : 4;
     c->fYB3 = 4;
     if (c->fast_x) {

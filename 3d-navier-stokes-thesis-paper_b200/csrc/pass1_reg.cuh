@@ -47,11 +47,10 @@ __device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_g
 // known at compile time, one thread takes one stage-1 and one stage-2 task,
 // and the 3/2-dealiased row count (DEAL: nz = 2 nz2/3) too: which of a
 // thread's N1 inputs are zero or mirrored is then a constant of n1 but for
-// the two at the edges.  us per launch before / now, mixed: k_zinv_r 121 / 84
-// and k_zfwd_r 234 / 166 at 256x193x256, 505 / 190 and 905 / 399 at
+// the two at the edges.  us per launch before / now, mixed: k_zinv_r 121 / 80
+// and k_zfwd_r 234 / 160 at 256x193x256, 505 / 190 and 905 / 399 at
 // 384x193x384; FP64 280 / 165 and 405 / 313 at 256x193x256.  What is left is
-// latency: both move two thirds of the copy bandwidth at best (k_zinv_r 4.6,
-// k_zfwd_r 3.7 TB/s at 256x193x256 mixed).
+// latency: k_zinv_r moves 4.8 and k_zfwd_r 3.8 TB/s at 256x193x256 mixed.
 template <typename T, int N, int YP> struct ZShape {
   static constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2;
   static constexpr int PITCH = N2 | 1;   // odd: rows of the exchange buffer on different banks
@@ -66,10 +65,12 @@ template <typename T, int N, int YP> struct ZShape {
   static constexpr int up32(int n) { return (n + 31) / 32 * 32; }
   static constexpr int INV_NT = up32(YP * (N1 > N2 ? N1 : N2));
   static constexpr int FWD_NT = up32(2 * YP * (N1 > N2 ? N1 : N2));
-  // blocks per SM to compile for: the registers that keep the FFT's values
-  // (the longer of N1, N2) without spilling
+  // blocks per SM to compile for: registers that keep the FFT's values with
+  // few spills (FP32, 64 / 80 registers: k_zinv_r 80 / 84 and k_zfwd_r 160 / 166
+  // us at 384 points, 193 / 190 and 413 / 398 at 576, the one length with two
+  // 24-point stages)
   static constexpr int LONG = N1 > N2 ? N1 : N2;
-  static constexpr int regs(bool f32) { return f32 ? (LONG > 18 ? 80 : LONG > 12 ? 64 : 56) : (LONG > 18 ? 168 : LONG > 12 ? 128 : 104); }
+  static constexpr int regs(bool f32) { return f32 ? (N1 + N2 > 42 ? 80 : LONG > 12 ? 64 : 56) : (LONG > 18 ? 168 : LONG > 12 ? 128 : 104); }
   static constexpr int blocks(int nt, bool f32) { return 65536 / (nt * regs(f32)) > 0 ? (65536 / (nt * regs(f32)) > 32 ? 32 : 65536 / (nt * regs(f32))) : 1; }
 };
 
