@@ -245,6 +245,7 @@ struct cfg_ctx {
   double2* mean_base = nullptr;
   const double2* mean_src = nullptr;   // of the current substep
   bool cfl_clean = false;   // the CFL maxima are zero (k_cfl_finalize resets them on one rank)
+  bool cfl_after = false;   // whether they are once this step's nonlinear term is enqueued
   bool les_on = false;
   LesDev les{};
   cfg_mlp* les_mlp = nullptr;
@@ -582,8 +583,16 @@ struct Impl {
         c->mean_src = c->mean_base;
       }
       c->mean64_valid = false;
-      if (do_cfl && !c->cfl_clean) CK(cudaMemsetAsync(c->cflbits, 0, sizeof(unsigned long long) * 3 * g.ny1, c->st));
-      if (do_cfl) c->cfl_clean = false;
+      if (do_cfl) {
+        c->cfl_after = c->cfl_clean;
+        if (!c->cfl_clean) {
+          CK(cudaMemsetAsync(c->cflbits, 0, sizeof(unsigned long long) * 3 * g.ny1, c->st));
+          // (captured, it has not run yet: the next eager step zeroes them too)
+          cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+          c->cfl_after = cudaStreamIsCapturing(c->st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+        }
+        c->cfl_clean = false;
+      }
       dim3 g1(g.nxh, (g.ny1 + c->YB1 - 1) / c->YB1);
       prof_begin(c, "k_zinv");
       if (c->fast_z) {
@@ -646,7 +655,7 @@ struct Impl {
       launch_chained(c->chained, lin ? k_cfl_finalize<true> : k_cfl_finalize<false>, dim3(1), dim3(256), 0, c->st,
                      c->cflbits, reset, g, c->gd, c->sc, c->cflp, c->p.lx, c->p.lz, c->p.dt_flag, c->p.cfl_max, step);
       CKL();
-      c->cfl_clean = reset;
+      c->cfl_clean = reset && c->cfl_after;
     }
     return CFG_OK;
   }
@@ -950,12 +959,20 @@ struct Impl {
 
   // the wall jet of substep rk of a time step on the side stream, beside the
   // nonlinear term, where dt is already final: five small kernels in a chain
-  // (25 us of a 290 us substep at 128x129x128) that only the solve needs
-  static int jet_beside(cfg_ctx* c, int rk) {
+  // (25 us of a 290 us substep at 128x129x128) that only the solve needs.
+  // The side stream forks before the nonlinear term (jet_fork); the jet is
+  // enqueued after it, so that a step whose launch is refused leaves the
+  // jet's random walk where it was.
+  static int jet_fork(cfg_ctx* c, int rk) {
     c->jet_rk = 0;
     if (!c->crossflow || (rk == 1 && c->p.dt_flag == 1)) return CFG_OK;
     CK(cudaEventRecord(c->ev_fork, c->st));
     CK(cudaStreamWaitEvent(c->st2, c->ev_fork, 0));
+    return CFG_OK;
+  }
+
+  static int jet_beside(cfg_ctx* c, int rk) {
+    if (!c->crossflow || (rk == 1 && c->p.dt_flag == 1)) return CFG_OK;
     const cudaStream_t main = c->st;
     c->st = c->st2;
     const int r = jet(c, rk, 0.0, 0.0, 1);
@@ -1466,9 +1483,11 @@ static int step_enqueue(cfg_ctx* c, bool lin) {
     if (r) return r;
   }
   for (int rk = 1; rk <= 3; ++rk) {
-    r = DISPATCH(c, jet_beside(c, rk));
+    r = DISPATCH(c, jet_fork(c, rk));
     if (r) return r;
     r = DISPATCH(c, nonlinear(c, c->step, rk, lin));
+    if (r) return r;
+    r = DISPATCH(c, jet_beside(c, rk));
     if (r) return r;
     r = DISPATCH(c, rhs(c, rk, 0, rk == 3));
     if (r) return r;

@@ -221,7 +221,8 @@ __global__ void __launch_bounds__(TILE) k_mlp_fwd(const uint4* __restrict__ img,
 // epilogue eight times over with one warp per scheduler, so half the epilogue
 // per thread shortens it; with the bias sums of 32 columns in 31 shuffles,
 // 16-byte gradient stores and the reduction's loads in flight, a batch of
-// 65536 rows takes 0.087 ms (0.151 before) and 16 of 4096 0.48 ms (0.72).
+// 65536 rows takes 0.087 ms (0.151 before) and 16 of 4096 0.48 ms (0.72), 0.40
+// with the dependent launches of the gradient and its slice sum.
 // Forward with the pre-activations
 // kept in TMEM, mean-square loss against t over the 6 outputs, backward, and
 // the tile's weight and bias gradients (FP32, flat parameter layout) and its
