@@ -805,7 +805,12 @@ __device__ __forceinline__ void k_flux_r_body(const uint3 bid, const T* __restri
   const int NXH = g.nxh, NZ2 = g.nz2, ny = g.ny;
   const bool deal = 3 * (NXH - 1) == N;
   const int z0 = bid.x * ZR;
-  const int nr = min(ZR, NZ2 - z0);
+  // (a test of the row in the point loop keeps its loads from being hoisted:
+  // without it 397 -> 386 us at 256x193x256, 79.7 -> 71.8 at 128x129x128, FP64
+  // 821 -> 786; with the stresses to add as well it is faster with the test,
+  // 47.2 / 49.7 at 128x65x128)
+  constexpr bool TAIL = !regfft_full(N) || SGS;
+  const int nr = TAIL ? min(ZR, NZ2 - z0) : ZR;
   const int k = 2 + bid.y;
   pdl_trigger();
   load_tw2<T, N, N1, N2>(tw, twx);
@@ -968,7 +973,7 @@ __device__ __forceinline__ void k_flux_r_body(const uint3 bid, const T* __restri
     const int idx = it * NT + (int)threadIdx.x;
     if ((ZR * N / 2) % NT != 0 && idx >= ZR * N / 2) break;
     const int x = 2 * (idx % (N / 2)), r = idx / (N / 2);
-    if (r >= nr) break;
+    if (TAIL && r >= nr) break;
     const size_t o = (size_t)r * N + x;
     auto ld2 = [&](const T* b) { return __ldg(reinterpret_cast<const V2*>(b + o)); };
     const V2 U = ld2(P0), V = ld2(P0 + cs), W = ld2(P0 + 2 * cs);
@@ -1050,7 +1055,7 @@ __device__ __forceinline__ void k_flux_r_body(const uint3 bid, const T* __restri
   const size_t base = (size_t)(k - 1) * 6;
   for (int idx = threadIdx.x; idx < NXH * ZR; idx += NT) {
     const int r = idx % ZR, kx = idx / ZR;
-    if (r >= nr) continue;
+    if (TAIL && r >= nr) continue;
     const T kxv = skx[kx];
     const int km = (kx == 0) ? 0 : N - kx;
     // one rank: local layout; several: column kx goes to the rank that owns it
