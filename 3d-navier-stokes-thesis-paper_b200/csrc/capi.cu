@@ -93,6 +93,28 @@ template <typename T>
 __global__ void k_real_out(const T* __restrict__ src, double* __restrict__ dst, size_t n) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) dst[i] = (double)src[i];
 }
+
+// the |k| < 4 list's columns in FP64 (n wavenumbers x nc x n1): from the FP32
+// state, and from and to an FP64 array whose element (kx, kz, c, j) lies at
+// kx s.kx + kz s.kz + c s.c + j s.j
+__global__ void k_low_widen(const int* __restrict__ list, const float2* __restrict__ src, double2* __restrict__ side,
+                            int nc_n1, size_t n) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const float2 v = src[(size_t)list[i / nc_n1] * nc_n1 + i % nc_n1];
+    side[i] = make_double2((double)v.x, (double)v.y);
+  }
+}
+struct LowStride { size_t kx, kz, c, j; };
+template <bool IN>
+__global__ void k_low_copy(const int* __restrict__ list, double2* __restrict__ side, double2* __restrict__ arr, int nc,
+                           int n1, int nz, LowStride s, size_t n) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const int w = list[i / ((size_t)nc * n1)], r = (int)(i % ((size_t)nc * n1));
+    double2* const e = arr + (w / nz) * s.kx + (w % nz) * s.kz + (r / n1) * s.c + (r % n1) * s.j;
+    if (IN) side[i] = *e;
+    else *e = side[i];
+  }
+}
 __global__ void k_advance_time(DevScalars* sc) { sc->t_total = sc->t_total + sc->dt; }
 
 // max |divergence| (check_divergence, PFC/pass2.f90:380-419), warp per wavenumber
@@ -159,6 +181,14 @@ struct cfg_ctx {
   // state
   void *vel = nullptr, *cru = nullptr, *prs = nullptr;
   double2 *mvel64 = nullptr, *mcru64 = nullptr;
+  // mixed precision: FP64 columns of the |k| < 4 list, in its order (n_prec x
+  // 3 x (ny+1) velocity and accumulator, n_prec x (ny+1) pressure), beside
+  // their FP32 rounding in vel, cru and prs.  A rounding of the stored columns
+  // reaches the pressure divided by k^2 dt: with FP32 alone these few
+  // wavenumbers set the error of the whole pressure.  low_ok: they hold the
+  // current state (not after a solve that reads the FP32 columns).
+  double2 *lvel64 = nullptr, *lcru64 = nullptr, *lprs64 = nullptr;
+  bool low_ok = true;
   void *T1 = nullptr, *T2 = nullptr;
   // physical planes of the split x stage (k_xinv_r -> k_flux_r)
   void* P = nullptr;
@@ -379,6 +409,40 @@ static cudaError_t allow_smem(K kernel) {
 __global__ void k_mean_base(const float2* __restrict__ v32, double2* __restrict__ base, int ny1) {
   for (int i = threadIdx.x; i < 3 * ny1; i += blockDim.x) base[i] = make_double2((double)v32[i].x, (double)v32[i].y);
 }
+
+// the FP64 columns of the |k| < 4 list from the FP32 state, on the context's
+// stream (captured, it has not run yet: the next eager solve does it too)
+static int low_widen(cfg_ctx* c) {
+  const size_t n = (size_t)c->n_prec * c->g.ny1;
+  if (n > 0) {
+    k_low_widen<<<grid1d(3 * n), 256, 0, c->st>>>(c->wl_prec, (const float2*)c->vel, c->lvel64, 3 * c->g.ny1, 3 * n);
+    CKL();
+    k_low_widen<<<grid1d(3 * n), 256, 0, c->st>>>(c->wl_prec, (const float2*)c->cru, c->lcru64, 3 * c->g.ny1, 3 * n);
+    CKL();
+    k_low_widen<<<grid1d(n), 256, 0, c->st>>>(c->wl_prec, (const float2*)c->prs, c->lprs64, c->g.ny1, n);
+    CKL();
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    c->low_ok = cudaStreamIsCapturing(c->st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+  }
+  return CFG_OK;
+}
+// the list's FP64 columns side (nc per wavenumber) from (IN) or to the FP64
+// array arr; the array's orders below
+template <bool IN>
+static int low_copy(cfg_ctx* c, double2* side, double2* arr, int nc, LowStride s) {
+  const size_t n = (size_t)c->n_prec * nc * c->g.ny1;
+  if (n == 0) return CFG_OK;
+  k_low_copy<IN><<<grid1d(n), 256, 0, c->st>>>(c->wl_prec, side, arr, nc, c->g.ny1, c->g.nz, s, n);
+  CKL();
+  return CFG_OK;
+}
+// data1 (nz, nxh, ny+1, 3); the device state [kx][kz][nc][ny+1]; a record of
+// the restart file per kx, (nz, ny+1, 3)
+static LowStride low_data1(const Geom& g) { return {(size_t)g.nz, 1, (size_t)g.nw * g.ny1, (size_t)g.nw}; }
+static LowStride low_state(const Geom& g, int nc) {
+  return {(size_t)g.nz * nc * g.ny1, (size_t)nc * g.ny1, (size_t)g.ny1, 1};
+}
+static LowStride low_record(const Geom& g) { return {(size_t)g.nz * g.ny1 * 3, 1, (size_t)g.nz * g.ny1, (size_t)g.nz}; }
 
 template <typename T>
 struct Impl {
@@ -717,8 +781,9 @@ struct Impl {
   // viscosity: a last-bit difference in the state flips points, and forty
   // steps later the states differ by 2e-5 (measured, against 3e-7 with the
   // eddy viscosity).  So that its runs repeat earlier ones bit for bit, a
-  // step with it keeps the summation order of its solves: the FP64 list and
-  // the mean mode by k_rhs2's partition method, a warp per wavenumber.
+  // step with it keeps the summation order of its solves and their FP32
+  // columns: the FP64 list and the mean mode by k_rhs2's partition method, a
+  // warp per wavenumber.
   static bool step_keeps_sums(const cfg_ctx* c) { return c->les_on && c->les.model == 2; }
 
   // launch records of k_rhs2: the fast list (storage precision) or, prec,
@@ -764,6 +829,7 @@ struct Impl {
     m.mean = g.kx0 == 0 ? 1 : 0;
     m.advance = c->advance ? 1 : 0;
     m.wlist = c->wl_prec; m.nlist = c->n_prec;
+    m.lvel64 = c->lvel64; m.lcru64 = c->lcru64; m.lprs64 = c->lprs64;
     m.wfast = c->wl_fast; m.nfast = c->rhs_rows ? c->n_fast : 0;
     m.st = c->rhs_rows ? c->st : c->st2;
     m.pdl = c->chained && c->rhs_rows ? 1 : 0;   // (the side stream's launch follows an event)
@@ -783,7 +849,12 @@ struct Impl {
       }
       c->jet_rk = 0;
     }
-    const bool keep = c->use_rhs2 && mode == 0 && step_keeps_sums(c);
+    const bool learned = mode == 0 && step_keeps_sums(c), keep = c->use_rhs2 && learned;
+    if (learned) c->low_ok = c->n_prec == 0;
+    else if (mode == 0 && !c->low_ok) {
+      const int r = low_widen(c);
+      if (r) return r;
+    }
     if (c->rhs_rows && mode == 0 && !keep) {
       prof_begin(c, "k_rhs");
       if (rhs_rows_launch(sizeof(T) == 4, rows_args(c, rk)) != 0) return fail(c, CFG_E_CUDA, "k_rhs_rows launch");
@@ -821,7 +892,10 @@ struct Impl {
         k_rhs<double, T, MM><<<c->n_prec, 32, c->sm_rhs64 / 4, c->st2>>>((C*)c->vel, (C*)c->cru, (C*)c->prs,
                                                                        (const C*)c->cbc + 3 * (size_t)g.nw,
                                                                        (const C*)c->cbc, g, c->gd, c->sc, c->rkt, rk,
-                                                                       c->p.re, mode, c->wl_prec, c->n_prec);
+                                                                       c->p.re, mode, c->wl_prec, c->n_prec,
+                                                                       mode || learned ? nullptr : c->lvel64,
+                                                                       mode || learned ? nullptr : c->lcru64,
+                                                                       mode || learned ? nullptr : c->lprs64);
         CKL();
       }
       if (g.kx0 == 0) {   // the mean mode lives on the rank that holds kx = 0
@@ -844,7 +918,8 @@ struct Impl {
       prof_begin(c, "k_rhs");
       k_rhs<T, T, MM><<<gr, 128, c->sm_rhs, c->st>>>((C*)c->vel, (C*)c->cru, (C*)c->prs,
                                                      (const C*)c->cbc + 3 * (size_t)g.nw, (const C*)c->cbc, g,
-                                                     c->gd, c->sc, c->rkt, rk, c->p.re, mode, c->wl_fast, c->n_fast);
+                                                     c->gd, c->sc, c->rkt, rk, c->p.re, mode, c->wl_fast, c->n_fast,
+                                                     nullptr, nullptr, nullptr);
       CKL();
     }
     // join
@@ -1233,6 +1308,15 @@ static int create_impl(const cfg_params* p, const cfg_grid* gr, const SlabPart* 
       return bad(CFG_E_NOMEM);
     if (!fast.empty()) cudaMemcpy(c->wl_fast, fast.data(), sizeof(int) * fast.size(), cudaMemcpyHostToDevice);
     if (!prec.empty()) cudaMemcpy(c->wl_prec, prec.data(), sizeof(int) * prec.size(), cudaMemcpyHostToDevice);
+    if (!prec.empty()) {
+      const size_t n = sizeof(double2) * prec.size() * n1;
+      if (cudaMalloc(&c->lvel64, 3 * n) != cudaSuccess || cudaMalloc(&c->lcru64, 3 * n) != cudaSuccess ||
+          cudaMalloc(&c->lprs64, n) != cudaSuccess)
+        return bad(CFG_E_NOMEM);
+      cudaMemset(c->lvel64, 0, 3 * n);
+      cudaMemset(c->lcru64, 0, 3 * n);
+      cudaMemset(c->lprs64, 0, n);
+    }
   }
   if (gr->buffer) {
     bool any = false;
@@ -1287,7 +1371,8 @@ void cfg_destroy(cfg_ctx* c) {
   if (c->ev_io_done) cudaEventDestroy(c->ev_io_done);
   if (c->st_io) cudaStreamDestroy(c->st_io);
   for (void* q : c->ipc_open) cudaIpcCloseMemHandle(q);
-  void* bufs[] = {c->dgrid, c->fringe, c->vel, c->cru, c->prs, c->mvel64, c->mcru64, c->T1, c->T2, c->P,
+  void* bufs[] = {c->dgrid, c->fringe, c->vel, c->cru, c->prs, c->mvel64, c->mcru64, c->lvel64, c->lcru64,
+                  c->lprs64, c->T1, c->T2, c->P,
                   c->rhs2_tbl, c->rhs2_tbl64, c->jst, c->pp_wy, c->pp_sy, c->pp_acc, c->cbc,
                   c->sc, c->d_um_dy, c->cflp, c->cflbits, c->l2acc, c->divbits, c->plist, c->pw_H,
                   c->pw_phys, c->pw_phys2, c->pw_in, c->stage, c->twx, c->twz, c->twxs, c->twzs,
@@ -1314,18 +1399,21 @@ int cfg_upload_state(cfg_ctx* c, const double* d1, const double* d2, const doubl
   const size_t nf = (size_t)g.nw * 3 * g.ny1;
   int r = ensure_stage(c, nf);
   if (r) return r;
+  if (!c->low_ok && (r = low_widen(c))) return r;
   if (d1) {
     CK(cudaMemcpyAsync(c->stage, d1, sizeof(double2) * nf, cudaMemcpyHostToDevice, c->st));
     c->mean64_valid = true;
     if (c->mixed) k_data1_in<float><<<grid1d(nf), 256, 0, c->st>>>(c->stage, (float2*)c->vel, mean_side(c, c->mvel64), g);
     else k_data1_in<double><<<grid1d(nf), 256, 0, c->st>>>(c->stage, (double2*)c->vel, nullptr, g);
     CKL();
+    if ((r = low_copy<true>(c, c->lvel64, c->stage, 3, low_data1(g)))) return r;
   }
   if (d2) {
     CK(cudaMemcpyAsync(c->stage, d2, sizeof(double2) * nf, cudaMemcpyHostToDevice, c->st));
     if (c->mixed) k_conv_in<float><<<grid1d(nf), 256, 0, c->st>>>(c->stage, (float2*)c->cru, nf, mean_side(c, c->mcru64), 3 * (size_t)g.ny1);
     else k_conv_in<double><<<grid1d(nf), 256, 0, c->st>>>(c->stage, (double2*)c->cru, nf, nullptr, 0);
     CKL();
+    if ((r = low_copy<true>(c, c->lcru64, c->stage, 3, low_state(g, 3)))) return r;
   }
   if (d4) {
     const size_t n = (size_t)g.nw * g.ny1;
@@ -1333,6 +1421,7 @@ int cfg_upload_state(cfg_ctx* c, const double* d1, const double* d2, const doubl
     if (c->mixed) k_conv_in<float><<<grid1d(n), 256, 0, c->st>>>(c->stage, (float2*)c->prs, n, nullptr, 0);
     else k_conv_in<double><<<grid1d(n), 256, 0, c->st>>>(c->stage, (double2*)c->prs, n, nullptr, 0);
     CKL();
+    if ((r = low_copy<true>(c, c->lprs64, c->stage, 1, low_state(g, 1)))) return r;
   }
   CK(cudaStreamSynchronize(c->st));
   return CFG_OK;
@@ -1349,6 +1438,7 @@ int cfg_download_state(cfg_ctx* c, double* d1, double* d2, double* d4) {
     if (c->mixed) k_data1_out<float><<<grid1d(nf), 256, 0, c->st>>>((const float2*)c->vel, c->mean64_valid ? mean_side(c, c->mvel64) : nullptr, c->stage, g);
     else k_data1_out<double><<<grid1d(nf), 256, 0, c->st>>>((const double2*)c->vel, nullptr, c->stage, g);
     CKL();
+    if (c->mean64_valid && c->low_ok && (r = low_copy<false>(c, c->lvel64, c->stage, 3, low_data1(g)))) return r;
     CK(cudaMemcpyAsync(d1, c->stage, sizeof(double2) * nf, cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
   }
@@ -1356,6 +1446,7 @@ int cfg_download_state(cfg_ctx* c, double* d1, double* d2, double* d4) {
     if (c->mixed) k_conv_out<float><<<grid1d(nf), 256, 0, c->st>>>((const float2*)c->cru, c->stage, nf, mean_side(c, c->mcru64), 3 * (size_t)g.ny1);
     else k_conv_out<double><<<grid1d(nf), 256, 0, c->st>>>((const double2*)c->cru, c->stage, nf, nullptr, 0);
     CKL();
+    if (c->low_ok && (r = low_copy<false>(c, c->lcru64, c->stage, 3, low_state(g, 3)))) return r;
     CK(cudaMemcpyAsync(d2, c->stage, sizeof(double2) * nf, cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
   }
@@ -1364,6 +1455,7 @@ int cfg_download_state(cfg_ctx* c, double* d1, double* d2, double* d4) {
     if (c->mixed) k_conv_out<float><<<grid1d(n), 256, 0, c->st>>>((const float2*)c->prs, c->stage, n, nullptr, 0);
     else k_conv_out<double><<<grid1d(n), 256, 0, c->st>>>((const double2*)c->prs, c->stage, n, nullptr, 0);
     CKL();
+    if (c->low_ok && (r = low_copy<false>(c, c->lprs64, c->stage, 1, low_state(g, 1)))) return r;
     CK(cudaMemcpyAsync(d4, c->stage, sizeof(double2) * n, cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
   }
@@ -1520,7 +1612,7 @@ int cfg_remove_initial_divergence(cfg_ctx* c) {
   if (r) return r;
   const size_t nf = (size_t)c->g.nw * 3 * c->g.ny1;
   CK(cudaMemcpyAsync(c->cru, c->vel, csize(c) * nf, cudaMemcpyDeviceToDevice, c->st));
-  return CFG_OK;
+  return low_widen(c);
 }
 
 int cfg_compute_initial_pressure(cfg_ctx* c, int linearized) {
@@ -1537,6 +1629,7 @@ int cfg_compute_initial_pressure(cfg_ctx* c, int linearized) {
   CK(cudaMemcpyAsync(c->vel, c->cru, csize(c) * nf, cudaMemcpyDeviceToDevice, c->st));
   if (c->mixed) CK(cudaMemcpyAsync(c->mvel64, c->mcru64, sizeof(double2) * 3 * c->g.ny1, cudaMemcpyDeviceToDevice, c->st));
   c->mean64_valid = true;
+  if ((r = low_widen(c))) return r;
   CK(cudaStreamSynchronize(c->st));
   return CFG_OK;
 }
@@ -1676,7 +1769,7 @@ int cfg_set_les(cfg_ctx* c, const cfg_les* l) {
   cudaSetDevice(c->dev);
   if (!l || l->model == 0) {
     c->les_on = false;
-    return CFG_OK;
+    return c->low_ok ? CFG_OK : low_widen(c);
   }
   if (l->model != 1 && l->model != 2) return fail(c, CFG_E_ARG, "cfg_set_les: model %d", l->model);
   if (!c->split_x || !c->full_len)
@@ -1720,6 +1813,10 @@ int cfg_set_les(cfg_ctx* c, const cfg_les* l) {
     d.out_scale[i] = l->out_scale[i];
   }
   c->les_mlp = l->mlp;
+  if (l->model == 1 && !c->low_ok) {
+    const int r = low_widen(c);
+    if (r) return r;
+  }
   CK(cudaStreamSynchronize(c->st));
   c->les_on = true;
   return CFG_OK;
@@ -2060,6 +2157,7 @@ int cfg_save_velocity(cfg_ctx* c, const char* path) {
   else
     k_restart_out<double><<<grid1d(nf), 256, 0, c->st>>>((const double2*)c->vel, nullptr, (double2*)c->io_dev, g);
   CKL();
+  if (c->mean64_valid && c->low_ok && (r = low_copy<false>(c, c->lvel64, (double2*)c->io_dev, 3, low_record(g)))) return r;
   const std::string p(path);
   const cfg_params prm = c->p;
   return start_io(c, bytes, [c, p, prm](std::string& why) {
@@ -2090,6 +2188,8 @@ int cfg_read_velocity(cfg_ctx* c, const char* path) {
   else
     k_restart_in<double><<<grid1d(nf), 256, 0, c->st>>>((const double2*)c->io_dev, (double2*)c->vel, nullptr, g);
   CKL();
+  if (!c->low_ok && (r = low_widen(c))) return r;
+  if ((r = low_copy<true>(c, c->lvel64, (double2*)c->io_dev, 3, low_record(g)))) return r;
   c->mean64_valid = true;
   // t_total from the file; dt too when dt_flag (PFC/read_write.f90:75-79)
   DevScalars h;
@@ -2726,6 +2826,12 @@ static int snap_take(cfg_ctx* c, TuneSnap& s) {
       {c->sc, sizeof(DevScalars)}, {c->d_um_dy, sizeof(double) * g.ny}};
   if (c->mvel64) live.push_back({c->mvel64, sizeof(double2) * 3 * g.ny1});
   if (c->mcru64) live.push_back({c->mcru64, sizeof(double2) * 3 * g.ny1});
+  if (c->n_prec > 0) {
+    const size_t n = sizeof(double2) * c->n_prec * g.ny1;
+    live.push_back({c->lvel64, 3 * n});
+    live.push_back({c->lcru64, 3 * n});
+    live.push_back({c->lprs64, n});
+  }
   if (c->jst) live.push_back({c->jst, sizeof(JetState)});
   for (auto& l : live) {
     void* d = nullptr;
@@ -2757,7 +2863,7 @@ int cfg_autotune(cfg_ctx* c, int trial_steps, int* choice) {
   if (r) { snap_free(snap); return r; }
   const int step0 = c->step;
   const long long launches0 = c->launches;
-  const bool mean_ok = c->mean64_valid;
+  const bool mean_ok = c->mean64_valid, low_ok = c->low_ok;
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
@@ -2766,6 +2872,8 @@ int cfg_autotune(cfg_ctx* c, int trial_steps, int* choice) {
   auto trial = [&]() -> float {
     if (snap_restore(c, snap)) return -1.f;
     c->step = step0;
+    c->mean64_valid = mean_ok;
+    c->low_ok = low_ok;
     if (step_enqueue(c, false)) { cudaGetLastError(); return -1.f; }
     cudaEventRecord(e0, c->st);
     for (int i = 0; i < trial_steps; ++i)
@@ -2788,6 +2896,8 @@ int cfg_autotune(cfg_ctx* c, int trial_steps, int* choice) {
     cudaEventDestroy(e1);
     c->step = step0;
     c->launches = launches0;
+    c->mean64_valid = mean_ok;
+    c->low_ok = low_ok;
     return fail(c, CFG_E_STATE, "cfg_autotune: the current settings do not run");
   }
   const bool f32 = c->mixed;
@@ -2829,6 +2939,7 @@ int cfg_autotune(cfg_ctx* c, int trial_steps, int* choice) {
   c->step = step0;
   c->launches = launches0;
   c->mean64_valid = mean_ok;
+  c->low_ok = low_ok;
   if (choice) {
     choice[0] = c->rhs2_warps;
     choice[1] = c->flux_zr;
@@ -3378,7 +3489,7 @@ int cfg_ensemble_create(int n, cfg_ctx* const* members, int autotune, cfg_ensemb
   e->batched = true;
   for (int i = 0; i < n; ++i) e->batched = e->batched && ens_batchable(members[i]);
   bool tune_batched = e->batched && autotune;
-  for (int i = 0; i < n; ++i) tune_batched = tune_batched && members[i]->mean64_valid;
+  for (int i = 0; i < n; ++i) tune_batched = tune_batched && members[i]->mean64_valid && members[i]->low_ok;
   if (tune_batched) {
     // one class per grid first (each grid's default tiles), tuned one class
     // at a time on the whole batched step
@@ -3413,11 +3524,11 @@ int cfg_ensemble_create(int n, cfg_ctx* const* members, int autotune, cfg_ensemb
 
 // one step of the ensemble (eagerly, or under stream capture): batched, or
 // every member on its own stream, forked from and joined to the ensemble
-// stream.  A batched step needs every member's FP64 mean copy current (it is
+// stream.  A batched step needs every member's FP64 copies current (they are
 // after any whole step).
 static int ensemble_enqueue(cfg_ensemble* e) {
   bool batched = e->batched;
-  for (const cfg_ctx* c : e->m) batched = batched && c->mean64_valid;
+  for (const cfg_ctx* c : e->m) batched = batched && c->mean64_valid && c->low_ok;
   e->last_batched = batched;
   if (batched) return ens_batched_enqueue(e);
   if (cudaEventRecord(e->ev_fork, e->st) != cudaSuccess) return CFG_E_CUDA;

@@ -268,7 +268,8 @@ __device__ __forceinline__ void sub_grad(cplx_t<T>* su, cplx_t<T>* sv, cplx_t<T>
 // (PFC/init_vel.f90:477-513): pressure from the velocity held in cru and the
 // nonlinear term in vel.
 // T is the arithmetic precision, S the storage precision of the state: the
-// mixed path runs its low-|k| wavenumbers with T = double over S = float.
+// mixed path runs its low-|k| wavenumbers with T = double over S = float, its
+// time steps (mode 0) from the list's FP64 columns vel64, cru64, prs64.
 template <typename T, typename S, int M>
 __global__ void __launch_bounds__(128) k_rhs(cplx_t<S>* __restrict__ vel,
                                              cplx_t<S>* __restrict__ cru,
@@ -277,7 +278,9 @@ __global__ void __launch_bounds__(128) k_rhs(cplx_t<S>* __restrict__ vel,
                                              const cplx_t<S>* __restrict__ cbc_bot, Geom g,
                                              GridDev gd, const DevScalars* __restrict__ sc,
                                              RkTab rkt, int rk, double re, int mode,
-                                             const int* __restrict__ wlist, int nlist) {
+                                             const int* __restrict__ wlist, int nlist,
+                                             double2* __restrict__ vel64, double2* __restrict__ cru64,
+                                             double2* __restrict__ prs64) {
   using C = cplx_t<T>;
   using CI = ColIdx<M>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -353,7 +356,10 @@ __global__ void __launch_bounds__(128) k_rhs(cplx_t<S>* __restrict__ vel,
     const T vis_exp = (T)(rkt.Cc(rk) * (dt / re));
     const T rk_press = (T)((rkt.Cc(rk) + rkt.D(rk)) * dt);
     C* scol[3] = {su, sv, sw};
-    for (int q = 0; q < 3; ++q) load_col<C, M>(scol[q], gcru + q * n1, n1, lane);
+    for (int q = 0; q < 3; ++q) {
+      if (cru64) load_col<C, M>(scol[q], cru64 + ((size_t)widx * 3 + q) * n1, n1, lane);
+      else load_col<C, M>(scol[q], gcru + q * n1, n1, lane);
+    }
     __syncwarp();
     for (int q = 0; q < 3; ++q) {
       const double* d2 = (q == 1) ? gd.d2n : gd.d2h;
@@ -378,7 +384,8 @@ __global__ void __launch_bounds__(128) k_rhs(cplx_t<S>* __restrict__ vel,
       for (int i = 0; i < M; ++i) scol[q][CI::at(lane * M + i)] = r[i];
       __syncwarp();
     }
-    load_col<C, M>(sp, gprs, n1, lane);
+    if (prs64) load_col<C, M>(sp, prs64 + (size_t)widx * n1, n1, lane);
+    else load_col<C, M>(sp, gprs, n1, lane);
     __syncwarp();
     if (rk == 1) sub_grad<T, M>(su, sv, sw, sp, rk_press, kx, kz, ny, gd, lane);
     // ---- stage B: Helmholtz solves for u, w (ny+1 rows, d2h) and v (ny rows, d2n)
@@ -475,14 +482,22 @@ __global__ void __launch_bounds__(128) k_rhs(cplx_t<S>* __restrict__ vel,
           }
         }
         gcru[q * n1 + j] = cvt<SC>(v);
+        if (cru64) cru64[((size_t)widx * 3 + q) * n1 + j] = cvt<double2>(v);
       }
     }
   } else {
-    for (int q = 0; q < 3; ++q) store_col<C, M>(gcru + q * n1, scol[q], n1, lane);
+    for (int q = 0; q < 3; ++q) {
+      store_col<C, M>(gcru + q * n1, scol[q], n1, lane);
+      if (cru64) store_col<C, M>(cru64 + ((size_t)widx * 3 + q) * n1, scol[q], n1, lane);
+    }
   }
   __syncwarp();
-  for (int q = 0; q < 3; ++q) store_col<C, M>(gvel + q * n1, scol[q], n1, lane);
+  for (int q = 0; q < 3; ++q) {
+    store_col<C, M>(gvel + q * n1, scol[q], n1, lane);
+    if (vel64) store_col<C, M>(vel64 + ((size_t)widx * 3 + q) * n1, scol[q], n1, lane);
+  }
   store_col<C, M>(gprs, sp, n1, lane);
+  if (prs64) store_col<C, M>(prs64 + (size_t)widx * n1, sp, n1, lane);
 }
 
 // The kx = kz = 0 mode in FP64 (PFC/pass2.f90:217-263, compute_p_grad

@@ -5,7 +5,8 @@
 //     whose pressure problem is ill-conditioned in FP32 on the stretched grid;
 //   - for all the others where the grid is so small that the main kernel
 //     (k_rhs2) would not fill the GPU.
-// The arithmetic is FP64 over the stored state.
+// The arithmetic is FP64 over the stored state; in mixed precision the mean
+// mode and the FP64 list keep FP64 columns beside their FP32 ones.
 //
 // What bounds these cases is the length of one block's chain, and a chain
 // executed once pays for every instruction it fetches: k_rhs2's form, several
@@ -106,9 +107,10 @@ __device__ __forceinline__ cplx_t<T> d2_of_row(const cplx_t<T>* s, const double*
   return mk<C>(d1 * fm.x + d0 * f0.x + d3 * fp.x, d1 * fm.y + d0 * f0.y + d3 * fp.y);
 }
 
-// wavenumber w over the storage precision S; mean: the mean mode (w = 0)
+// wavenumber w over the storage precision S; mean: the mean mode (w = 0);
+// low: its place in the FP64 list, -1 outside it
 template <typename S>
-__device__ __forceinline__ void k_rhs_rows_body(int w, bool mean, const RhsRowsLaunch& a) {
+__device__ __forceinline__ void k_rhs_rows_body(int w, bool mean, int low, const RhsRowsLaunch& a) {
   using T = double;
   using C = cplx_t<T>;
   using CS = cplx_t<S>;
@@ -126,7 +128,11 @@ __device__ __forceinline__ void k_rhs_rows_body(int w, bool mean, const RhsRowsL
   CS* const gprs = (CS*)a.prs + (size_t)w * n1;
   const CS* const top = (const CS*)a.cbc_top;
   const CS* const bot = (const CS*)a.cbc_bot;
-  const bool side = mean && a.mcru64 != nullptr;
+  // the FP64 columns, where this wavenumber has them (the mean's pressure is 0)
+  const bool side = a.mcru64 != nullptr && (mean || low >= 0), side_p = side && !mean;
+  double2* const vel64 = mean ? a.mvel64 : a.lvel64 + (ptrdiff_t)low * 3 * n1;
+  double2* const cru64 = mean ? a.mcru64 : a.lcru64 + (ptrdiff_t)low * 3 * n1;
+  double2* const prs64 = a.lprs64 + (ptrdiff_t)low * n1;
   C* const sV = reinterpret_cast<C*>(smem_raw);   // 3 columns of nt rows
   C* const sP = sV + 3 * nt;                      // 1 column
   const C zero = czero<C>();
@@ -137,10 +143,10 @@ __device__ __forceinline__ void k_rhs_rows_body(int w, bool mean, const RhsRowsL
   C cr[3], nl[3], p = zero;
 #pragma unroll
   for (int q = 0; q < 3; ++q) {
-    cr[q] = !row ? zero : side ? cvt<C>(a.mcru64[q * n1 + j]) : cvt<C>(gcru[q * n1 + j]);
+    cr[q] = !row ? zero : side ? cru64[q * n1 + j] : cvt<C>(gcru[q * n1 + j]);
     nl[q] = row ? cvt<C>(gvel[q * n1 + j]) : zero;
   }
-  if (row && !mean) p = cvt<C>(gprs[j]);
+  if (row && !mean) p = side_p ? prs64[j] : cvt<C>(gprs[j]);
   const double dt = a.sc->dt;
   const T coef = (T)(a.rkt.B(rk) * dt);
   const T vis_imp = (T)(a.rkt.D(rk) * (dt / a.re));
@@ -306,11 +312,12 @@ __device__ __forceinline__ void k_rhs_rows_body(int w, bool mean, const RhsRowsL
       gvel[q * n1 + j] = cvt<CS>(v[q]);
       gcru[q * n1 + j] = cvt<CS>(acc[q]);
       if (side) {
-        a.mvel64[q * n1 + j] = cvt<double2>(v[q]);
-        a.mcru64[q * n1 + j] = cvt<double2>(acc[q]);
+        vel64[q * n1 + j] = v[q];
+        cru64[q * n1 + j] = acc[q];
       }
     }
     gprs[j] = cvt<CS>(pn);
+    if (side_p) prs64[j] = pn;
   }
   if (mean) {
     const double* dm = gd.dm;
@@ -327,8 +334,8 @@ __device__ __forceinline__ void k_rhs_rows_body(int w, bool mean, const RhsRowsL
 // block b of the launch: the mean mode (a.mean), the FP64 list, the fast list
 template <typename S>
 __device__ __forceinline__ void k_rhs_rows_block(int b, const RhsRowsLaunch& a) {
-  const int low = a.mean + a.nlist;
-  k_rhs_rows_body<S>(b < a.mean ? 0 : b < low ? a.wlist[b - a.mean] : a.wfast[b - low], b < a.mean, a);
+  const int i = b - a.mean;   // place in the FP64 list, then in the fast list
+  k_rhs_rows_body<S>(i < 0 ? 0 : i < a.nlist ? a.wlist[i] : a.wfast[i - a.nlist], i < 0, i < a.nlist ? i : -1, a);
 }
 
 }  // namespace cfd

@@ -72,6 +72,7 @@ struct RhsRowsLaunch {
   int advance;                // the mean mode's block adds dt to t_total
   const int* wlist;           // FP64 list
   int nlist;
+  double2 *lvel64, *lcru64, *lprs64;   // its FP64 columns (nlist x 3 x ny1 and nlist x ny1)
   const int* wfast;           // the fast list, nfast 0 where k_rhs2 takes it
   int nfast;
   int pdl;
