@@ -189,6 +189,11 @@ struct cfg_ctx {
   // current state (not after a solve that reads the FP32 columns).
   double2 *lvel64 = nullptr, *lcru64 = nullptr, *lprs64 = nullptr;
   bool low_ok = true;
+  // the wall jet in FP64 for the list: its planes, the wall values of v (bot,
+  // top) and whether they are the current ones
+  double* jphys64 = nullptr;
+  double2* jet64 = nullptr;
+  bool jet_ok = false;
   void *T1 = nullptr, *T2 = nullptr;
   // physical planes of the split x stage (k_xinv_r -> k_flux_r)
   void* P = nullptr;
@@ -830,6 +835,7 @@ struct Impl {
     m.advance = c->advance ? 1 : 0;
     m.wlist = c->wl_prec; m.nlist = c->n_prec;
     m.lvel64 = c->lvel64; m.lcru64 = c->lcru64; m.lprs64 = c->lprs64;
+    m.jet64 = c->jet_ok ? c->jet64 : nullptr;
     m.wfast = c->wl_fast; m.nfast = c->rhs_rows ? c->n_fast : 0;
     m.st = c->rhs_rows ? c->st : c->st2;
     m.pdl = c->chained && c->rhs_rows ? 1 : 0;   // (the side stream's launch follows an event)
@@ -1021,7 +1027,8 @@ struct Impl {
     k_jet_walk<<<1, 32, 0, c->st>>>(c->jst, c->jp, c->sc, c->rkt, rk, time, incr, use_sc);
     CKL();
     prof_begin(c, "k_jet_field");
-    k_jet_field<T><<<dim3(g.nz, 3), 128, 0, c->st>>>((T*)c->pw_phys, c->jp, c->jst, g.nx, g.nz, c->p.lx, c->p.lz);
+    k_jet_field<T><<<dim3(g.nz, 3), 128, 0, c->st>>>((T*)c->pw_phys, c->jphys64, c->jp, c->jst, g.nx, g.nz, c->p.lx,
+                                                     c->p.lz);
     CKL();
     int r = small_r2c(c, (const T*)c->pw_phys, 3, (C*)c->pw_in, (size_t)g.nw, g.nz, 1, (C*)c->pw_H);
     if (r) return r;
@@ -1029,6 +1036,13 @@ struct Impl {
     k_jet_combine<T><<<(g.nw + 255) / 256, 256, 0, c->st>>>((const C*)c->pw_in, (C*)c->cbc, c->jp, c->gd, g.nx,
                                                              g.nz, g.nxh, c->p.lx, c->p.lz);
     CKL();
+    c->jet_ok = c->jet64 && !step_keeps_sums(c);
+    if (c->jet_ok) {
+      prof_begin(c, "k_jet_low");
+      k_jet_low<<<c->n_prec, 256, 0, c->st>>>(c->n_prec, c->wl_prec, c->jphys64, (const float2*)c->cbc, c->jet64, c->jp,
+                                              c->gd, g.nx, g.nz, g.nxh, c->p.lx, c->p.lz);
+      CKL();
+    }
     return CFG_OK;
   }
 
@@ -1061,6 +1075,7 @@ struct Impl {
   static int boundary(cfg_ctx* c) {
     const Geom& g = c->g;
     CK(cudaMemsetAsync(c->cbc, 0, sizeof(C) * 6 * (size_t)g.nw, c->st));
+    c->jet_ok = false;
     const size_t np = (size_t)g.nx2 * g.nz2;
     for (int q = 0; q < 3; q += 2) {
       const double gain = q == 0 ? c->p.ctrlu : c->p.ctrlw;
@@ -1372,7 +1387,7 @@ void cfg_destroy(cfg_ctx* c) {
   if (c->st_io) cudaStreamDestroy(c->st_io);
   for (void* q : c->ipc_open) cudaIpcCloseMemHandle(q);
   void* bufs[] = {c->dgrid, c->fringe, c->vel, c->cru, c->prs, c->mvel64, c->mcru64, c->lvel64, c->lcru64,
-                  c->lprs64, c->T1, c->T2, c->P,
+                  c->lprs64, c->jphys64, c->jet64, c->T1, c->T2, c->P,
                   c->rhs2_tbl, c->rhs2_tbl64, c->jst, c->pp_wy, c->pp_sy, c->pp_acc, c->cbc,
                   c->sc, c->d_um_dy, c->cflp, c->cflbits, c->l2acc, c->divbits, c->plist, c->pw_H,
                   c->pw_phys, c->pw_phys2, c->pw_in, c->stage, c->twx, c->twz, c->twxs, c->twzs,
@@ -1498,6 +1513,7 @@ int cfg_set_wall_bc(cfg_ctx* c, const double* top, const double* bot) {
   int r = ensure_stage(c, 2 * n);
   if (r) return r;
   const double* src[2] = {bot, top};
+  c->jet_ok = false;
   for (int k = 0; k < 2; ++k) {
     if (!src[k]) continue;
     CK(cudaMemcpyAsync(c->stage, src[k], sizeof(double2) * n, cudaMemcpyHostToDevice, c->st));
@@ -1884,6 +1900,10 @@ int cfg_set_jet(cfg_ctx* c, const cfg_jet* j) {
   p.jet_diam = j->jet_diam; p.width = j->width; p.freq = j->freq; p.frac_xbuff = j->frac_xbuff;
   p.filter = j->filter_jet_profile; p.seed = j->seed;
   if (!c->jst && cudaMalloc(&c->jst, sizeof(JetState)) != cudaSuccess) return fail(c, CFG_E_NOMEM, "jet state");
+  if (c->n_prec > 0 &&
+      ((!c->jphys64 && cudaMalloc(&c->jphys64, sizeof(double) * 3 * c->g.nx * c->g.nz) != cudaSuccess) ||
+       (!c->jet64 && cudaMalloc(&c->jet64, sizeof(double2) * 2 * c->n_prec) != cudaSuccess)))
+    return fail(c, CFG_E_NOMEM, "jet planes");
   JetState h{};
   memcpy(h.jf, j->jet_forcing, sizeof(h.jf));
   memcpy(h.inc, j->jet_forcing_incr, sizeof(h.inc));
@@ -3010,6 +3030,9 @@ struct EnsJet {
   const DevScalars* sc;
   RkTab rkt;
   float* phys;
+  double* phys64;
+  double2* jet64;
+  const int* list;
   float2 *H, *spec, *cbc;
   GridDev gd;
   FftPlan px, pz;
@@ -3040,8 +3063,8 @@ __global__ void k_jet_walk_b(const EnsJet* __restrict__ tab, int rk) {
 __global__ void k_jet_field_b(const EnsJet* __restrict__ tab, unsigned gx) {
   const unsigned m = blockIdx.x / gx;
   const EnsJet& a = tab[m];
-  k_jet_field_body<float>(make_uint3(blockIdx.x - m * gx, blockIdx.y, 0), a.phys, a.jp, a.st, a.nx, a.nz, a.lx,
-                          a.lz);
+  k_jet_field_body<float>(make_uint3(blockIdx.x - m * gx, blockIdx.y, 0), a.phys, a.phys64, a.jp, a.st, a.nx, a.nz,
+                          a.lx, a.lz);
 }
 
 __global__ void k_px_fwd_b(const EnsJet* __restrict__ tab, unsigned gx) {
@@ -3063,6 +3086,13 @@ __global__ void k_jet_combine_b(const EnsJet* __restrict__ tab, unsigned gx) {
   const EnsJet& a = tab[m];
   k_jet_combine_body<float>(make_uint3(blockIdx.x - m * gx, 0, 0), a.spec, a.cbc, a.jp, a.gd, a.nx, a.nz, a.nxh,
                             a.lx, a.lz);
+}
+
+__global__ void __launch_bounds__(256) k_jet_low_b(const EnsJet* __restrict__ tab, unsigned gx) {
+  const unsigned m = blockIdx.x / gx;
+  const EnsJet& a = tab[m];
+  k_jet_low_body((int)(blockIdx.x - m * gx), (int)gx, a.list, a.phys64, a.cbc, a.jet64, a.jp, a.gd, a.nx, a.nz, a.nxh,
+                 a.lx, a.lz);
 }
 
 // one class of a batched ensemble: members with the same grid and tiles
@@ -3192,6 +3222,7 @@ static int ens_build_classes(cfg_ensemble* e) {
         r2[(rk - 1) * n + q] = I::rhs2_args(c, rk, false);
         rl[(rk - 1) * n + q] = I::rows_args(c, rk);
         rl[(rk - 1) * n + q].advance = rk == 3;
+        rl[(rk - 1) * n + q].jet64 = c->crossflow ? c->jet64 : nullptr;
         flux[(rk - 1) * n + q].mean64 = c->mvel64;
       }
       EnsMember& a = sm[q];
@@ -3215,6 +3246,9 @@ static int ens_build_classes(cfg_ensemble* e) {
       a.sc = c->sc;
       a.rkt = c->rkt;
       a.phys = (float*)c->pw_phys;
+      a.phys64 = c->jphys64;
+      a.jet64 = c->jet64;
+      a.list = c->wl_prec;
       a.H = (float2*)c->pw_H;
       a.spec = (float2*)c->pw_in;
       a.cbc = (float2*)c->cbc;
@@ -3328,6 +3362,11 @@ static int ens_class_enqueue(cfg_ensemble* e, EnsClass& k) {
       const unsigned gxc = (unsigned)((k.ncbc / 6 + 255) / 256);
       k_jet_combine_b<<<gxc * nj, 256, 0, k.st>>>(k.jt, gxc);
       launches += 5;
+      const unsigned nl = (unsigned)c0->n_prec;
+      if (nl > 0) {
+        k_jet_low_b<<<nl * nj, 256, 0, k.st>>>(k.jt, nl);
+        ++launches;
+      }
       if (int r = ck(true, "batched wall jet")) return r;
     }
     // the FP64 |k| < 4 list and the mean mode beside the main kernel

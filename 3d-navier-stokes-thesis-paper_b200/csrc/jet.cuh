@@ -9,6 +9,8 @@
 //                   Gaussian spanwise slot)
 //   k_jet_combine : after the small forward transforms: filter_cosine passes
 //                   (:658-671), top-wall sign, suction balance (:493-537)
+//   k_jet_low     : mixed precision: the same coefficients in FP64 for the
+//                   |k| < 4 list
 #pragma once
 #include <cstdint>
 
@@ -90,9 +92,10 @@ __device__ __forceinline__ double abs_cmplx_single(double a, double b) {
 }
 
 // grid (nz, 3), block 128: planes 0 suction, 1 bottom jet, 2 top jet;
-// phys[p][z][x] on the nx x nz grid
+// phys[p][z][x] on the nx x nz grid, in FP64 to phys64 too when given
 template <typename T>
-__device__ __forceinline__ void k_jet_field_body(const uint3 bid, T* __restrict__ phys, JetParams jp,
+__device__ __forceinline__ void k_jet_field_body(const uint3 bid, T* __restrict__ phys, double* __restrict__ phys64,
+                                                 JetParams jp,
                                                  const JetState* __restrict__ st, int nx, int nz, double lx,
                                                  double lz) {
   const int z = bid.x, p = bid.y;
@@ -152,13 +155,14 @@ __device__ __forceinline__ void k_jet_field_body(const uint3 bid, T* __restrict_
       }
     }
     phys[((size_t)p * nz + z) * nx + x] = (T)v;
+    if (phys64) phys64[((size_t)p * nz + z) * nx + x] = v;
   }
 }
 
 template <typename T>
-__global__ void k_jet_field(T* __restrict__ phys, JetParams jp, const JetState* __restrict__ st, int nx, int nz,
-                            double lx, double lz) {
-  k_jet_field_body<T>(blockIdx, phys, jp, st, nx, nz, lx, lz);
+__global__ void k_jet_field(T* __restrict__ phys, double* __restrict__ phys64, JetParams jp,
+                            const JetState* __restrict__ st, int nx, int nz, double lx, double lz) {
+  k_jet_field_body<T>(blockIdx, phys, phys64, jp, st, nx, nz, lx, lz);
 }
 
 // spec[p][kx][kz] (p = 0 suction, 1 bottom, 2 top) -> cbc(:,:,2) of the
@@ -204,6 +208,72 @@ template <typename T>
 __global__ void k_jet_combine(const cplx_t<T>* __restrict__ spec, cplx_t<T>* __restrict__ cbc, JetParams jp,
                               GridDev gd, int nx, int nz, int nxh, double lx, double lz) {
   k_jet_combine_body<T>(blockIdx, spec, cbc, jp, gd, nx, nz, nxh, lx, lz);
+}
+
+// k_jet_low: grid (n), block 256: the forced walls' coefficients of the list's
+// wavenumbers in FP64, out[wall][n], by direct sums over the planes phys64.
+// The change of a wall value from substep to substep reaches the pressure
+// divided by k dt, and the rounding of FP32 values with it: 1e-6 of velocity
+// and pressure together, all of it in the lowest few kx (36x46x24, dt 0.002,
+// jet amplitude 0.1).  Nyquist coefficients keep the FP32 value (cbc, after
+// k_jet_combine).
+__device__ __forceinline__ void k_jet_low_body(int i, int n, const int* __restrict__ list,
+                                               const double* __restrict__ phys64, const float2* __restrict__ cbc,
+                                               double2* __restrict__ out, JetParams jp, GridDev gd, int nx, int nz,
+                                               int nxh, double lx, double lz) {
+  __shared__ double red[9][8];
+  const int w = list[i], kx = w / nz, kz = w % nz, t = threadIdx.x;
+  const size_t np = (size_t)nx * nz, nw = (size_t)nz * nxh;
+  double a[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};   // per plane: the coefficient, the mean
+  for (size_t q = t; q < np; q += 256) {
+    const int x = (int)(q % nx), z = (int)(q / nx);
+    double sn, cs;
+    sincospi(2.0 * ((double)((long long)kx * x % nx) / nx + (double)((long long)kz * z % nz) / nz), &sn, &cs);
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+      const double v = phys64[p * np + q];
+      a[3 * p] += v * cs;
+      a[3 * p + 1] -= v * sn;
+      a[3 * p + 2] += v;
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < 9; ++r) {
+    for (int o = 16; o > 0; o >>= 1) a[r] += __shfl_xor_sync(0xffffffffu, a[r], o);
+    if ((t & 31) == 0) red[r][t >> 5] = a[r];
+  }
+  __syncthreads();
+  if (t >= 2) return;
+  for (int r = 0; r < 9; ++r) {
+    a[r] = 0.0;
+    for (int o = 0; o < 8; ++o) a[r] += red[r][o];
+  }
+  const int wall = t;
+  if (kx == nx / 2 || kz == nz / 2) {
+    const float2 v = cbc[((size_t)wall * 3 + 1) * nw + w];
+    out[(size_t)wall * n + i] = make_double2((double)v.x, (double)v.y);
+    return;
+  }
+  double2 v = make_double2(0.0, 0.0);
+  if (jp.mode != 0 && jp.jetmag[wall] != 0.0) {
+    const double pi = 3.14159265358979323846;
+    const double fx = 1.0 + cos(pi * gd.kx[kx] / ((double)(nx / 2) * 2.0 * pi / lx));
+    const double fz = 1.0 + cos(pi * gd.kz[kz] / ((double)(nz / 2) * 2.0 * pi / lz));
+    double f = 1.0 / (double)np;
+    for (int r = 0; r < jp.filter; ++r) f *= 0.25 * fx * fz;
+    const double sg = wall == 1 ? -1.0 : 1.0;
+    const double* const j = a + 3 * (1 + wall);
+    const double q = sg * j[2] / a[2];
+    v = make_double2(f * (sg * j[0] - q * a[0]), f * (sg * j[1] - q * a[1]));
+  }
+  out[(size_t)wall * n + i] = v;
+}
+
+__global__ void __launch_bounds__(256) k_jet_low(int n, const int* __restrict__ list,
+                                                 const double* __restrict__ phys64, const float2* __restrict__ cbc,
+                                                 double2* __restrict__ out, JetParams jp, GridDev gd, int nx, int nz,
+                                                 int nxh, double lx, double lz) {
+  k_jet_low_body((int)blockIdx.x, n, list, phys64, cbc, out, jp, gd, nx, nz, nxh, lx, lz);
 }
 
 // ---------------------------------------------------------------------------

@@ -198,12 +198,14 @@ __device__ __forceinline__ void k_rhs_rows_body(int w, bool mean, int low, const
     v[0].x -= (T)(cos(a.beta) * rk_press * pg);
     v[2].x -= (T)(sin(a.beta) * rk_press * pg);
   }
-  // Helmholtz solves: u and w (d2h), v (d2n), wall rows from cbc
+  // Helmholtz solves: u and w (d2h), v (d2n), wall rows from cbc or, v of the
+  // FP64 list with the wall jet, in FP64
   {
+    const double2* const jet = low >= 0 ? a.jet64 : nullptr;
     T ca[2] = {0, 0}, cc[2] = {0, 0}, ce[2] = {1, 1};
     C f[3] = {zero, zero, zero};
     if (j == 0) {
-      f[0] = cvt<C>(bot[w]); f[1] = cvt<C>(bot[2 * nw + w]); f[2] = cvt<C>(bot[nw + w]);
+      f[0] = cvt<C>(bot[w]); f[1] = cvt<C>(bot[2 * nw + w]); f[2] = jet ? jet[low] : cvt<C>(bot[nw + w]);
     } else {
       if (j == n1 - 1) {
         f[0] = cvt<C>(top[w]); f[1] = cvt<C>(top[2 * nw + w]);
@@ -216,7 +218,7 @@ __device__ __forceinline__ void k_rhs_rows_body(int w, bool mean, int low, const
         f[1] = cscale(r, v[2]);
       }
       if (j == ny - 1) {
-        f[2] = cvt<C>(top[nw + w]);
+        f[2] = jet ? jet[a.nlist + low] : cvt<C>(top[nw + w]);
       } else if (j < ny - 1) {
         const T r = rcpv<T>(alpha - vis_imp * (T)gd.d2n[3 * j + 1]);
         ca[1] = vis_imp * (T)gd.d2n[3 * j] * r;

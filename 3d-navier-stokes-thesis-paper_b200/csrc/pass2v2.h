@@ -73,6 +73,7 @@ struct RhsRowsLaunch {
   const int* wlist;           // FP64 list
   int nlist;
   double2 *lvel64, *lcru64, *lprs64;   // its FP64 columns (nlist x 3 x ny1 and nlist x ny1)
+  const double2* jet64;       // the list's wall-normal wall values [bot, top][nlist], or null (cbc)
   const int* wfast;           // the fast list, nfast 0 where k_rhs2 takes it
   int nfast;
   int pdl;

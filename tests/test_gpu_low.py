@@ -7,6 +7,10 @@
   is left is the rounding of the FP32 transforms, 1.2e-7 of the nonlinear term
   at every length, and of the |k| >= 4 columns, whose part of the pressure is
   at least 16 times smaller: the bar, against the same run in FP64, is 1.2e-7.
+- The wall jet, whose rounding in FP32 changes from substep to substep and
+  reaches the pressure divided by k dt: 1e-6 of the norm, all of it at kx of
+  0.5 and 1.  Its coefficients at |k| < 4 are in FP64; the others' part is at
+  most an eighth of that.  The bar: an eighth of 1e-6 and the 1.2e-7 of a run.
 - Where the columns can go out of date or get lost: a state taken out and put
   back (at the end of a step and within one, through the arrays and through
   the restart file), the learned closure's solves, which read the FP32
@@ -83,6 +87,33 @@ def test_error_of_a_run(cf, nx, ny, nz, dt):
         f.close()
     err = np.linalg.norm(out[1] - out[0]) / np.linalg.norm(out[0])
     assert err < 1.2e-7, err
+
+
+def slot_jet(cf):
+    j = cf.CfgJet()
+    j.mode = 2
+    j.xjet[0], j.zjet[0] = 0.3 * LX, 0.5 * LZ
+    j.jetmag[0] = 0.1
+    j.width, j.freq, j.frac_xbuff, j.seed = 0.2, 0.5, 0.2, 2
+    return j
+
+
+@pytest.mark.parametrize("dt_flag", [0, 1])
+@pytest.mark.parametrize("nx,ny,nz,dt", [(36, 46, 24, 0.002), (32, 86, 36, 0.002), (96, 30, 48, 0.002)])
+def test_error_of_a_run_with_the_wall_jet(cf, nx, ny, nz, dt, dt_flag):
+    out = []
+    for prec in (0, 1):
+        f = cf.ChannelFlow(cf.Grid(nx, ny, nz, lx=LX, lz=LZ, stretch=1.5), re=3000.0, dt=dt, precision=prec,
+                           dt_flag=dt_flag, cfl_max=0.05)
+        start(f, nx)
+        f.set_jet(slot_jet(cf))
+        f.timestep(40)
+        d1, _, d4 = f.download_state()
+        assert f.status() == 0
+        out.append(np.concatenate([d1.ravel(), d4.ravel()]))
+        f.close()
+    err = np.linalg.norm(out[1] - out[0]) / np.linalg.norm(out[0])
+    assert err < 2.45e-7, err
 
 
 @pytest.mark.parametrize("nx,ny,nz", [(32, 33, 32), (96, 40, 96)])
