@@ -92,6 +92,11 @@ struct Scatter {
 // fill of the SMs run under the previous kernel's last blocks (a chain of
 // twelve 5 us kernels a step on the smallest grids).  Without the launch
 // attribute both are no-ops.
+// What an earlier kernel of the chain writes is still being written while a
+// dependent's blocks are resident: it is read by plain loads after pdl_wait(),
+// through pointers without __restrict__, never by __ldg or another load that
+// takes the data as constant for the kernel's lifetime.  Tables (twiddles,
+// wavenumbers, grid metrics, the fringe) are constant and keep both.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

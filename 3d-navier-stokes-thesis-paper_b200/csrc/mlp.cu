@@ -73,13 +73,13 @@ __device__ __forceinline__ void issue_dw(uint32_t d, uint32_t sDZ, uint32_t sX, 
 // ------------------------------------------------------------- tile helpers
 // half of a point's features into X0 (10, BF16, padded to 16; half 0 features
 // 0-7, half 1 the other two); rows are 8-byte aligned
-__device__ __forceinline__ void load_x0(uint4* sm, const float* __restrict__ x, long long row, bool valid, int p,
+__device__ __forceinline__ void load_x0(uint4* sm, const float* x, long long row, bool valid, int p,
                                         int half) {
   const float2* src = reinterpret_cast<const float2*>(x + row * IN) + 4 * half;
   float v[8];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const float2 f = valid && (half == 0 || i == 0) ? __ldg(src + i) : make_float2(0.f, 0.f);
+    const float2 f = valid && (half == 0 || i == 0) ? src[i] : make_float2(0.f, 0.f);
     v[2 * i] = f.x;
     v[2 * i + 1] = f.y;
   }
@@ -230,10 +230,9 @@ __global__ void __launch_bounds__(TILE) k_mlp_fwd(const uint4* __restrict__ img,
 // every weight gradient by the one thread that holds it, every bias gradient
 // and the loss as the sum of the four warps' sums in warp order, so that the
 // slice does not depend on the order in which warps or tiles finish.
-__global__ void __launch_bounds__(NTH, 1) k_mlp_train(const uint4* __restrict__ img, const float* __restrict__ bias,
-                                                      const float* __restrict__ x, const float* __restrict__ t,
-                                                      const int* __restrict__ idx, int batch,
-                                                      float* __restrict__ part, int* __restrict__ err) {
+__global__ void __launch_bounds__(NTH, 1) k_mlp_train(const uint4* img, const float* bias,
+                                                      const float* x, const float* t, const int* idx, int batch,
+                                                      float* part, int* err) {
   extern __shared__ __align__(128) uint4 sm[];
   __shared__ __align__(8) uint64_t bar;
   __shared__ uint32_t tslot;
@@ -294,7 +293,7 @@ __global__ void __launch_bounds__(NTH, 1) k_mlp_train(const uint4* __restrict__ 
       for (int c = 0; c < 16; ++c) {
         dz[c] = 0.f;
         if (c < OUT && valid) {
-          const float d = z[c] + sb[bias_base(3) + c] - __ldg(t + row * OUT + c);
+          const float d = z[c] + sb[bias_base(3) + c] - t[row * OUT + c];
           lsum += d * d;
           dz[c] = sc * d;
         }
@@ -375,15 +374,14 @@ __global__ void __launch_bounds__(NTH, 1) k_mlp_train(const uint4* __restrict__ 
 // accumulators (the same sums, bit for bit, on every run); blocks of one warp
 // pair, so that the few thousand sums spread over the SMs, and 16 slices'
 // loads in flight
-__global__ void __launch_bounds__(64) k_mlp_reduce(const float* __restrict__ part, int ntiles, float* __restrict__ G,
-                             float* __restrict__ loss) {
+__global__ void __launch_bounds__(64) k_mlp_reduce(const float* part, int ntiles, float* G, float* loss) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   cfd::pdl_trigger();
   cfd::pdl_wait();
   if (i > NPARAM) return;
   float s = 0.f;
 #pragma unroll 16
-  for (int b = 0; b < ntiles; ++b) s += __ldcg(part + (size_t)b * PART_STRIDE + i);
+  for (int b = 0; b < ntiles; ++b) s += part[(size_t)b * PART_STRIDE + i];
   if (i < NPARAM) G[i] += s;
   else *loss += s;
 }

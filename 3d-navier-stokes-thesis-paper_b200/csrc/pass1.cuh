@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(256) k_zfwd(const cplx_t<T>* __restrict__ T2,
 // check_cfl + dt adaptation (PFC/pass1.f90:202-250, 106-124): one block.
 // reset: the maxima are cleared for the next step.
 template <bool LIN>
-__device__ __forceinline__ void k_cfl_finalize_body(const uint3 bid, unsigned long long* __restrict__ cflbits, int reset,
+__device__ __forceinline__ void k_cfl_finalize_body(const uint3 bid, unsigned long long* cflbits, int reset,
                                                     Geom g, GridDev gd, DevScalars* sc, double* cfl, double lx,
                                                     double lz, int dt_flag, double cfl_max_param, int step) {
   __shared__ double smax[256];
@@ -402,7 +402,7 @@ __device__ __forceinline__ void k_cfl_finalize_body(const uint3 bid, unsigned lo
 }
 
 template <bool LIN>
-__global__ void k_cfl_finalize(unsigned long long* __restrict__ cflbits, int reset, Geom g, GridDev gd, DevScalars* sc,
+__global__ void k_cfl_finalize(unsigned long long* cflbits, int reset, Geom g, GridDev gd, DevScalars* sc,
                                double* cfl, double lx, double lz, int dt_flag, double cfl_max_param, int step) {
   k_cfl_finalize_body<LIN>(blockIdx, cflbits, reset, g, gd, sc, cfl, lx, lz, dt_flag, cfl_max_param, step);
 }

@@ -80,8 +80,8 @@ template <typename T, int N, int YP> struct ZShape {
 // gathered with cp.async into a raw tile first, so that all of its loads are
 // in flight at once.
 template <typename T, int NZ2, int YP, bool DEAL>
-__device__ __forceinline__ void k_zinv_r_body(const uint3 bid, const cplx_t<T>* __restrict__ vel,
-                                              cplx_t<T>* __restrict__ T1, Geom g, const cplx_t<T>* __restrict__ twz,
+__device__ __forceinline__ void k_zinv_r_body(const uint3 bid, const cplx_t<T>* vel,
+                                              cplx_t<T>* T1, Geom g, const cplx_t<T>* __restrict__ twz,
                                               Scatter sc, int split) {
   using C = cplx_t<T>;
   using Z = ZShape<T, NZ2, YP>;
@@ -187,7 +187,7 @@ __device__ __forceinline__ void k_zinv_r_body(const uint3 bid, const cplx_t<T>* 
 
 template <typename T, int NZ2, int YP, bool DEAL>
 __global__ void __launch_bounds__(ZShape<T, NZ2, YP>::INV_NT, ZShape<T, NZ2, YP>::blocks(ZShape<T, NZ2, YP>::INV_NT, sizeof(T) == 4))
-k_zinv_r(const cplx_t<T>* __restrict__ vel, cplx_t<T>* __restrict__ T1, Geom g, const cplx_t<T>* __restrict__ twz,
+k_zinv_r(const cplx_t<T>* vel, cplx_t<T>* T1, Geom g, const cplx_t<T>* __restrict__ twz,
          Scatter sc, int split) {
   k_zinv_r_body<T, NZ2, YP, DEAL>(blockIdx, vel, T1, g, twz, sc, split);
 }
@@ -197,8 +197,8 @@ k_zinv_r(const cplx_t<T>* __restrict__ vel, cplx_t<T>* __restrict__ T1, Geom g, 
 // one equation's two parts, fold, scale and ikz combine
 // (PFC/transform.f90:317-333, 639-688).
 template <typename T, int NZ2, int YP, bool DEAL>
-__device__ __forceinline__ void k_zfwd_r_body(const uint3 bid, const cplx_t<T>* __restrict__ T2,
-                                              cplx_t<T>* __restrict__ vel, Geom g, const cplx_t<T>* __restrict__ twz,
+__device__ __forceinline__ void k_zfwd_r_body(const uint3 bid, const cplx_t<T>* T2,
+                                              cplx_t<T>* vel, Geom g, const cplx_t<T>* __restrict__ twz,
                                               GridDev gd) {
   using C = cplx_t<T>;
   using Z = ZShape<T, NZ2, YP>;
@@ -287,7 +287,7 @@ __device__ __forceinline__ void k_zfwd_r_body(const uint3 bid, const cplx_t<T>* 
 
 template <typename T, int NZ2, int YP, bool DEAL>
 __global__ void __launch_bounds__(ZShape<T, NZ2, YP>::FWD_NT, ZShape<T, NZ2, YP>::blocks(ZShape<T, NZ2, YP>::FWD_NT, sizeof(T) == 4))
-k_zfwd_r(const cplx_t<T>* __restrict__ T2, cplx_t<T>* __restrict__ vel, Geom g, const cplx_t<T>* __restrict__ twz,
+k_zfwd_r(const cplx_t<T>* T2, cplx_t<T>* vel, Geom g, const cplx_t<T>* __restrict__ twz,
          GridDev gd) {
   k_zfwd_r_body<T, NZ2, YP, DEAL>(blockIdx, T2, vel, g, twz, gd);
 }
@@ -657,7 +657,7 @@ template <int N, int ZB> __host__ __device__ constexpr int xinv_threads() {
 // 133 / 106 at 256x193x256 mixed (5.4 TB/s), 389 / 256 at 384x193x384, 304 /
 // 220 in FP64 at 256x193x256.
 template <typename T, int NX2, int ZB, bool DEAL>
-__device__ __forceinline__ void k_xinv_r_body(const uint3 bid, const cplx_t<T>* __restrict__ T1, T* __restrict__ P,
+__device__ __forceinline__ void k_xinv_r_body(const uint3 bid, const cplx_t<T>* T1, T* P,
                                               Geom g, const cplx_t<T>* __restrict__ twx) {
   using C = cplx_t<T>;
   constexpr int N1 = Split<NX2>::N1, N2 = Split<NX2>::N2, PITCH = N2 + 1, SEQ = SeqPitch<NX2>::V;
@@ -745,7 +745,7 @@ template <typename T, int N, int ZB> constexpr int xinv_blocks() {
 
 template <typename T, int NX2, int ZB, bool DEAL>
 __global__ void __launch_bounds__(xinv_threads<NX2, ZB>(), xinv_blocks<T, NX2, ZB>())
-k_xinv_r(const cplx_t<T>* __restrict__ T1, T* __restrict__ P, Geom g, const cplx_t<T>* __restrict__ twx) {
+k_xinv_r(const cplx_t<T>* T1, T* P, Geom g, const cplx_t<T>* __restrict__ twx) {
   k_xinv_r_body<T, NX2, ZB, DEAL>(blockIdx, T1, P, g, twx);
 }
 
@@ -777,11 +777,11 @@ template <typename T, int NT> __host__ __device__ constexpr int flux_blocks() {
 }
 
 template <typename T, int NX2, int ZR, int NT, int MODE>
-__device__ __forceinline__ void k_flux_r_body(const uint3 bid, const T* __restrict__ P, cplx_t<T>* __restrict__ T2,
+__device__ __forceinline__ void k_flux_r_body(const uint3 bid, const T* P, cplx_t<T>* T2,
                                               Geom g, const cplx_t<T>* __restrict__ twx, GridDev gd,
                                               const T* __restrict__ fringe, int has_fringe,
-                                              unsigned long long* __restrict__ cflbits, int do_cfl, Scatter sc,
-                                              const T* __restrict__ S, const double2* __restrict__ mean64) {
+                                              unsigned long long* cflbits, int do_cfl, Scatter sc,
+                                              const T* S, const double2* mean64) {
   constexpr int PROD = MODE % FLUX_KEEP;
   constexpr bool LIN = PROD == 1, SGS = PROD == 2, SPLIT = PROD == 3;
   constexpr bool OLDSUM = SGS || MODE >= FLUX_KEEP;
@@ -975,7 +975,7 @@ __device__ __forceinline__ void k_flux_r_body(const uint3 bid, const T* __restri
     const int x = 2 * (idx % (N / 2)), r = idx / (N / 2);
     if (TAIL && r >= nr) break;
     const size_t o = (size_t)r * N + x;
-    auto ld2 = [&](const T* b) { return __ldg(reinterpret_cast<const V2*>(b + o)); };
+    auto ld2 = [&](const T* b) { return *reinterpret_cast<const V2*>(b + o); };
     const V2 U = ld2(P0), V = ld2(P0 + cs), W = ld2(P0 + 2 * cs);
     const V2 Up = ld2(Pp), Wp = ld2(Pp + 2 * cs);
     const V2 Vp = (k < ny) ? ld2(Pp + cs) : V;
@@ -991,7 +991,7 @@ __device__ __forceinline__ void k_flux_r_body(const uint3 bid, const T* __restri
       const int pd[11] = {0, 0, 0, 0, 0, 0, -1, -1, 1, 1, 1};
 #pragma unroll
       for (int q = 0; q < 11; ++q) {
-        const V2 v = __ldg(reinterpret_cast<const V2*>(S + (size_t)((long long)so + (long long)pd[q] * (long long)ss) +
+        const V2 v = *reinterpret_cast<const V2*>((S + (size_t)((long long)so + (long long)pd[q] * (long long)ss) +
                                                        (size_t)c0[q] * NZ2 * N));
         ta[q] = v.x;
         tb[q] = v.y;
@@ -1083,9 +1083,9 @@ __device__ __forceinline__ void k_flux_r_body(const uint3 bid, const T* __restri
 
 template <typename T, int NX2, int ZR, int NT, int MODE>
 __global__ void __launch_bounds__(NT, flux_blocks<T, NT>())
-k_flux_r(const T* __restrict__ P, cplx_t<T>* __restrict__ T2, Geom g, const cplx_t<T>* __restrict__ twx, GridDev gd,
-         const T* __restrict__ fringe, int has_fringe, unsigned long long* __restrict__ cflbits, int do_cfl,
-         Scatter sc, const T* __restrict__ S, const double2* __restrict__ mean64) {
+k_flux_r(const T* P, cplx_t<T>* T2, Geom g, const cplx_t<T>* __restrict__ twx, GridDev gd,
+         const T* __restrict__ fringe, int has_fringe, unsigned long long* cflbits, int do_cfl,
+         Scatter sc, const T* S, const double2* mean64) {
   k_flux_r_body<T, NX2, ZR, NT, MODE>(blockIdx, P, T2, g, twx, gd, fringe, has_fringe, cflbits, do_cfl, sc, S,
                                       mean64);
 }

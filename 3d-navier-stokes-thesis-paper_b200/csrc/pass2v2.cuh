@@ -162,10 +162,10 @@ __host__ __device__ __forceinline__ int rhs2_ld(int n1) { return (n1 + 1) & ~1; 
 // T is the arithmetic precision, S the storage precision of the state (the
 // mixed path runs its |k| < 4 list with T = double over S = float).
 template <typename T, typename S, int M, int G>
-__device__ __forceinline__ void k_rhs2_body(const uint3 bid, cplx_t<S>* __restrict__ vel, cplx_t<S>* __restrict__ cru,
-                                            cplx_t<S>* __restrict__ prs, const cplx_t<S>* __restrict__ cbc_top,
-                                            const cplx_t<S>* __restrict__ cbc_bot, Geom g, GridDev gd,
-                                            const DevScalars* __restrict__ sc, RkTab rkt, int rk, double re,
+__device__ __forceinline__ void k_rhs2_body(const uint3 bid, cplx_t<S>* vel, cplx_t<S>* cru,
+                                            cplx_t<S>* prs, const cplx_t<S>* cbc_top,
+                                            const cplx_t<S>* cbc_bot, Geom g, GridDev gd,
+                                            const DevScalars* sc, RkTab rkt, int rk, double re,
                                             const int* __restrict__ wlist, int nlist, const T* __restrict__ tbl) {
   using C = cplx_t<T>;
   using CS = cplx_t<S>;
@@ -427,9 +427,9 @@ __device__ __forceinline__ void k_rhs2_body(const uint3 bid, cplx_t<S>* __restri
 
 template <typename T, typename S, int M, int G>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 1)
-k_rhs2(cplx_t<S>* __restrict__ vel, cplx_t<S>* __restrict__ cru, cplx_t<S>* __restrict__ prs,
-       const cplx_t<S>* __restrict__ cbc_top, const cplx_t<S>* __restrict__ cbc_bot, Geom g, GridDev gd,
-       const DevScalars* __restrict__ sc, RkTab rkt, int rk, double re, const int* __restrict__ wlist, int nlist,
+k_rhs2(cplx_t<S>* vel, cplx_t<S>* cru, cplx_t<S>* prs,
+       const cplx_t<S>* cbc_top, const cplx_t<S>* cbc_bot, Geom g, GridDev gd,
+       const DevScalars* sc, RkTab rkt, int rk, double re, const int* __restrict__ wlist, int nlist,
        const T* __restrict__ tbl) {
   k_rhs2_body<T, S, M, G>(blockIdx, vel, cru, prs, cbc_top, cbc_bot, g, gd, sc, rkt, rk, re, wlist, nlist, tbl);
 }
