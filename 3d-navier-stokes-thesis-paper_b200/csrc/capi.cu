@@ -189,10 +189,10 @@ struct cfg_ctx {
   // current state (not after a solve that reads the FP32 columns).
   double2 *lvel64 = nullptr, *lcru64 = nullptr, *lprs64 = nullptr;
   bool low_ok = true;
-  // the wall jet in FP64 for the list: its planes, the wall values of v (bot,
-  // top) and whether they are the current ones
-  double* jphys64 = nullptr;
-  double2* jet64 = nullptr;
+  // the wall jet in FP64 for the list, whose kx are below low_nk: its planes'
+  // rows, the wall values of v (bot, top) and whether they are the current ones
+  double2 *jrows64 = nullptr, *jet64 = nullptr;
+  int low_nk = 0;
   bool jet_ok = false;
   void *T1 = nullptr, *T2 = nullptr;
   // physical planes of the split x stage (k_xinv_r -> k_flux_r)
@@ -1027,8 +1027,8 @@ struct Impl {
     k_jet_walk<<<1, 32, 0, c->st>>>(c->jst, c->jp, c->sc, c->rkt, rk, time, incr, use_sc);
     CKL();
     prof_begin(c, "k_jet_field");
-    k_jet_field<T><<<dim3(g.nz, 3), 128, 0, c->st>>>((T*)c->pw_phys, c->jphys64, c->jp, c->jst, g.nx, g.nz, c->p.lx,
-                                                     c->p.lz);
+    k_jet_field<T><<<dim3(g.nz, 3), 128, c->jrows64 ? jet_row_smem(g.nx) : 0, c->st>>>(
+        (T*)c->pw_phys, c->jrows64, c->low_nk, c->jp, c->jst, g.nx, g.nz, c->p.lx, c->p.lz);
     CKL();
     int r = small_r2c(c, (const T*)c->pw_phys, 3, (C*)c->pw_in, (size_t)g.nw, g.nz, 1, (C*)c->pw_H);
     if (r) return r;
@@ -1039,8 +1039,8 @@ struct Impl {
     c->jet_ok = c->jet64 && !step_keeps_sums(c);
     if (c->jet_ok) {
       prof_begin(c, "k_jet_low");
-      k_jet_low<<<c->n_prec, 256, 0, c->st>>>(c->n_prec, c->wl_prec, c->jphys64, (const float2*)c->cbc, c->jet64, c->jp,
-                                              c->gd, g.nx, g.nz, g.nxh, c->p.lx, c->p.lz);
+      k_jet_low<<<c->n_prec, 128, 0, c->st>>>(c->n_prec, c->wl_prec, c->jrows64, c->low_nk, (const float2*)c->cbc,
+                                              c->jet64, c->jp, c->gd, g.nx, g.nz, g.nxh, c->p.lx, c->p.lz);
       CKL();
     }
     return CFG_OK;
@@ -1318,6 +1318,7 @@ static int create_impl(const cfg_params* p, const cfg_grid* gr, const SlabPart* 
     }
     c->n_fast = (int)fast.size();
     c->n_prec = (int)prec.size();
+    c->low_nk = prec.empty() ? 0 : prec.back() / g.nz + 1;
     if (cudaMalloc(&c->wl_fast, sizeof(int) * std::max<size_t>(1, fast.size())) != cudaSuccess ||
         cudaMalloc(&c->wl_prec, sizeof(int) * std::max<size_t>(1, prec.size())) != cudaSuccess)
       return bad(CFG_E_NOMEM);
@@ -1387,7 +1388,7 @@ void cfg_destroy(cfg_ctx* c) {
   if (c->st_io) cudaStreamDestroy(c->st_io);
   for (void* q : c->ipc_open) cudaIpcCloseMemHandle(q);
   void* bufs[] = {c->dgrid, c->fringe, c->vel, c->cru, c->prs, c->mvel64, c->mcru64, c->lvel64, c->lcru64,
-                  c->lprs64, c->jphys64, c->jet64, c->T1, c->T2, c->P,
+                  c->lprs64, c->jrows64, c->jet64, c->T1, c->T2, c->P,
                   c->rhs2_tbl, c->rhs2_tbl64, c->jst, c->pp_wy, c->pp_sy, c->pp_acc, c->cbc,
                   c->sc, c->d_um_dy, c->cflp, c->cflbits, c->l2acc, c->divbits, c->plist, c->pw_H,
                   c->pw_phys, c->pw_phys2, c->pw_in, c->stage, c->twx, c->twz, c->twxs, c->twzs,
@@ -1901,7 +1902,7 @@ int cfg_set_jet(cfg_ctx* c, const cfg_jet* j) {
   p.filter = j->filter_jet_profile; p.seed = j->seed;
   if (!c->jst && cudaMalloc(&c->jst, sizeof(JetState)) != cudaSuccess) return fail(c, CFG_E_NOMEM, "jet state");
   if (c->n_prec > 0 &&
-      ((!c->jphys64 && cudaMalloc(&c->jphys64, sizeof(double) * 3 * c->g.nx * c->g.nz) != cudaSuccess) ||
+      ((!c->jrows64 && cudaMalloc(&c->jrows64, sizeof(double2) * 3 * c->low_nk * c->g.nz) != cudaSuccess) ||
        (!c->jet64 && cudaMalloc(&c->jet64, sizeof(double2) * 2 * c->n_prec) != cudaSuccess)))
     return fail(c, CFG_E_NOMEM, "jet planes");
   JetState h{};
@@ -3030,8 +3031,8 @@ struct EnsJet {
   const DevScalars* sc;
   RkTab rkt;
   float* phys;
-  double* phys64;
-  double2* jet64;
+  double2 *rows64, *jet64;
+  int nk;
   const int* list;
   float2 *H, *spec, *cbc;
   GridDev gd;
@@ -3063,8 +3064,8 @@ __global__ void k_jet_walk_b(const EnsJet* __restrict__ tab, int rk) {
 __global__ void k_jet_field_b(const EnsJet* __restrict__ tab, unsigned gx) {
   const unsigned m = blockIdx.x / gx;
   const EnsJet& a = tab[m];
-  k_jet_field_body<float>(make_uint3(blockIdx.x - m * gx, blockIdx.y, 0), a.phys, a.phys64, a.jp, a.st, a.nx, a.nz,
-                          a.lx, a.lz);
+  k_jet_field_body<float>(make_uint3(blockIdx.x - m * gx, blockIdx.y, 0), a.phys, a.rows64, a.nk, a.jp, a.st, a.nx,
+                          a.nz, a.lx, a.lz);
 }
 
 __global__ void k_px_fwd_b(const EnsJet* __restrict__ tab, unsigned gx) {
@@ -3088,11 +3089,11 @@ __global__ void k_jet_combine_b(const EnsJet* __restrict__ tab, unsigned gx) {
                             a.lx, a.lz);
 }
 
-__global__ void __launch_bounds__(256) k_jet_low_b(const EnsJet* __restrict__ tab, unsigned gx) {
+__global__ void __launch_bounds__(128) k_jet_low_b(const EnsJet* __restrict__ tab, unsigned gx) {
   const unsigned m = blockIdx.x / gx;
   const EnsJet& a = tab[m];
-  k_jet_low_body((int)(blockIdx.x - m * gx), (int)gx, a.list, a.phys64, a.cbc, a.jet64, a.jp, a.gd, a.nx, a.nz, a.nxh,
-                 a.lx, a.lz);
+  k_jet_low_body((int)(blockIdx.x - m * gx), (int)gx, a.list, a.rows64, a.nk, a.cbc, a.jet64, a.jp, a.gd, a.nx, a.nz,
+                 a.nxh, a.lx, a.lz);
 }
 
 // one class of a batched ensemble: members with the same grid and tiles
@@ -3246,7 +3247,8 @@ static int ens_build_classes(cfg_ensemble* e) {
       a.sc = c->sc;
       a.rkt = c->rkt;
       a.phys = (float*)c->pw_phys;
-      a.phys64 = c->jphys64;
+      a.rows64 = c->jrows64;
+      a.nk = c->low_nk;
       a.jet64 = c->jet64;
       a.list = c->wl_prec;
       a.H = (float2*)c->pw_H;
@@ -3355,7 +3357,7 @@ static int ens_class_enqueue(cfg_ensemble* e, EnsClass& k) {
       // nonlinear term on a side stream (from rk 2, when dt is final) it
       // measured slower: 8.70 against 8.62 ms per 64-member step
       k_jet_walk_b<<<nj, 32, 0, k.st>>>(k.jt, rk);
-      k_jet_field_b<<<dim3(k.nz * nj, 3), 128, 0, k.st>>>(k.jt, (unsigned)k.nz);
+      k_jet_field_b<<<dim3(k.nz * nj, 3), 128, jet_row_smem(k.nx), k.st>>>(k.jt, (unsigned)k.nz);
       const unsigned gxx = (unsigned)(k.nz + 1) / 2;
       k_px_fwd_b<<<dim3(gxx * nj, 3), 128, sizeof(float2) * 3 * k.nx, k.st>>>(k.jt, gxx);
       k_pz_fwd_b<<<dim3((unsigned)k.nxh * nj, 3), 128, sizeof(float2) * 3 * k.nz, k.st>>>(k.jt, (unsigned)k.nxh);
@@ -3364,7 +3366,7 @@ static int ens_class_enqueue(cfg_ensemble* e, EnsClass& k) {
       launches += 5;
       const unsigned nl = (unsigned)c0->n_prec;
       if (nl > 0) {
-        k_jet_low_b<<<nl * nj, 256, 0, k.st>>>(k.jt, nl);
+        k_jet_low_b<<<nl * nj, 128, 0, k.st>>>(k.jt, nl);
         ++launches;
       }
       if (int r = ck(true, "batched wall jet")) return r;

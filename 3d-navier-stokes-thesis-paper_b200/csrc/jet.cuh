@@ -92,16 +92,22 @@ __device__ __forceinline__ double abs_cmplx_single(double a, double b) {
 }
 
 // grid (nz, 3), block 128: planes 0 suction, 1 bottom jet, 2 top jet;
-// phys[p][z][x] on the nx x nz grid, in FP64 to phys64 too when given
+// phys[p][z][x] on the nx x nz grid.  With rows64: also the row's first nk
+// coefficients in FP64, rows64[p][kx][z] (not scaled), by direct sums;
+// dynamic shared memory jet_row_smem(nx)
+__host__ __device__ __forceinline__ size_t jet_row_smem(int nx) { return (size_t)nx * (sizeof(double2) + sizeof(double)); }
 template <typename T>
-__device__ __forceinline__ void k_jet_field_body(const uint3 bid, T* __restrict__ phys, double* __restrict__ phys64,
-                                                 JetParams jp,
+__device__ __forceinline__ void k_jet_field_body(const uint3 bid, T* __restrict__ phys, double2* __restrict__ rows64,
+                                                 int nk, JetParams jp,
                                                  const JetState* __restrict__ st, int nx, int nz, double lx,
                                                  double lz) {
   const int z = bid.x, p = bid.y;
   const double pi = 3.14159265358979323846;
   const double time = st->time;
   const double zc = (double)z * lz / (double)nz;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double2* const tw = reinterpret_cast<double2*>(smem_raw);   // exp(-2 pi i m / nx)
+  double* const row = reinterpret_cast<double*>(tw + nx);
   for (int x = threadIdx.x; x < nx; x += blockDim.x) {
     const double xc = (double)x * lx / (double)nx;
     double v = 0.0;
@@ -155,14 +161,33 @@ __device__ __forceinline__ void k_jet_field_body(const uint3 bid, T* __restrict_
       }
     }
     phys[((size_t)p * nz + z) * nx + x] = (T)v;
-    if (phys64) phys64[((size_t)p * nz + z) * nx + x] = v;
+    if (rows64) {
+      row[x] = v;
+      sincospi(-2.0 * (double)x / (double)nx, &tw[x].y, &tw[x].x);
+    }
+  }
+  if (!rows64) return;
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  for (int kx = threadIdx.x >> 5; kx < nk; kx += blockDim.x >> 5) {
+    double re = 0.0, im = 0.0;
+    for (int x = lane; x < nx; x += 32) {
+      const double2 c = tw[kx * x % nx];
+      re += row[x] * c.x;
+      im += row[x] * c.y;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      re += __shfl_xor_sync(0xffffffffu, re, o);
+      im += __shfl_xor_sync(0xffffffffu, im, o);
+    }
+    if (lane == 0) rows64[((size_t)p * nk + kx) * nz + z] = make_double2(re, im);
   }
 }
 
 template <typename T>
-__global__ void k_jet_field(T* __restrict__ phys, double* __restrict__ phys64, JetParams jp,
+__global__ void k_jet_field(T* __restrict__ phys, double2* __restrict__ rows64, int nk, JetParams jp,
                             const JetState* __restrict__ st, int nx, int nz, double lx, double lz) {
-  k_jet_field_body<T>(blockIdx, phys, phys64, jp, st, nx, nz, lx, lz);
+  k_jet_field_body<T>(blockIdx, phys, rows64, nk, jp, st, nx, nz, lx, lz);
 }
 
 // spec[p][kx][kz] (p = 0 suction, 1 bottom, 2 top) -> cbc(:,:,2) of the
@@ -210,31 +235,32 @@ __global__ void k_jet_combine(const cplx_t<T>* __restrict__ spec, cplx_t<T>* __r
   k_jet_combine_body<T>(blockIdx, spec, cbc, jp, gd, nx, nz, nxh, lx, lz);
 }
 
-// k_jet_low: grid (n), block 256: the forced walls' coefficients of the list's
-// wavenumbers in FP64, out[wall][n], by direct sums over the planes phys64.
-// The change of a wall value from substep to substep reaches the pressure
-// divided by k dt, and the rounding of FP32 values with it: 1e-6 of velocity
-// and pressure together, all of it in the lowest few kx (36x46x24, dt 0.002,
-// jet amplitude 0.1).  Nyquist coefficients keep the FP32 value (cbc, after
-// k_jet_combine).
+// k_jet_low: grid (n), block 128: the forced walls' coefficients of the list's
+// wavenumbers in FP64, out[wall][n], by direct sums over z of the rows'
+// coefficients rows64.  The change of a wall value from substep to substep
+// reaches the pressure divided by k dt, and the rounding of FP32 values with
+// it: 1e-6 of velocity and pressure together, all of it in the lowest few kx
+// (36x46x24, dt 0.002, jet amplitude 0.1).  Nyquist coefficients keep the FP32
+// value (cbc, after k_jet_combine).  Sums over the whole planes instead took
+// 75 us a substep at 128x129x128, more than the jet has beside the nonlinear
+// term.
 __device__ __forceinline__ void k_jet_low_body(int i, int n, const int* __restrict__ list,
-                                               const double* __restrict__ phys64, const float2* __restrict__ cbc,
-                                               double2* __restrict__ out, JetParams jp, GridDev gd, int nx, int nz,
-                                               int nxh, double lx, double lz) {
-  __shared__ double red[9][8];
+                                               const double2* __restrict__ rows64, int nk,
+                                               const float2* __restrict__ cbc, double2* __restrict__ out, JetParams jp,
+                                               GridDev gd, int nx, int nz, int nxh, double lx, double lz) {
+  __shared__ double red[9][4];
   const int w = list[i], kx = w / nz, kz = w % nz, t = threadIdx.x;
   const size_t np = (size_t)nx * nz, nw = (size_t)nz * nxh;
   double a[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};   // per plane: the coefficient, the mean
-  for (size_t q = t; q < np; q += 256) {
-    const int x = (int)(q % nx), z = (int)(q / nx);
+  for (int z = t; z < nz; z += 128) {
     double sn, cs;
-    sincospi(2.0 * ((double)((long long)kx * x % nx) / nx + (double)((long long)kz * z % nz) / nz), &sn, &cs);
+    sincospi(-2.0 * (double)((long long)kz * z % nz) / (double)nz, &sn, &cs);
 #pragma unroll
     for (int p = 0; p < 3; ++p) {
-      const double v = phys64[p * np + q];
-      a[3 * p] += v * cs;
-      a[3 * p + 1] -= v * sn;
-      a[3 * p + 2] += v;
+      const double2 v = rows64[((size_t)p * nk + kx) * nz + z];
+      a[3 * p] += v.x * cs - v.y * sn;
+      a[3 * p + 1] += v.x * sn + v.y * cs;
+      a[3 * p + 2] += rows64[(size_t)p * nk * nz + z].x;
     }
   }
 #pragma unroll
@@ -244,10 +270,8 @@ __device__ __forceinline__ void k_jet_low_body(int i, int n, const int* __restri
   }
   __syncthreads();
   if (t >= 2) return;
-  for (int r = 0; r < 9; ++r) {
-    a[r] = 0.0;
-    for (int o = 0; o < 8; ++o) a[r] += red[r][o];
-  }
+#pragma unroll
+  for (int r = 0; r < 9; ++r) a[r] = red[r][0] + red[r][1] + red[r][2] + red[r][3];
   const int wall = t;
   if (kx == nx / 2 || kz == nz / 2) {
     const float2 v = cbc[((size_t)wall * 3 + 1) * nw + w];
@@ -262,18 +286,18 @@ __device__ __forceinline__ void k_jet_low_body(int i, int n, const int* __restri
     double f = 1.0 / (double)np;
     for (int r = 0; r < jp.filter; ++r) f *= 0.25 * fx * fz;
     const double sg = wall == 1 ? -1.0 : 1.0;
-    const double* const j = a + 3 * (1 + wall);
-    const double q = sg * j[2] / a[2];
-    v = make_double2(f * (sg * j[0] - q * a[0]), f * (sg * j[1] - q * a[1]));
+    const double q = sg * (wall ? a[8] : a[5]) / a[2];
+    v = make_double2(f * (sg * (wall ? a[6] : a[3]) - q * a[0]), f * (sg * (wall ? a[7] : a[4]) - q * a[1]));
   }
   out[(size_t)wall * n + i] = v;
 }
 
-__global__ void __launch_bounds__(256) k_jet_low(int n, const int* __restrict__ list,
-                                                 const double* __restrict__ phys64, const float2* __restrict__ cbc,
-                                                 double2* __restrict__ out, JetParams jp, GridDev gd, int nx, int nz,
-                                                 int nxh, double lx, double lz) {
-  k_jet_low_body((int)blockIdx.x, n, list, phys64, cbc, out, jp, gd, nx, nz, nxh, lx, lz);
+__global__ void __launch_bounds__(128) k_jet_low(int n, const int* __restrict__ list,
+                                                 const double2* __restrict__ rows64, int nk,
+                                                 const float2* __restrict__ cbc, double2* __restrict__ out,
+                                                 JetParams jp, GridDev gd, int nx, int nz, int nxh, double lx,
+                                                 double lz) {
+  k_jet_low_body((int)blockIdx.x, n, list, rows64, nk, cbc, out, jp, gd, nx, nz, nxh, lx, lz);
 }
 
 // ---------------------------------------------------------------------------
