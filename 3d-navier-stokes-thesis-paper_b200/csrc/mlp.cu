@@ -237,7 +237,11 @@ __global__ void __launch_bounds__(NTH, 1) k_mlp_train(const uint4* img, const fl
   __shared__ __align__(8) uint64_t bar;
   __shared__ uint32_t tslot;
   __shared__ float sb[NBIAS];
-  __shared__ float sg[4][H + 1];   // per-warp sums: bias gradients, the loss at H
+  // per-warp sums: bias gradients, the loss at H; two copies, a layer's and the
+  // next one's: between a copy's reads and its next writes lies the other
+  // layer's block barrier (a product's mbarrier would not do: it completes on
+  // thread 0's commit, whatever the reading warps are at)
+  __shared__ float sg[2][4][H + 1];
   const int tid = threadIdx.x, p = tid & (TILE - 1), half = tid / TILE;
   const int warp = (tid >> 5) & 3, lane = tid & 31;   // warp: of the tile's four groups of 32 points
   const int r = blockIdx.x * TILE + p;
@@ -301,12 +305,12 @@ __global__ void __launch_bounds__(NTH, 1) k_mlp_train(const uint4* img, const fl
       sm[Smem::DZ + unit_of(p, 0, TILE)] = pack8(dz);
       sm[Smem::DZ + unit_of(p, 8, TILE)] = pack8(dz + 8);
 #pragma unroll
-      for (int c = 0; c < OUT; ++c) warp_sum_to(dz[c], &sg[warp][c]);
-      warp_sum_to(lsum / (6.0f * (float)batch), &sg[warp][H]);
+      for (int c = 0; c < OUT; ++c) warp_sum_to(dz[c], &sg[0][warp][c]);
+      warp_sum_to(lsum / (6.0f * (float)batch), &sg[0][warp][H]);
     }
     sync_for_mma();
-    if (tid < OUT) grad[OFF_B3 + p] = sg[0][p] + sg[1][p] + sg[2][p] + sg[3][p];
-    if (tid == TILE - 1) grad[NPARAM] = sg[0][H] + sg[1][H] + sg[2][H] + sg[3][H];
+    if (tid < OUT) grad[OFF_B3 + p] = sg[0][0][p] + sg[0][1][p] + sg[0][2][p] + sg[0][3][p];
+    if (tid == TILE - 1) grad[NPARAM] = sg[0][0][H] + sg[0][1][H] + sg[0][2][H] + sg[0][3][H];
   }
   // backward through layers 3, 2, 1 (weight and input gradients), then the
   // weight gradient of layer 0
@@ -356,12 +360,12 @@ __global__ void __launch_bounds__(NTH, 1) k_mlp_train(const uint4* img, const fl
       for (int i = 0; i < 32; ++i) dx[i] = valid ? dx[i] * gelu_d(z[i] + sb[bias_base(lp) + 32 * half + i]) : 0.f;
 #pragma unroll
       for (int q = 0; q < 4; ++q) sm[Smem::DZ + unit_of(p, 32 * half + 8 * q, TILE)] = pack8(dx + 8 * q);
-      sg[warp][32 * half + lane] = warp_sums32(dx);
+      sg[l & 1][warp][32 * half + lane] = warp_sums32(dx);
     }
     sync_for_mma();
-    // the bias gradient of layer l - 1 (sg is next written after the next
-    // product's barrier)
-    if (l > 0 && tid < H) grad[layer(l - 1).boff + p] = sg[0][p] + sg[1][p] + sg[2][p] + sg[3][p];
+    // the bias gradient of layer l - 1
+    if (l > 0 && tid < H)
+      grad[layer(l - 1).boff + p] = sg[l & 1][0][p] + sg[l & 1][1][p] + sg[l & 1][2][p] + sg[l & 1][3][p];
   }
   if (!ok && tid == 0) atomicExch(err, 1);
   fence_before_sync();

@@ -31,3 +31,27 @@ def test_steps_equal_their_routines(cf, nx, ny, nz, steps, prec):
     assert ends[0][3][0] != 1e-3
     for a, b in zip(*ends):
         np.testing.assert_array_equal(a, b)
+
+
+def test_training_batches_equal_separate_ones(cf):
+    """The gradients of batches in a row, of changing sizes, against the same batches with a wait after each."""
+    import torch
+    rng = np.random.default_rng(2)
+    x, t = (torch.from_numpy(rng.standard_normal((20000, n)).astype(np.float32)).cuda() for n in (10, 6))
+    params = (0.1 * rng.standard_normal(9414)).astype(np.float32)
+    idx = [torch.from_numpy(rng.integers(0, 20000, b).astype(np.int32)).cuda()
+           for b in [20000] + [1, 127, 128, 129, 4096, 3000, 20000, 64] * 8]
+    ends = []
+    for wait in (False, True):
+        m = cf.Mlp(params=params)
+        for i in idx:
+            m.accumulate_grad(x.data_ptr(), t.data_ptr(), i.data_ptr(), len(i))
+            if wait:
+                torch.cuda.synchronize()
+        g, loss = m.grads()
+        m.adam_step(1e-3)
+        ends.append((g, np.float32(loss), m.get_params()))
+        assert m.status() == 0
+        m.close()
+    for a, b in zip(*ends):
+        np.testing.assert_array_equal(a, b)
