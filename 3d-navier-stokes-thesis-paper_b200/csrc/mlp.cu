@@ -72,14 +72,18 @@ __device__ __forceinline__ void issue_dw(uint32_t d, uint32_t sDZ, uint32_t sX, 
 
 // ------------------------------------------------------------- tile helpers
 // half of a point's features into X0 (10, BF16, padded to 16; half 0 features
-// 0-7, half 1 the other two); rows are 8-byte aligned
+// 0-7, half 1 the other two).  PAIRS: x on 8 bytes, read two floats at a time;
+// a caller's array may lie at any float
+template <bool PAIRS>
 __device__ __forceinline__ void load_x0(uint4* sm, const float* x, long long row, bool valid, int p,
                                         int half) {
-  const float2* src = reinterpret_cast<const float2*>(x + row * IN) + 4 * half;
+  const float* src = x + row * IN + 8 * half;
   float v[8];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const float2 f = valid && (half == 0 || i == 0) ? src[i] : make_float2(0.f, 0.f);
+    float2 f = make_float2(0.f, 0.f);
+    if (valid && (half == 0 || i == 0))
+      f = PAIRS ? reinterpret_cast<const float2*>(src)[i] : make_float2(src[2 * i], src[2 * i + 1]);
     v[2 * i] = f.x;
     v[2 * i + 1] = f.y;
   }
@@ -153,7 +157,7 @@ struct PlainOut {
 // the GELU its half.  (Two threads per point, as in training, run 17 % slower
 // here: 48 warps of 40 registers spill, and the six CTAs hide each other's
 // waits already.)
-template <class Out>
+template <class Out, bool PAIRS>
 __global__ void __launch_bounds__(TILE) k_mlp_fwd(const uint4* __restrict__ img, const float* __restrict__ bias,
                                                  const float* __restrict__ x, Out out, long long n,
                                                  int* __restrict__ err) {
@@ -180,8 +184,8 @@ __global__ void __launch_bounds__(TILE) k_mlp_fwd(const uint4* __restrict__ img,
   const long long ntiles = (n + TILE - 1) / TILE;
   for (long long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
     const long long row = tile * TILE + p;
-    load_x0(sm, x, row, row < n, p, 0);
-    load_x0(sm, x, row, row < n, p, 1);
+    load_x0<PAIRS>(sm, x, row, row < n, p, 0);
+    load_x0<PAIRS>(sm, x, row, row < n, p, 1);
     for (int l = 0; l < 4 && ok; ++l) {
       sync_for_mma();
       if (p == 0) {
@@ -230,6 +234,7 @@ __global__ void __launch_bounds__(TILE) k_mlp_fwd(const uint4* __restrict__ img,
 // every weight gradient by the one thread that holds it, every bias gradient
 // and the loss as the sum of the four warps' sums in warp order, so that the
 // slice does not depend on the order in which warps or tiles finish.
+template <bool PAIRS>
 __global__ void __launch_bounds__(NTH, 1) k_mlp_train(const uint4* img, const float* bias,
                                                       const float* x, const float* t, const int* idx, int batch,
                                                       float* part, int* err) {
@@ -259,7 +264,7 @@ __global__ void __launch_bounds__(NTH, 1) k_mlp_train(const uint4* img, const fl
     fence_mbar_init();
   }
   float* const grad = part + (size_t)blockIdx.x * PART_STRIDE;
-  load_x0(sm, x, row, valid, p, half);
+  load_x0<PAIRS>(sm, x, row, valid, p, half);
   sync_for_mma();
   fence_after_sync();
   const uint32_t tm = tslot, tlane = tm + ((uint32_t)(32 * warp) << 16);
@@ -484,21 +489,19 @@ int cfg_mlp_create(int device, cfg_mlp** out) {
   cudaMemset(m->loss, 0, sizeof(float) + sizeof(int));
   cudaMemset(m->img, 0, IMG_UNITS * sizeof(uint4));   // the padding stays zero
   cudaMemset(m->bias, 0, NBIAS * sizeof(float));
-  if (cudaFuncSetAttribute(k_mlp_fwd<PlainOut>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_FWD) !=
-          cudaSuccess ||
-      cudaFuncSetAttribute(k_mlp_fwd<cfd::LesBlend<float>>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)SMEM_FWD) != cudaSuccess ||
-      cudaFuncSetAttribute(k_mlp_fwd<cfd::LesBlend<double>>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)SMEM_FWD) != cudaSuccess ||
-      cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_TRAIN) != cudaSuccess ||
-      // the whole of the SM's on-chip memory as shared memory: six forward
-      // CTAs per SM
-      cudaFuncSetAttribute(k_mlp_fwd<PlainOut>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                           (int)cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
-      cudaFuncSetAttribute(k_mlp_fwd<cfd::LesBlend<float>>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                           (int)cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
-      cudaFuncSetAttribute(k_mlp_fwd<cfd::LesBlend<double>>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                           (int)cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
+  // forward: the whole of the SM's on-chip memory as shared memory, six CTAs
+  // per SM
+  auto fwd_attr = [](auto kernel) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_FWD) == cudaSuccess &&
+           cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                (int)cudaSharedmemCarveoutMaxShared) == cudaSuccess;
+  };
+  auto train_attr = [](auto kernel) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_TRAIN) == cudaSuccess;
+  };
+  if (!fwd_attr(k_mlp_fwd<PlainOut, true>) || !fwd_attr(k_mlp_fwd<PlainOut, false>) ||
+      !fwd_attr(k_mlp_fwd<cfd::LesBlend<float>, true>) || !fwd_attr(k_mlp_fwd<cfd::LesBlend<double>, true>) ||
+      !train_attr(k_mlp_train<true>) || !train_attr(k_mlp_train<false>) ||
       cudaDeviceSynchronize() != cudaSuccess) {
     cfg_mlp_destroy(m);
     return CFG_E_CUDA;
@@ -535,6 +538,9 @@ int cfg_mlp_get_params(cfg_mlp* m, float* params) {
                                                                                                   : CFG_E_CUDA;
 }
 
+// the alignment that the feature loads in pairs need
+static bool on_8_bytes(const void* p) { return reinterpret_cast<uintptr_t>(p) % 8 == 0; }
+
 int cfg_mlp_forward(cfg_mlp* m, const float* x, float* y, long long n, void* stream) {
   if (!m || n < 0 || (n > 0 && (!x || !y))) return CFG_E_ARG;
   if (n == 0) return CFG_OK;
@@ -544,7 +550,8 @@ int cfg_mlp_forward(cfg_mlp* m, const float* x, float* y, long long n, void* str
   // would hold eight); a grid past what is resident leaves a second,
   // partial wave (measured 2.5x slower)
   const int grid = (int)(ntiles < 6LL * m->nsm ? ntiles : 6LL * m->nsm);
-  k_mlp_fwd<PlainOut><<<grid, TILE, SMEM_FWD, (cudaStream_t)stream>>>(m->img, m->bias, x, PlainOut{y}, n, m->err);
+  auto* const kernel = on_8_bytes(x) ? k_mlp_fwd<PlainOut, true> : k_mlp_fwd<PlainOut, false>;
+  kernel<<<grid, TILE, SMEM_FWD, (cudaStream_t)stream>>>(m->img, m->bias, x, PlainOut{y}, n, m->err);
   return cudaGetLastError() == cudaSuccess ? CFG_OK : CFG_E_CUDA;
 }
 
@@ -565,7 +572,7 @@ int cfg_mlp_accumulate_grad(cfg_mlp* m, const float* x, const float* t, const in
   const cudaStream_t st = (cudaStream_t)stream;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   const bool pdl = cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
-  cfd::launch_chained(pdl, k_mlp_train, dim3(ntiles), dim3(NTH), SMEM_TRAIN, st, (const uint4*)m->img,
+  cfd::launch_chained(pdl, on_8_bytes(x) ? k_mlp_train<true> : k_mlp_train<false>, dim3(ntiles), dim3(NTH), SMEM_TRAIN, st, (const uint4*)m->img,
                       (const float*)m->bias, x, t, idx, batch, m->part, m->err);
   cfd::launch_chained(pdl, k_mlp_reduce, dim3((NPARAM + 1 + 63) / 64), dim3(64), 0, st, (const float*)m->part, ntiles,
                       m->G, m->loss);
@@ -619,7 +626,7 @@ int mlp_forward_blend(cfg_mlp* m, long long n, const LesBlend<T>& b, void* strea
   cudaSetDevice(m->dev);
   const long long ntiles = (n + TILE - 1) / TILE;
   const int grid = (int)(ntiles < 6LL * m->nsm ? ntiles : 6LL * m->nsm);
-  k_mlp_fwd<LesBlend<T>><<<grid, TILE, SMEM_FWD, (cudaStream_t)stream>>>(m->img, m->bias, b.F, b, n, m->err);
+  k_mlp_fwd<LesBlend<T>, true><<<grid, TILE, SMEM_FWD, (cudaStream_t)stream>>>(m->img, m->bias, b.F, b, n, m->err);
   return cudaGetLastError() == cudaSuccess ? CFG_OK : CFG_E_CUDA;
 }
 template int mlp_forward_blend<float>(cfg_mlp*, long long, const LesBlend<float>&, void*);
