@@ -121,10 +121,16 @@ __global__ void __launch_bounds__(256) k_les_sgs(const T* __restrict__ P, T* __r
   }
   if (les.model == 2) {
     __syncthreads();
-    // (plane is even, so the block's part of F starts on 8 bytes)
+    // (plane is even, so the block's part of F starts on 8 bytes if F does; a
+    // caller's array may lie at any float)
     const int n2 = min(256, plane - base) * 5;
-    float2* const out = reinterpret_cast<float2*>(F + ((size_t)(k - 2) * plane + base) * 10);
-    for (int i = threadIdx.x; i < n2; i += 256) out[i] = reinterpret_cast<const float2*>(sf)[i];
+    float* const out = F + ((size_t)(k - 2) * plane + base) * 10;
+    if (reinterpret_cast<size_t>(F) % 8 == 0) {
+      for (int i = threadIdx.x; i < n2; i += 256)
+        reinterpret_cast<float2*>(out)[i] = reinterpret_cast<const float2*>(sf)[i];
+    } else {
+      for (int i = threadIdx.x; i < 2 * n2; i += 256) out[i] = sf[i];
+    }
   }
 }
 

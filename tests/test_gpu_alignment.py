@@ -36,3 +36,20 @@ def test_network_arrays_at_an_odd_float(cf, n):
     for a, b in zip(*ends):
         np.testing.assert_array_equal(a, b)
     net.close()
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+def test_les_features_at_an_odd_float(cf, prec):
+    import torch
+    f = cf.ChannelFlow(cf.Grid(32, 17, 32, stretch=1.5), re=3000.0, dt=0.004, precision=prec)
+    f.define_initial_field(10, seed=4, ampl=5e-2)
+    f.set_les(2, mlp=cf.Mlp(params=np.zeros(9414, np.float32)))
+    n = (f.ny - 1) * f.grid.nz2 * f.grid.nx2 * 10
+    a = torch.zeros(n, device="cuda")
+    b = shifted(torch.zeros(n, device="cuda"))
+    for out in (a, b):
+        f.les_features(out.data_ptr())
+        f.synchronize()
+    assert a.cpu().numpy().any()
+    np.testing.assert_array_equal(a.cpu().numpy(), b.cpu().numpy())
+    f.close()
