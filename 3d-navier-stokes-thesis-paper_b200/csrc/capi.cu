@@ -199,7 +199,6 @@ struct cfg_ctx {
   void* P = nullptr;
   bool split_x = false;
   int flux_zr = 4;
-  bool flux_given = false;   // flux_zr was asked for: products without that block refuse it
   void* cbc = nullptr;   // [bot, top][3][nw]
   DevScalars* sc = nullptr;
   double* d_um_dy = nullptr;
@@ -527,8 +526,7 @@ struct Impl {
     // 74.6 us), 4 beyond (192x129x192, 256x193x256: 164 / 196, 405 / 450); 2 in
     // FP64
     c->flux_zr = f32 ? (g.nx2 <= 192 && (gp.nz2 % 8 == 0 || !regfft_full(g.nx2)) ? 8 : 4) : 2;
-    c->flux_given = getenv("CHANFLOW_FLUX_ZR") != nullptr;
-    if (c->flux_given) {
+    if (getenv("CHANFLOW_FLUX_ZR")) {
       c->flux_zr = atoi(getenv("CHANFLOW_FLUX_ZR"));
       if (c->flux_zr != 2 && !(c->flux_zr == 8 && f32)) c->flux_zr = 4;   // 8 rows: FP32 only
     }
@@ -594,13 +592,12 @@ struct Impl {
   }
 
   // z rows per flux block: the tile where the products have that block (8
-  // rows: not the linearized and the LES ones; asked for, the lengths of
-  // regfft_full leave that to the launch), else 4; lengths of regfft_full also
-  // want it to divide the z2 rows
+  // rows: not the linearized and the LES ones), whoever chose it, else 4;
+  // lengths of regfft_full also want it to divide the z2 rows
   static int flux_rows(const cfg_ctx* c, bool plain_products) {
     const int zr = c->flux_zr, nz2 = c->gP.nz2;
     const bool full = regfft_full(c->g.nx2);
-    if ((nz2 % zr == 0 || !full) && (zr < 8 || plain_products || (c->flux_given && full))) return zr;
+    if ((nz2 % zr == 0 || !full) && (zr < 8 || plain_products)) return zr;
     return nz2 % 4 == 0 || !full ? 4 : 2;
   }
 
@@ -2938,11 +2935,10 @@ int cfg_autotune(cfg_ctx* c, int trial_steps, int* choice) {
     else tune(&c->rhs2_warps, {1, 2});
   }
 
-  // a row count that does not split, or the 8-row block outside the
-  // FP32 nonlinear products, fails its trial
-  const int zr0 = c->flux_zr;
-  if (c->split_x) tune(&c->flux_zr, {2, 4, 8});
-  c->flux_given = c->flux_given || c->flux_zr != zr0;
+  // (8 rows: only where these products have that block; elsewhere its trial
+  // would run 4 and win or lose by noise)
+  if (c->split_x && f32 && !c->les_on) tune(&c->flux_zr, {2, 4, 8});
+  else if (c->split_x) tune(&c->flux_zr, {2, 4});
   if (c->fast_z) {
     // planes per z-transform block (a block too large for its launch fails
     // its trial)
@@ -2987,7 +2983,6 @@ int cfg_set_tiles(cfg_ctx* c, const int* tiles) {
     return fail(c, CFG_E_ARG, "cfg_set_tiles: unsupported tiles");
   c->rhs2_warps = w;
   c->flux_zr = fz;
-  c->flux_given = true;
   c->fYB1 = y1;
   c->fYB3 = y3;
   return CFG_OK;
@@ -3490,9 +3485,7 @@ static int ens_tune_batched(cfg_ensemble* e, int trial_steps) {
       for (int i : groups[q]) e->m[i]->*knob = bestv;
     };
     tune(&cfg_ctx::rhs2_warps, {2, 3, 4});
-    const int zr0 = e->m[groups[q][0]]->flux_zr;
     tune(&cfg_ctx::flux_zr, {2, 4, 8});
-    for (int i : groups[q]) e->m[i]->flux_given = e->m[i]->flux_given || e->m[i]->flux_zr != zr0;
     tune(&cfg_ctx::fYB1, {1, 2, 4, 8});
     tune(&cfg_ctx::fYB3, {1, 2, 4, 8});
     tune(&cfg_ctx::xinv_zb, {8, 16, 24});
