@@ -1796,10 +1796,17 @@ int cfg_set_les(cfg_ctx* c, const cfg_les* l) {
   const size_t cs = (size_t)g.nz2 * g.nx2;
   const size_t tsz = c->mixed ? sizeof(float) : sizeof(double);
   c->les_points = (unsigned long long)(g.ny - 1) * cs;
+  // (each by itself: a call that ran out of memory may be made again)
+  if ((!c->les_nfall && cudaMalloc(&c->les_nfall, 8) != cudaSuccess) ||
+      (!c->les_len && cudaMalloc(&c->les_len, sizeof(double) * (g.ny + 1)) != cudaSuccess)) {
+    cudaGetLastError();
+    return fail(c, CFG_E_NOMEM, "LES lengths");
+  }
   if (!c->les_S) {
-    if (cudaMalloc(&c->les_S, tsz * 6 * cs * g.ny1) != cudaSuccess || cudaMalloc(&c->les_nfall, 8) != cudaSuccess ||
-        cudaMalloc(&c->les_len, sizeof(double) * (g.ny + 1)) != cudaSuccess)
+    if (cudaMalloc(&c->les_S, tsz * 6 * cs * g.ny1) != cudaSuccess) {
+      cudaGetLastError();
       return fail(c, CFG_E_NOMEM, "LES stresses");
+    }
     CK(cudaMemsetAsync(c->les_S, 0, tsz * 6 * cs * g.ny1, c->st));   // wall planes stay zero
   }
   if (l->model == 2 && !c->les_F) {
