@@ -2892,9 +2892,15 @@ int cfg_autotune(cfg_ctx* c, int trial_steps, int* choice) {
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
-  // one trial: restore, one untimed step, trial_steps timed steps; a
-  // failing launch or a device error flag disqualifies the setting
+  // one trial: restore, one untimed step, trial_steps timed steps, with the
+  // dependent launches of cfg_timestep; a failing launch or a device error
+  // flag disqualifies the setting
   auto trial = [&]() -> float {
+    struct Chained {
+      cfg_ctx* c;
+      explicit Chained(cfg_ctx* x) : c(x) { c->chained = true; }
+      ~Chained() { c->chained = false; }
+    } chained(c);
     if (snap_restore(c, snap)) return -1.f;
     c->step = step0;
     c->mean64_valid = mean_ok;
