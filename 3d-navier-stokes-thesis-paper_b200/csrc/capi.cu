@@ -566,11 +566,19 @@ struct Impl {
     }
     c->rhs2_warps = f32 ? 3 : 2;
     // a thread per row (k_rhs_rows) for every wavenumber up to 512 rows per
-    // SM, what its registers let an SM hold at once: beyond one wave its
-    // extra (FP64) operations cost more than k_rhs2's unfilled SMs (us per
-    // step, k_rhs2 / k_rhs_rows, mixed: 32x33x32 133 / 120, 32x65x32 145 /
-    // 132, 48x49x48 175 / 173, 64x33x64 161 / 180, 96x97x96 385 / 552; FP64:
-    // 126 / 119, 148 / 136, 180 / 190, 213 / 201, 755 / 749).
+    // SM, what its registers let an SM hold at once, where it is ahead of
+    // k_rhs2's unfilled SMs in both precisions.  us per step, k_rhs2 /
+    // k_rhs_rows, by rows per SM, mixed and FP64:
+    //    235 (32x33x32)   83 /  70    85 /  75
+    //    353 (32x65x32)   95 /  85   107 /  96
+    //    519 (48x33x48)  119 / 100   105 / 104
+    //    519 (48x49x48)  140 / 110   121 / 126
+    //    913 (64x33x64)  113 / 118   151 / 129
+    //   1370 (64x65x64)  136 / 164   210 / 201
+    //   4068 (96x97x96)  292 / 432   638 / 603
+    // Beyond it mixed precision loses, its FP64 operations costing more than
+    // the FP32 ones of k_rhs2, and FP64 gains on most grids: the line is the
+    // one that loses nowhere, not the best one of either.
     // The whole grid's count, so that the ranks of a group solve as one
     // context does.  CHANFLOW_RHS_ROWS=0|1 overrides.
     c->rhs_rows = c->use_rhs2 && (size_t)g.nz * g.nxh_all * ((g.ny1 + 31) / 32 * 32) <= 148 * 512;
@@ -1787,7 +1795,8 @@ int cfg_set_les(cfg_ctx* c, const cfg_les* l) {
   }
   if (l->model != 1 && l->model != 2) return fail(c, CFG_E_ARG, "cfg_set_les: model %d", l->model);
   if (!c->split_x || !c->full_len)
-    return fail(c, CFG_E_ARG, "cfg_set_les: needs the register-FFT x stage (nx2 of 24 .. 576)");
+    return fail(c, CFG_E_ARG, "cfg_set_les: needs the register-FFT x stage (nx2 of 24, 48, 72, 96, 144, 192, 288, 384 or 576, "
+                "nz2 in eights)");
   if (l->model == 2 && !l->mlp) return fail(c, CFG_E_ARG, "cfg_set_les: model 2 needs the network");
   if (!(l->cs >= 0.0) || !(l->aplus > 0.0) || !(l->beta >= 0.0)) return fail(c, CFG_E_ARG, "cfg_set_les: cs, aplus, beta");
   for (int i = 0; i < 10; ++i)
@@ -2958,8 +2967,8 @@ int cfg_autotune(cfg_ctx* c, int trial_steps, int* choice) {
     tune(&c->fYB1, {1, 2, 4, 8});
     tune(&c->fYB3, {1, 2, 4, 8});
   }
-  // z2 rows per inverse-x block (not one of the four public tiles; a row
-  // count that does not divide the slab fails its trial)
+  // z2 rows per inverse-x block (not one of the four public tiles; the last
+  // block takes the rows that are left)
   if (c->split_x) tune(&c->xinv_zb, {8, 16, 24});
   snap_restore(c, snap);
   CK(cudaStreamSynchronize(c->st));

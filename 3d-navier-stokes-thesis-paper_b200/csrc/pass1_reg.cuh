@@ -42,7 +42,7 @@ __device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_g
 // component (k_zinv_r) or equation (k_zfwd_r): the spectral state keeps y
 // innermost, so YP is the run its reads or writes make there, 8 planes of
 // FP32 a 64-byte run, where a block of fewer planes and all three components
-// (as this was: 2 to 4 planes at 256x193x256, 1 to 2 at 384x193x384) moves 8
+// (2 to 4 planes at 256x193x256, 1 to 2 at 384x193x384) moves 8
 // to 32 bytes of each 32-byte sector.  Everything that indexes by plane is
 // known at compile time, one thread takes one stage-1 and one stage-2 task,
 // and the 3/2-dealiased row count (DEAL: nz = 2 nz2/3) too: which of a

@@ -198,7 +198,7 @@ template <> struct Split<576> { static constexpr int N1 = 24, N2 = 24; };
 // Every 2^a 3^b length of 3/2-dealiased grids from 16 to 384 points: the
 // shared-memory Stockham passes (fft.cuh) read and write a sequence once per
 // radix and take 2.1 ms for a step at 144x100x108 (lengths 216 and 162) that
-// takes 0.67 ms here.
+// takes 0.52 ms here.
 __host__ __device__ constexpr bool regfft_supported(int n) {
   return n == 24 || n == 36 || n == 48 || n == 54 || n == 72 || n == 96 || n == 108 || n == 144 || n == 162 || n == 192 ||
          n == 216 || n == 288 || n == 324 || n == 384 || n == 432 || n == 576;
