@@ -3141,6 +3141,7 @@ struct cfg_ensemble {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   std::vector<long long> launches_per_step;
+  std::vector<bool> low_after;   // each member's low_ok after a step of the graph
   bool batched = false;        // step layout of the next capture
   bool last_batched = false;   // layout of the last enqueued step
   std::vector<EnsClass> cls;   // batched: the classes (built on first use)
@@ -3637,6 +3638,22 @@ int cfg_ensemble_timestep(cfg_ensemble* e, int nsteps) {
       // the capture advanced the host step counters without running a step
       e->m[i]->step -= 1;
       e->m[i]->launches = before[i];
+    }
+    e->low_after.clear();
+    for (const cfg_ctx* c : e->m) e->low_after.push_back(c->low_ok);
+  }
+  if (nsteps > 0) {
+    // what a member did by itself since: the graph solves from the FP64
+    // columns of the |k| < 4 lists where it was captured so, and takes the CFL
+    // maxima as they are
+    for (size_t i = 0; i < e->m.size(); ++i) {
+      cfg_ctx* c = e->m[i];
+      const bool widen = e->low_after[i] && !c->low_ok, clear = !c->cfl_clean;
+      if (widen && (r = low_widen(c))) return r;
+      if (clear) CK(cudaMemsetAsync(c->cflbits, 0, sizeof(unsigned long long) * 3 * c->g.ny1, c->st));
+      if (widen || clear) CK(cudaStreamSynchronize(c->st));
+      c->cfl_clean = true;
+      c->low_ok = e->low_after[i];
     }
   }
   for (int s = 0; s < nsteps; ++s) {

@@ -171,3 +171,46 @@ def test_autotune_restores(cf):
     for f in (a, b):
         f.timestep(2)
     same(state(a), state(b))
+
+
+@pytest.mark.parametrize("batched", [True, False])
+def test_ensemble_graph_after_learned_steps(cf, batched):
+    """A captured ensemble step goes on from what its members did by themselves in between."""
+    rng = np.random.default_rng(5)
+    net = cf.Mlp(params=(0.1 * rng.standard_normal(9414)).astype(np.float32))
+    m = [flow_of(cf, 32, 33, 32, 1) for _ in range(2)]
+    alone = flow_of(cf, 32, 33, 32, 1)
+    for i, f in enumerate(m):
+        start(f, 20 + i)
+    ens = cf.Ensemble(m, autotune=False, batched=batched)
+    ens.timestep(4)
+    ens.synchronize()
+    m[1].set_les(2, mlp=net)
+    m[1].timestep(2)
+    restore(alone, state(m[1]))
+    ens.timestep(3)
+    ens.synchronize()
+    alone.timestep(3)
+    same(state(m[1]), state(alone))
+    ens.close()
+
+
+def test_steps_after_a_captured_learned_member(cf):
+    rng = np.random.default_rng(6)
+    net = cf.Mlp(params=(0.1 * rng.standard_normal(9414)).astype(np.float32))
+    m = [flow_of(cf, 32, 33, 32, 1) for _ in range(2)]
+    alone = flow_of(cf, 32, 33, 32, 1)
+    for i, f in enumerate(m):
+        start(f, 30 + i)
+    m[1].set_les(2, mlp=net)
+    ens = cf.Ensemble(m, autotune=False)
+    ens.timestep(3)
+    ens.synchronize()
+    m[1].set_les(0)
+    ens.timestep(2)       # the captured step is the learned one
+    ens.synchronize()
+    restore(alone, state(m[1]))
+    for f in (m[1], alone):
+        f.timestep(2)
+    same(state(m[1]), state(alone))
+    ens.close()
